@@ -127,10 +127,13 @@ int env_int(const char *name, int fallback) {
 // A hash-kernel configuration chosen by the autotuner: samples per lane,
 // minimum resident blocks per SM (register budget) and items per resident
 // warp (chunk granularity).
+// filter: the bound-filtered kernel, which has one register budget and its own
+// tile (spl and minb then describe it: 4 samples per lane, 4 blocks per SM).
 struct TuneChoice {
   uint32_t spl = 4;
   uint32_t minb = 4;
   uint32_t waves = 32;
+  bool filter = false;
 };
 
 // The autotuner's two choices for a shape class.  `alone` is the fastest
@@ -177,7 +180,12 @@ struct MinhashCudaGenerator_ {
   int device = 0;
   uint32_t s_pad = 0;
   int sm_count = 0;
-  float *params = nullptr;  // [dim][3][s_pad]
+  float *params = nullptr;  // [dim][s_pad / 2][r r c c b b]
+  // Bound table of the filtered kernels, [dim][bound_stride(s_pad)]; nullptr
+  // when there is none.  bounds_ok: it belongs to the current parameters.
+  uint8_t *bounds = nullptr;
+  mutable std::atomic<bool> bounds_ok{false};
+  const uint8_t *usable_bounds() const { return bounds_ok.load() ? bounds : nullptr; }
   cudaStream_t stream = nullptr;
 
   // Serialises calls on one generator (the reference's generator is not
@@ -291,10 +299,22 @@ bool tuned_choice(const Gen *gen, uint64_t nnz, uint64_t rows, TuneChoice *out,
   return true;
 }
 
+constexpr uint32_t kFilterMinRow = 48;
+constexpr uint64_t kFilterMinEvals = 1ull << 29;
+
+// Whether a launch takes the bound-filtered kernel (filter_kernels.cu).
+bool use_filter(const Gen *gen, uint64_t nnz, uint64_t rows, const TuneChoice *tuned) {
+  if (!gen->usable_bounds()) return false;
+  const int forced = env_int("MHCUDA_B200_FILTER", -1);
+  if (forced >= 0) return forced != 0;
+  if (tuned) return tuned->filter;
+  return nnz >= kFilterMinRow * rows && nnz * gen->s_pad >= kFilterMinEvals;
+}
+
 // min_items: items per resident warp the chunk is capped to give (8 for the
 // engine's own calls; the server asks for 2, its launches overlap).
 HashPlan make_plan(const Gen *gen, uint64_t nnz, uint64_t rows, const TuneChoice *force = nullptr,
-                   uint32_t min_items = 8) {
+                   uint32_t min_items = 8, bool allow_filter = true) {
   HashPlan p{};
   const uint32_t s_pad = gen->s_pad;
   TuneChoice tuned{};
@@ -323,15 +343,17 @@ HashPlan make_plan(const Gen *gen, uint64_t nnz, uint64_t rows, const TuneChoice
   }
   p.spl = static_cast<uint32_t>(spl);
   p.minb = 4;
+  p.filter = allow_filter && use_filter(gen, nnz, rows, have_tuned ? &tuned : nullptr) ? 1u : 0u;
+  if (p.filter) p.spl = 4;
   if (p.spl == 4) {
     const int minb = env_int("MHCUDA_B200_MINB", have_tuned ? static_cast<int>(tuned.minb) : 4);
     p.minb = (minb == 3 || minb == 2) ? static_cast<uint32_t>(minb) : 4u;
   }
-  const uint32_t tile_w = 32u * p.spl;
+  const uint32_t tile_w = p.filter ? mhb::filter_tile(s_pad) : 32u * p.spl;
   p.ntiles = (s_pad + tile_w - 1) / tile_w;
-  const int bps = mhb::hash_blocks_per_sm(p.spl, p.minb, s_pad);
+  const int bps = mhb::plan_blocks_per_sm(p, s_pad);
   const uint64_t resident_warps =
-      static_cast<uint64_t>(gen->sm_count) * bps * (mhb::kHashBlock / 32);
+      static_cast<uint64_t>(gen->sm_count) * bps * mhb::plan_block_warps(p);
   const int waves = std::max(
       1, env_int("MHCUDA_B200_WAVES", have_tuned ? static_cast<int>(tuned.waves) : 32));
   const uint64_t target_items = resident_warps * waves;
@@ -343,7 +365,11 @@ HashPlan make_plan(const Gen *gen, uint64_t nnz, uint64_t rows, const TuneChoice
   // warp ends on a ragged last wave: keep at least min_items items per
   // resident warp even if rows then span chunks (their partials are merged
   // by finalize).
-  {
+  if (p.filter) {
+    // A row in pieces starts its search anew in each: chunks of a mean row at
+    // least.
+    chunk = std::max<uint64_t>(chunk, std::min<uint64_t>(avg_row, 4096));
+  } else {
     const uint64_t want = resident_warps * std::max<uint32_t>(1, min_items);
     chunk = std::min<uint64_t>(chunk, std::max<uint64_t>(64, (nnz * p.ntiles + want - 1) / want));
   }
@@ -355,7 +381,8 @@ HashPlan make_plan(const Gen *gen, uint64_t nnz, uint64_t rows, const TuneChoice
   const uint64_t nchunks = nnz == 0 ? 1 : (nnz + chunk - 1) / chunk;
   p.nchunks = static_cast<uint32_t>(nchunks);
   const uint64_t items = nchunks * p.ntiles;
-  const uint64_t want_blocks = (items + (mhb::kHashBlock / 32) - 1) / (mhb::kHashBlock / 32);
+  const uint32_t warps = mhb::plan_block_warps(p);
+  const uint64_t want_blocks = (items + warps - 1) / warps;
   const uint64_t max_blocks = static_cast<uint64_t>(gen->sm_count) * bps;
   p.grid = static_cast<uint32_t>(std::max<uint64_t>(1, std::min(want_blocks, max_blocks)));
   return p;
@@ -376,6 +403,9 @@ MHCUDAResult prepare_launch(const Gen *gen, uint32_t rows, uint32_t nnz, const H
   a->dim = gen->dim;
   a->samples = gen->samples;
   a->s_pad = gen->s_pad;
+  a->bounds = gen->usable_bounds();
+  a->b_stride = mhb::bound_stride(gen->s_pad);
+  a->snap_rows = plan.filter;
   a->rows = rows;
   a->nnz = nnz;
   a->chunk = plan.chunk;
@@ -868,7 +898,11 @@ MHCUDAResult calc_pipelined(const Gen *gen, const HostCsr &in, uint32_t length,
 
 // Scratch per buffer when the [samples][dim] parameter streams are handled a
 // block of sample rows at a time (init, retrieve, assign).
-constexpr uint64_t kParamChunkBytes = 1ull << 30;
+constexpr uint64_t kParamChunkBytes = 512ull << 20;
+
+// Largest bound table: with init's scratch it keeps a generator's device memory
+// within 4 GiB of its parameter table.
+constexpr size_t kMaxBoundBytes = size_t{2} << 30;
 
 // Sample rows per block: about kParamChunkBytes of floats, whole 8-row groups
 // (32-byte write segments in the table) when a block holds 8 rows or more.
@@ -881,66 +915,64 @@ uint32_t param_chunk_rows(uint32_t dim, uint32_t samples) {
   return static_cast<uint32_t>(std::min<uint64_t>(std::max<uint64_t>(rows, 1), samples));
 }
 
-// Fills the table from `seed` as minhashcuda.cc:179-199 does: one cuRAND
+// Fills the tables from `seed` as minhashcuda.cc:179-199 does: one cuRAND
 // generator of type CURAND_RNG_PSEUDO_DEFAULT draws five runs of dim*samples
 // uniforms U1..U5, and rs = -logf(U2*U1), ln_cs = logf(-logf(U3*U4)),
 // betas = U5, each run in [samples][dim] order.  The runs are not
-// materialised whole: two generators with that seed start at the absolute
-// offsets of a run pair (curandSetGeneratorOffset: draws k and k+1 begin at
-// k*n and (k+1)*n), each produces its run a block of sample rows at a time,
-// and every block is combined and transposed into the table at once.  Values
-// at an absolute offset do not depend on how the sequence is split into
-// calls, so the table equals the reference's bit for bit with scratch of two
-// blocks instead of two full runs (2 x 17 GB at 2^24 x 256).
+// materialised whole: five generators with that seed start at the runs'
+// absolute offsets (curandSetGeneratorOffset: run k begins at k*n), each
+// produces its run a block of sample rows at a time, and every block of the
+// five is combined, transposed into the parameter table and reduced to its
+// bound bytes at once.  Values at an absolute offset do not depend on how the
+// sequence is split into calls, so the table equals the reference's bit for
+// bit with scratch of five blocks instead of full runs (17 GB each at
+// 2^24 x 256).
 MHCUDAResult init_params(Gen *gen, uint32_t seed) {
   const uint32_t D = gen->dim, S = gen->samples, P = gen->s_pad;
   const uint64_t n = static_cast<uint64_t>(D) * S;
   const uint32_t rows = param_chunk_rows(D, S);
   const size_t block = static_cast<size_t>(rows) * D;
-  DevBuf a, b;
-  MHB_CHECK(gen, a.ensure(block * sizeof(float)), mhcudaMemoryAllocationFailure);
-  MHB_CHECK(gen, b.ensure(block * sizeof(float)), mhcudaMemoryAllocationFailure);
-  curandGenerator_t rng[2] = {nullptr, nullptr};
+  // Without room for five blocks the three parameters are filled in turn from
+  // two, and there are no bounds.
+  DevBuf buf;
+  const bool whole = buf.ensure(5 * block * sizeof(float)) == cudaSuccess;
+  if (!whole)
+    MHB_CHECK(gen, buf.ensure(2 * block * sizeof(float)), mhcudaMemoryAllocationFailure);
+  curandGenerator_t rng[5] = {};
   auto finish = [&](MHCUDAResult code) {
     for (curandGenerator_t g : rng)
       if (g) curandDestroyGenerator(g);
     return code;
   };
-  for (curandGenerator_t &g : rng) {
-    if (curandCreateGenerator(&g, CURAND_RNG_PSEUDO_DEFAULT) != CURAND_STATUS_SUCCESS) {
-      g = nullptr;
+  for (uint64_t k = 0; k < 5; ++k) {
+    if (curandCreateGenerator(&rng[k], CURAND_RNG_PSEUDO_DEFAULT) != CURAND_STATUS_SUCCESS) {
+      rng[k] = nullptr;
       return finish(mhcudaRuntimeError);
     }
-    if (curandSetStream(g, gen->stream) != CURAND_STATUS_SUCCESS ||
-        curandSetPseudoRandomGeneratorSeed(g, seed) != CURAND_STATUS_SUCCESS)
+    if (curandSetStream(rng[k], gen->stream) != CURAND_STATUS_SUCCESS ||
+        curandSetPseudoRandomGeneratorSeed(rng[k], seed) != CURAND_STATUS_SUCCESS ||
+        curandSetGeneratorOffset(rng[k], k * n) != CURAND_STATUS_SUCCESS)
       return finish(mhcudaRuntimeError);
   }
-  struct Pass {
-    mhb::PairOp op;
-    uint32_t which;     // table slot: 0 rs, 1 ln_cs, 2 betas
-    uint64_t first;     // index of the first uniform run it consumes
-    bool pair;          // consumes runs first and first+1
-  };
-  const Pass passes[3] = {{mhb::PairOp::kGamma, 0, 0, true},
-                          {mhb::PairOp::kLogGamma, 1, 2, true},
-                          {mhb::PairOp::kCopy, 2, 4, false}};
-  float *A = a.as<float>(), *B = b.as<float>();
-  for (const Pass &p : passes) {
-    if (curandSetGeneratorOffset(rng[0], p.first * n) != CURAND_STATUS_SUCCESS ||
-        (p.pair && curandSetGeneratorOffset(rng[1], (p.first + 1) * n) != CURAND_STATUS_SUCCESS))
-      return finish(mhcudaRuntimeError);
+  for (uint32_t parts : whole ? std::vector<uint32_t>{7u} : std::vector<uint32_t>{1u, 2u, 4u}) {
     for (uint32_t s0 = 0; s0 < S; s0 += rows) {
       const uint32_t cnt = std::min(rows, S - s0);
-      const size_t len = static_cast<size_t>(cnt) * D;
-      if (curandGenerateUniform(rng[0], A, len) != CURAND_STATUS_SUCCESS ||
-          (p.pair && curandGenerateUniform(rng[1], B, len) != CURAND_STATUS_SUCCESS))
-        return finish(mhcudaRuntimeError);
-      if (mhb::launch_pack_params(A, p.pair ? B : nullptr, p.op, p.which, D, s0, cnt, P,
-                                  gen->params, gen->stream) != cudaSuccess)
+      mhb::ParamSources in{};
+      for (uint32_t k = 0; k < 5; ++k) {
+        if (!(parts >> (k / 2) & 1u)) continue;  // U1, U2: r; U3, U4: ln_c; U5: beta
+        float *u = buf.as<float>() + static_cast<size_t>(whole ? k : k % 2) * block;
+        in.src[k] = u;
+        if (curandGenerateUniform(rng[k], u, static_cast<size_t>(cnt) * D) !=
+            CURAND_STATUS_SUCCESS)
+          return finish(mhcudaRuntimeError);
+      }
+      if (mhb::launch_pack_params(in, true, parts, D, s0, cnt, P, gen->params, gen->bounds,
+                                  gen->stream) != cudaSuccess)
         return finish(mhcudaRuntimeError);
     }
   }
   if (cudaStreamSynchronize(gen->stream) != cudaSuccess) return finish(mhcudaRuntimeError);
+  gen->bounds_ok = gen->bounds && whole;
   return finish(mhcudaSuccess);
 }
 
@@ -1011,13 +1043,14 @@ DeviceGuard::~DeviceGuard() {
 }
 
 HashPlan plan_for_generator(const MinhashCudaGenerator_ *gen, uint64_t nnz, uint64_t rows,
-                            uint32_t min_items) {
-  return make_plan(gen, nnz, rows, nullptr, min_items);
+                            uint32_t min_items, bool allow_filter) {
+  return make_plan(gen, nnz, rows, nullptr, min_items, allow_filter);
 }
 
 bool generator_view(const MinhashCudaGenerator_ *gen, GeneratorView *view) {
   if (!gen || !view) return false;
   view->params = gen->params;
+  view->bounds = gen->usable_bounds();
   view->dim = gen->dim;
   view->samples = gen->samples;
   view->s_pad = gen->s_pad;
@@ -1068,7 +1101,21 @@ MinhashCudaGenerator *mhcuda_init(uint32_t dim, uint16_t samples, uint32_t seed,
     return nullptr;
   }
   const size_t table = static_cast<size_t>(dim) * 3 * gen->s_pad * sizeof(float);
-  if (cudaMalloc(&gen->params, table) != cudaSuccess) {
+  // Behind it the bound table of the filtered kernels, a twelfth of the
+  // parameters: up to kMaxBoundBytes, and if a quarter of the device's memory
+  // is still free with both (the caller's data and the workspace come first).
+  // Without it the dense kernels serve all calls.  One allocation: each costs
+  // about a millisecond to make and to free.
+  const size_t bound_at = (table + 255) & ~static_cast<size_t>(255);
+  const size_t bound_bytes = static_cast<size_t>(dim) * mhb::bound_stride(gen->s_pad);
+  size_t free_now = 0, total_now = 0;
+  if (gen->s_pad >= mhb::kFilterMinSamples && bound_bytes <= kMaxBoundBytes &&
+      cudaMemGetInfo(&free_now, &total_now) == cudaSuccess &&
+      free_now >= bound_at + bound_bytes + total_now / 4 &&
+      cudaMalloc(&gen->params, bound_at + bound_bytes) == cudaSuccess)
+    gen->bounds = reinterpret_cast<uint8_t *>(gen->params) + bound_at;
+  cudaGetLastError();
+  if (!gen->bounds && cudaMalloc(&gen->params, table) != cudaSuccess) {
     cudaGetLastError();
     gen->params = nullptr;
     MHB_INFO(gen.get(), "failed to allocate %zu bytes for the parameter table\n", table);
@@ -1076,7 +1123,8 @@ MinhashCudaGenerator *mhcuda_init(uint32_t dim, uint16_t samples, uint32_t seed,
     return nullptr;
   }
   // Zero fill: padding samples and, with `deferred`, the whole table.
-  if (cudaMemsetAsync(gen->params, 0, table, gen->stream) != cudaSuccess) {
+  if ((deferred || gen->s_pad != samples) &&
+      cudaMemsetAsync(gen->params, 0, table, gen->stream) != cudaSuccess) {
     set(mhcudaRuntimeError);
     return nullptr;
   }
@@ -1145,23 +1193,33 @@ enum MHCUDAResult mhcuda_assign_random_vars(const MinhashCudaGenerator *gen, con
   MHB_ON_DEVICE(gen);
   const uint32_t D = gen->dim, S = gen->samples;
   const uint32_t rows = param_chunk_rows(D, S);
-  DevBuf tmp;
-  MHB_CHECK(gen, tmp.ensure(static_cast<size_t>(rows) * D * sizeof(float)),
-            mhcudaMemoryAllocationFailure);
+  const size_t block = static_cast<size_t>(rows) * D;
   const float *src[3] = {rs, ln_cs, betas};
-  for (uint32_t which = 0; which < 3; ++which) {
+  gen->bounds_ok = false;
+  // Without room for a block of each array, one array at a time and no bounds.
+  DevBuf tmp;
+  const bool whole = tmp.ensure(3 * block * sizeof(float)) == cudaSuccess;
+  if (!whole) MHB_CHECK(gen, tmp.ensure(block * sizeof(float)), mhcudaMemoryAllocationFailure);
+  for (uint32_t parts : whole ? std::vector<uint32_t>{7u} : std::vector<uint32_t>{1u, 2u, 4u}) {
     for (uint32_t s0 = 0; s0 < S; s0 += rows) {
       const uint32_t cnt = std::min(rows, S - s0);
-      const size_t len = static_cast<size_t>(cnt) * D;
-      MHB_CHECK(gen, cudaMemcpyAsync(tmp.ptr, src[which] + static_cast<size_t>(s0) * D,
-                                     len * sizeof(float), cudaMemcpyHostToDevice, gen->stream),
-                mhcudaMemoryCopyError);
-      MHB_CHECK(gen, mhb::launch_pack_params(tmp.as<float>(), nullptr, mhb::PairOp::kCopy, which,
-                                             D, s0, cnt, gen->s_pad, gen->params, gen->stream),
+      mhb::ParamSources in{};
+      for (uint32_t which = 0; which < 3; ++which) {
+        if (!(parts >> which & 1u)) continue;
+        float *t = tmp.as<float>() + (whole ? which * block : 0);
+        in.src[which] = t;
+        MHB_CHECK(gen, cudaMemcpyAsync(t, src[which] + static_cast<size_t>(s0) * D,
+                                       static_cast<size_t>(cnt) * D * sizeof(float),
+                                       cudaMemcpyHostToDevice, gen->stream),
+                  mhcudaMemoryCopyError);
+      }
+      MHB_CHECK(gen, mhb::launch_pack_params(in, false, parts, D, s0, cnt, gen->s_pad,
+                                             gen->params, gen->bounds, gen->stream),
                 mhcudaRuntimeError);
     }
   }
   MHB_CHECK(gen, cudaStreamSynchronize(gen->stream), mhcudaMemoryCopyError);
+  gen->bounds_ok = gen->bounds && whole;
   return mhcudaSuccess;
 }
 
@@ -1362,12 +1420,32 @@ enum MHCUDAResult mhcuda_calc_batch_device(const MinhashCudaGenerator *gen, uint
 
   // Kernel variant as for one large launch; the chunk size is chosen on the
   // device from the batch's nnz (batch_setup_kernel).
-  const HashPlan vp = make_plan(gen, 1ull << 30, 1ull << 20);
-  const int bps = mhb::hash_blocks_per_sm(vp.spl, vp.minb, gen->s_pad);
-  const uint64_t resident_warps =
-      static_cast<uint64_t>(gen->sm_count) * bps * (mhb::kHashBlock / 32);
+  HashPlan vp = make_plan(gen, 1ull << 30, 1ull << 20, nullptr, 8, false);
+  HashPlan fp = vp;
+  fp.filter = 1;
+  fp.ntiles = (gen->s_pad + mhb::filter_tile(gen->s_pad) - 1) / mhb::filter_tile(gen->s_pad);
+  // Whether the batch is filtered is decided on the device too; a batch of few
+  // rows is not worth the second launch that takes.
+  const int force_filter = env_int("MHCUDA_B200_FILTER", -1);
+  const bool may_filter = gen->usable_bounds() && force_filter != 0 &&
+                          (force_filter > 0 || plan_threads >= 4096);
   TuneChoice tc{};
   const int waves = std::max(1, env_int("MHCUDA_B200_WAVES", static_cast<int>(tc.waves)));
+  mhb::BatchArgs b{};
+  HashPlan *const plans[2] = {&vp, &fp};
+  uint64_t resident_warps = 0;
+  for (int f = 0; f < (may_filter ? 2 : 1); ++f) {
+    const int bps = mhb::plan_blocks_per_sm(*plans[f], gen->s_pad);
+    const uint64_t warps =
+        static_cast<uint64_t>(gen->sm_count) * bps * mhb::plan_block_warps(*plans[f]);
+    resident_warps = std::max(resident_warps, warps);
+    b.target_items[f] = warps * static_cast<uint64_t>(waves);
+    b.want_items[f] = warps * 8;
+    b.ntiles[f] = plans[f]->ntiles;
+    plans[f]->grid = static_cast<uint32_t>(static_cast<uint64_t>(gen->sm_count) * bps);
+  }
+  b.filter_min_row = !may_filter ? 0 : force_filter > 0 ? 1 : kFilterMinRow;
+  b.filter_min_nnz = force_filter > 0 ? 0 : kFilterMinEvals / gen->s_pad;
   const uint64_t max_chunks64 = count + resident_warps * 8 + 1;
   if (max_chunks64 >= 0xFFFFFFFFull) return mhcudaInvalidArguments;
   const uint32_t max_chunks = static_cast<uint32_t>(max_chunks64);
@@ -1388,7 +1466,8 @@ enum MHCUDAResult mhcuda_calc_batch_device(const MinhashCudaGenerator *gen, uint
                             static_cast<size_t>(count) * sizeof(uint32_t);
   const void *batch_scratch[2] = {gen->d_chunk_owner.ptr, gen->d_batch_plan.ptr};
   std::vector<unsigned char> key(mats_bytes + count * sizeof(uint32_t) + sizeof(st) +
-                                 sizeof(base) + sizeof(vp) + sizeof(batch_scratch));
+                                 sizeof(base) + sizeof(vp) + sizeof(b.filter_min_row) +
+                                 sizeof(batch_scratch));
   {
     unsigned char *k = key.data();
     memcpy(k, mats.data(), mats_bytes);
@@ -1401,6 +1480,8 @@ enum MHCUDAResult mhcuda_calc_batch_device(const MinhashCudaGenerator *gen, uint
     k += sizeof(base);
     memcpy(k, &vp, sizeof(vp));
     k += sizeof(vp);
+    memcpy(k, &b.filter_min_row, sizeof(b.filter_min_row));
+    k += sizeof(b.filter_min_row);
     memcpy(k, batch_scratch, sizeof(batch_scratch));
   }
   BatchEntry *e = nullptr;
@@ -1422,7 +1503,6 @@ enum MHCUDAResult mhcuda_calc_batch_device(const MinhashCudaGenerator *gen, uint
     gen->batches.push_back(std::move(ne));
     e = gen->batches.back().get();
   }
-  mhb::BatchArgs b{};
   b.base = base;
   b.mats = e->desc.as<mhb::BatchMatrix>();
   b.plan_base = reinterpret_cast<const uint32_t *>(e->desc.as<unsigned char>() + desc_bytes -
@@ -1431,14 +1511,10 @@ enum MHCUDAResult mhcuda_calc_batch_device(const MinhashCudaGenerator *gen, uint
   b.max_chunks = max_chunks;
   b.plan = gen->d_batch_plan.as<mhb::BatchPlan>();
   b.chunk_owner = gen->d_chunk_owner.as<uint32_t>();
-  b.target_items = resident_warps * static_cast<uint64_t>(waves);
-  b.want_items = resident_warps * 8;
-  HashPlan lp = vp;
-  lp.grid = static_cast<uint32_t>(static_cast<uint64_t>(gen->sm_count) * bps);
   const uint32_t pt = static_cast<uint32_t>(plan_threads);
   auto enqueue = [&]() -> MHCUDAResult {
     MHB_CHECK(gen, cudaMemsetAsync(base.status, 0, sizeof(uint32_t), st), mhcudaRuntimeError);
-    MHB_CHECK(gen, mhb::launch_batch(b, lp, pt, st), mhcudaRuntimeError);
+    MHB_CHECK(gen, mhb::launch_batch(b, vp, fp, pt, st), mhcudaRuntimeError);
     return mhcudaSuccess;
   };
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
@@ -1506,6 +1582,8 @@ enum MHCUDAResult mhcuda_autotune(const MinhashCudaGenerator *gen, const float *
     for (uint32_t minb : spl == 4 ? std::vector<uint32_t>{4u, 3u, 2u} : std::vector<uint32_t>{4u})
       for (uint32_t waves : {8u, 32u, 128u}) cands.push_back(TuneChoice{spl, minb, waves});
   }
+  if (gen->usable_bounds())
+    for (uint32_t waves : {8u, 32u, 128u}) cands.push_back(TuneChoice{4, 4, waves, true});
   cudaEvent_t e0 = nullptr, e1 = nullptr;
   MHB_CHECK(gen, cudaEventCreate(&e0), mhcudaRuntimeError);
   MHB_CHECK(gen, cudaEventCreate(&e1), mhcudaRuntimeError);
@@ -1543,7 +1621,7 @@ enum MHCUDAResult mhcuda_autotune(const MinhashCudaGenerator *gen, const float *
   double best_streamed_t = 1e300;
   for (size_t i = 0; i < times.size(); ++i) {
     const TuneChoice &c = cands[i];
-    if (c.spl == best.spl && c.minb == 4 && times[i] < best_streamed_t) {
+    if (c.filter == best.filter && c.spl == best.spl && c.minb == 4 && times[i] < best_streamed_t) {
       best_streamed_t = times[i];
       best_streamed = c;
     }

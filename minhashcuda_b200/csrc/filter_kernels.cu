@@ -1,0 +1,558 @@
+// Bound-filtered weighted-minhash kernels for sm_100a.
+//
+// The dense kernels (hash_kernels.cu) evaluate every (entry, sample) of a
+// row from 12 bytes of parameters, although only a sample's running minimum
+// matters.  These kernels read one byte per (entry, sample) and evaluate only
+// the entries that byte cannot rule out.
+//
+// With u = t - beta the evaluated value (kernel.cu:101-105 of
+// src-d/minhashcuda) is ln_a = ln_c - u*r - r, and t = floor(w/r + beta)
+// gives w - r < u*r <= w, so
+//     ln_c - r - w <= ln_a < ln_c - w.
+// ln_c - r depends on the table alone: the byte table `bounds` holds it
+// rounded down in steps of 1/20.  An entry is skipped when its bound minus w
+// is above a threshold that the sample's minimum does not exceed; the others
+// go through the dense kernels' evaluation in float32 with the exact quotient.
+// A skipped entry could not have replaced the minimum, so the hashes are the
+// dense kernels' bit for bit.
+//
+// The threshold is the sample's running minimum or, while that is higher, a
+// guess: a row's minimum of ln_a is distributed as ln(Exp(1) / sum of weights)
+// whatever the weights, so ln(kGuess / sum) is exceeded by one sample in
+// e^kGuess.  Samples that end above the guess are found at the end of the row
+// and scanned again without it (rescan).  With the generator's distributions
+// (r ~ Gamma(2), c ~ Gamma(2)) the share of entries whose c * e^-r lies below
+// x is x * (ln(1/x) + 0.42), which makes about 19 candidates per sample of a
+// 1400-entry row and 14 of a 200-entry one; with the running minimum alone
+// they are 29 and 17, and a row's first entries all pass.
+//
+// Rounding.  In float32 the computed ln_a may lie below the real
+// ln_c - r - w by at most 2^-24 * (6|w| + 5 r (1 + |beta|) + 3|ln_c|) (one
+// relative error of 2^-24 per operation; the quotient's and the sum's enter
+// through t <= RN(RN(w/r) + beta)).  |w| <= 104 for a finite nonzero float32
+// weight; with r <= 64, |beta| <= 2 and |ln_c| <= 64 that is below 2^-13, and
+// kBoundSlack = 2^-9 is subtracted before the bound is rounded down.  A
+// parameter outside those ranges (assigned tables; r = 0, NaN) or a bound
+// below the byte's range gets byte 0, which always passes.
+#include <algorithm>
+#include <cfloat>
+#include <cstdint>
+
+#include "hash_device.cuh"
+#include "wmh_internal.h"
+
+namespace mhb {
+namespace {
+
+// ---- Threshold arithmetic --------------------------------------------------
+// In units of 1/20 with everything rounded up: entry i passes for a sample
+// when byte <= m + l + 240, m = ceil(20 * threshold), l = ceil(20 * w_i).
+// Two samples share a register as 16-bit halves; the halves' signed sums are
+// formed by one 32-bit addition each because the biased total
+//     D = (0xC000 + byte) - (m + 241 + 16384) - l = 0x8000 + byte - T,
+//     T = m + l + 241,
+// stays within 16 bits; bit 15 of D is clear exactly when byte < T.
+
+constexpr int kLimit = 8191;  // |m|, |l| are clamped to it
+constexpr int kThrBias = 241 + 16384;
+constexpr uint32_t kThrOpen = kLimit + kThrBias;  // every entry passes
+constexpr float kGuess = 7.0f;
+// A threshold is kept within this of the row's guess (3 in ln_a).  The few
+// samples with a lower minimum let a few entries more pass; the lower end of
+// the byte's range (T >= 1) would otherwise be set for all samples by the one
+// with the least minimum.
+constexpr uint32_t kThrSpread = 60;
+
+// ceil(20 * x) clamped; 0.01 covers the product's rounding.
+__device__ __forceinline__ int quant_up(float x) {
+  return min(max(__float2int_ru(__fmaf_rn(x, kBoundScale, 0.01f)), -kLimit - 1), kLimit);
+}
+// Finite minima above 400 (no table of the generator's gives one) keep the
+// threshold open, so the upper clamp of m never hides a candidate.
+__device__ __forceinline__ uint32_t threshold(float mn) {
+  return static_cast<uint32_t>(quant_up(mn) + kThrBias);
+}
+
+// Minima as ordered keys: (monotone image of ln_a, position).  The smallest
+// key is the smallest ln_a and, among equal ones, the earliest position: the
+// first strict minimum of kernel.cu:106, in whatever order it is combined.
+__device__ __forceinline__ uint32_t ordered(float x) {
+  const uint32_t u = __float_as_uint(__fadd_rn(x, 0.0f));  // -0 -> +0: equal as floats
+  return u ^ (static_cast<uint32_t>(static_cast<int32_t>(u) >> 31) | 0x80000000u);
+}
+__device__ __forceinline__ float unordered(uint32_t k) {
+  return __uint_as_float(k ^ ((k >> 31) ? 0x80000000u : 0xFFFFFFFFu));
+}
+__device__ __forceinline__ unsigned long long make_key(float x, uint32_t pos) {
+  return static_cast<unsigned long long>(ordered(x)) << 32 | pos;
+}
+
+// ln_a of one (entry, sample), kernel.cu:101-105.
+__device__ __forceinline__ float exact_ln_a(float w, float r, float c, float b) {
+  const float t = exact_t(w, r, b);
+  return __fsub_rn(__fmaf_rn(-__fsub_rn(t, b), r, c), r);
+}
+
+// The sign bits of the four halves of (d0, d1), each spread over a byte (prmt
+// with the replicate-sign bit of its selectors, which __byte_perm masks off).
+__device__ __forceinline__ uint32_t half_signs(uint32_t d0, uint32_t d1) {
+  uint32_t r;
+  asm("prmt.b32 %0, %1, %2, 0xFDB9;" : "=r"(r) : "r"(d0), "r"(d1));
+  return r;
+}
+
+#ifndef FB
+#define FB 5
+#endif
+constexpr int kFilterBlocks = FB;
+constexpr uint32_t kFWin = 128;    // CSR positions per staged window
+constexpr uint32_t kQueue = 1024;  // candidates a warp holds
+
+// One warp's shared memory; TILE samples per tile.
+template <uint32_t TILE>
+struct alignas(16) FilterStage {
+  WarpStageT<kFWin> st;
+  int32_t l[kFWin];              // l of the window's entries in both halves (l * 65537)
+  unsigned long long key[TILE];  // running minima of the tile's samples
+  uint16_t thr[TILE];            // their thresholds, m + kThrBias
+  uint16_t queue[kQueue];        // candidates: window position | sample << 8
+};
+
+// Inclusive prefix sum over the warp.
+__device__ __forceinline__ uint32_t warp_prefix(uint32_t x, uint32_t lane) {
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, x, o);
+    x += lane >= static_cast<uint32_t>(o) ? y : 0u;
+  }
+  return x;
+}
+
+// One (chunk c, sample tile) item, as hash_item of the dense kernels: the
+// rows inside chunk c are finished, partial minima of the rows that cross its
+// ends are left for the finalize pass.  Chunks begin at a row where one
+// starts soon enough (chunk_begin).
+//
+// LN lanes hold 16 samples each of one entry, so a tile is 16 * LN samples
+// and one warp load fetches the bytes of 32 / LN entries (16 per lane).  A
+// batch is 8 such loads, kept four ahead; its candidates go to a queue in
+// shared memory.  The queue is evaluated and the thresholds are updated at the
+// end of a window of 128 entries, four candidates per lane at a time so that
+// their parameter gathers overlap.
+template <int LN, int SPAD, bool PACKED>
+__device__ __forceinline__ bool filter_item(const HashArgs &a, uint32_t c, uint32_t tile,
+                                            WarpCtxT<kFWin> &wc, FilterStage<16 * LN> &fs) {
+  constexpr uint32_t TILE = 16 * LN;
+  constexpr uint32_t GRP = 8 * (32 / LN);  // entries per batch
+  const uint32_t lane = wc.lane;
+  const uint32_t sub8 = lane / LN * 8;     // the lane's eight entries of a batch
+  const uint32_t sl = lane % LN * 16;      // and its samples in the tile
+  WarpStageT<kFWin> &stg = fs.st;
+  uint32_t &parity = wc.parity;
+  const uint32_t base = a.indptr[0];
+  const uint32_t spad = SPAD ? static_cast<uint32_t>(SPAD) : a.s_pad;
+  const uint32_t bstride = SPAD ? bound_stride(SPAD) : a.b_stride;
+  const uintptr_t col_addr =
+      PACKED ? (reinterpret_cast<uintptr_t>(a.cols_lo) | reinterpret_cast<uintptr_t>(a.cols_hi))
+             : reinterpret_cast<uintptr_t>(a.cols);
+  const bool bulk_ok =
+      !a.host_csr && ((reinterpret_cast<uintptr_t>(a.weights) | col_addr) & 15u) == 0;
+  const uint32_t t0 = tile * TILE;         // first sample of the tile
+  const uint32_t width = min(TILE, a.samples - t0);  // samples of the tile that exist
+  // Lanes past the last sample read the tile's first bytes; their candidate
+  // bits are masked off.
+  const uint8_t *__restrict__ qbase = a.bounds + t0 + (t0 + sl < bstride ? sl : 0);
+  const float *__restrict__ ptile = a.params + param_index(t0);
+
+  const uint32_t cs = chunk_begin(a, c, base);
+  const uint32_t ce = chunk_begin(a, c + 1, base);
+  uint32_t r_next = a.chunk_row[c];
+  const uint32_t r_stop = (c + 1 < a.nchunks) ? a.chunk_row[c + 1] : a.rows;
+  uint32_t row = kNone, row_end = cs, row_begin = cs;  // row_begin: its first position in the chunk
+  bool head = false, fresh = true;  // fresh: none of the row's entries has been looked at
+  if (r_next > 0) {
+    const uint32_t e = a.indptr[r_next] - base;
+    if (e > cs) {
+      row = r_next - 1;
+      row_end = e;
+      head = true;
+    }
+  }
+  uint32_t thr[8];         // thresholds of the lane's 16 samples, two per register
+  uint32_t thr_min = 0;    // the least of the tile's
+  uint32_t thr_guess = kThrOpen, thr_floor = 0;
+  bool guessing = true;
+
+  // Thresholds from the keys, to shared memory and to the lanes that use them.
+  auto refresh = [&]() {
+    uint32_t least = kThrOpen;
+#pragma unroll
+    for (uint32_t v = 0; v < TILE / 32; ++v) {
+      const uint32_t hi = static_cast<uint32_t>(fs.key[v * 32 + lane] >> 32);
+      const uint32_t t = max(min(thr_guess, threshold(unordered(hi))), thr_floor);
+      fs.thr[v * 32 + lane] = static_cast<uint16_t>(t);
+      least = min(least, t);
+    }
+    thr_min = __reduce_min_sync(0xFFFFFFFFu, least);
+    __syncwarp();
+    const uint4 x = *reinterpret_cast<const uint4 *>(&fs.thr[sl]);
+    const uint4 y = *reinterpret_cast<const uint4 *>(&fs.thr[sl + 8]);
+    thr[0] = x.x; thr[1] = x.y; thr[2] = x.z; thr[3] = x.w;
+    thr[4] = y.x; thr[5] = y.y; thr[6] = y.z; thr[7] = y.w;
+  };
+
+  // Scans the row's entries [row_begin, end) again for every sample whose
+  // minimum is above the guess, one sample at a time, lanes over entries.
+  auto rescan = [&](uint32_t end) {
+    uint32_t failed = 0;
+    for (uint32_t s1 = 0; s1 < width; s1 += 32) {
+      const bool above =
+          s1 + lane < width &&
+          threshold(unordered(static_cast<uint32_t>(fs.key[s1 + lane] >> 32))) > thr_guess;
+      uint32_t todo = __ballot_sync(0xFFFFFFFFu, above);
+      while (todo) {
+        const uint32_t s = s1 + __ffs(todo) - 1;
+        todo &= todo - 1;
+        ++failed;
+        unsigned long long best = fs.key[s];
+        for (uint32_t p = row_begin + lane; p < end; p += 32) {
+          uint32_t col = PACKED ? packed_col(a, p) : a.cols[p];
+          if (col >= a.dim) col = 0;
+          const float w = logf(a.weights[p]);
+          const uint32_t byte = a.bounds[static_cast<size_t>(col) * bstride + t0 + s];
+          const int m = quant_up(unordered(static_cast<uint32_t>(best >> 32)));
+          if (static_cast<int>(byte) > max(m + quant_up(w) + 240, 0)) continue;
+          const float *p3 = ptile + static_cast<size_t>(col) * 3 * spad + param_index(s);
+          const float x = exact_ln_a(w, __ldg(p3), __ldg(p3 + 2), __ldg(p3 + 4));
+          if (x < FLT_MAX) best = min(best, make_key(x, p));
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1)
+          best = min(best, __shfl_xor_sync(0xFFFFFFFFu, best, o));
+        __syncwarp();
+        if (lane == 0) fs.key[s] = best;
+      }
+    }
+    // A table of other distributions, for which the guess does not hold.
+    if (failed > TILE / 8) guessing = false;
+    __syncwarp();
+  };
+
+  // Leaves the row that ends (in this chunk) at `end`.
+  auto flush = [&](uint32_t end) {
+    if (row == kNone) return;
+    if (!fresh) rescan(end);
+    const bool partial = head || row_end > ce;
+    for (uint32_t s = lane; s < width; s += 32) {
+      const unsigned long long k = fresh ? make_key(FLT_MAX, kNone) : fs.key[s];
+      const uint32_t pos = static_cast<uint32_t>(k);
+      if (partial) {
+        const size_t off = static_cast<size_t>(2 * c + (head ? 0 : 1)) * spad + t0 + s;
+        a.part_ln[off] = unordered(static_cast<uint32_t>(k >> 32));
+        a.part_kt[off] = make_uint2(pos, 0u);
+      } else {
+        reinterpret_cast<uint2 *>(a.out)[static_cast<size_t>(row) * a.samples + t0 + s] =
+            resolve(a, pos, t0 + s);
+      }
+    }
+    __syncwarp();
+  };
+
+  // Windows start at multiples of 32 positions (16-byte aligned bulk copies
+  // of every array), the first one possibly before the chunk.
+  const uint32_t w0 = cs & ~31u;
+  const uint32_t nwin = ce > cs ? (ce - w0 + kFWin - 1) / kFWin : 0;
+  if (nwin > 0) issue_window<PACKED>(a, stg, wc.pk, 0, w0, min(kFWin, ce - w0), bulk_ok, lane);
+  if (nwin > 1)
+    issue_window<PACKED>(a, stg, wc.pk, 1, w0 + kFWin, min(kFWin, ce - w0 - kFWin), bulk_ok, lane);
+  auto drain_copies = [&](uint32_t from) {
+    for (uint32_t kk = from; kk < nwin && kk < from + 2; ++kk) {
+      const uint32_t bb = kk & 1u;
+      for (uint32_t spins = 0; !mbar_try_wait(&stg.bar[bb], (parity >> bb) & 1u);)
+        if (++spins > kSpinLimit) break;
+      parity ^= 1u << bb;
+    }
+  };
+
+  for (uint32_t k = 0; k < nwin; ++k) {
+    const uint32_t b = k & 1u;
+    const uint32_t ws = w0 + k * kFWin;
+    const uint32_t n = min(kFWin, ce - ws);
+    if (!finish_window<PACKED>(a, stg, wc.pk, b, (parity >> b) & 1u, ws, n, bulk_ok, lane)) {
+      if (lane == 0) atomicOr(a.status, kStatusStall);
+      drain_copies(k);
+      return false;
+    }
+    parity ^= 1u << b;
+    const float *__restrict__ lw = stg.w[b];
+    uint32_t *__restrict__ cl = stg.c[b];
+    for (uint32_t i = lane; i < n; i += 32) fs.l[i] = quant_up(lw[i]) * 65537;
+    // Entries past the window's end in its last batch: column 0, masked off.
+    for (uint32_t i = n + lane; i < ((n + GRP - 1) & ~(GRP - 1)); i += 32) cl[i] = 0;
+    __syncwarp();
+
+    // Evaluates the queued candidates, four per lane at a time.
+    uint32_t count = 0;
+    auto evaluate = [&]() {
+      for (uint32_t at = 0; at < count; at += 128) {
+        uint32_t e[4];
+        float r[4], lc[4], be[4];
+#pragma unroll
+        for (uint32_t j = 0; j < 4; ++j) {
+          // Lanes past the end repeat the last candidate: the same key again.
+          e[j] = fs.queue[min(at + 32 * j + lane, count - 1)];
+          const float *p = ptile + static_cast<size_t>(cl[e[j] & 0xFFu]) * 3 * spad + param_index(e[j] >> 8);
+          r[j] = __ldg(p);
+          lc[j] = __ldg(p + 2);
+          be[j] = __ldg(p + 4);
+        }
+#pragma unroll
+        for (uint32_t j = 0; j < 4; ++j) {
+          const uint32_t i = e[j] & 0xFFu;
+          const float x = exact_ln_a(lw[i], r[j], lc[j], be[j]);
+          if (at + 32 * j + lane < count && x < FLT_MAX) atomicMin(&fs.key[e[j] >> 8], make_key(x, ws + i));
+        }
+      }
+      count = 0;
+      __syncwarp();
+    };
+
+    uint32_t i = k == 0 ? cs - w0 : 0;
+    while (i < n) {
+      while (ws + i >= row_end) {
+        flush(row_end);
+        if (r_next >= r_stop) {  // only reachable with inconsistent offsets
+          if (lane == 0) atomicOr(a.status, kStatusBadIndptr);
+          drain_copies(k + 1);
+          return false;
+        }
+        row = r_next++;
+        row_begin = row_end;
+        row_end = a.indptr[row + 1] - base;
+        head = false;
+        fresh = true;
+      }
+      const uint32_t seg = min(row_end - ws, n);
+      if (fresh) {
+        // First look at the row: no minima yet, thresholds at the guess.
+        fresh = false;
+        thr_guess = kThrOpen;
+        thr_floor = 0;
+        if (guessing) {
+          float sum = 0.0f;
+          const uint32_t end = min(row_end, ce);
+#pragma unroll 8
+          for (uint32_t p = row_begin + lane; p < end; p += 32) sum += fmaxf(a.weights[p], 0.0f);
+#pragma unroll
+          for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xFFFFFFFFu, sum, o);
+          if (sum > 0.0f && sum < FLT_MAX) {
+            thr_guess = threshold(__logf(kGuess / sum));
+            thr_floor = thr_guess - kThrSpread;
+          }
+        }
+        thr_min = thr_guess;
+#pragma unroll
+        for (int v = 0; v < 8; ++v) thr[v] = thr_guess * 65537u;
+#pragma unroll
+        for (uint32_t v = 0; v < TILE / 32; ++v) fs.key[v * 32 + lane] = make_key(FLT_MAX, kNone);
+        __syncwarp();
+      }
+      uint32_t g = i & ~(GRP - 1);
+      uint4 q[4];
+      auto load = [&](uint32_t col) {
+        return __ldg(reinterpret_cast<const uint4 *>(qbase + static_cast<size_t>(col) * bstride));
+      };
+      auto load4 = [&](uint32_t at) {
+        const uint4 cc = *reinterpret_cast<const uint4 *>(&cl[at]);
+        q[0] = load(cc.x); q[1] = load(cc.y); q[2] = load(cc.z); q[3] = load(cc.w);
+      };
+      load4(g + sub8);
+      while (g < seg) {
+        const uint32_t h = g + sub8;
+        const int32_t l_lo = (1 + 16384 - static_cast<int32_t>(thr_min)) * 65537;
+        uint32_t miss[4] = {0, 0, 0, 0};  // byte j of [v], bit x: entry h + x cannot win 4v + j
+#pragma unroll
+        for (int y = 0; y < 2; ++y) {
+          const int4 l4 = *reinterpret_cast<const int4 *>(&fs.l[h + 4 * y]);
+          const int32_t ll[4] = {l4.x, l4.y, l4.z, l4.w};
+          // The loads four entries ahead; the last batch's repeat its own.
+          const uint32_t next = y == 0 ? h + 4 : g + GRP < seg ? h + GRP : h;
+          const uint4 c4 = *reinterpret_cast<const uint4 *>(&cl[next]);
+          const uint32_t cc[4] = {c4.x, c4.y, c4.z, c4.w};
+#pragma unroll
+          for (int x = 0; x < 4; ++x) {
+            // l is kept above the value at which some T would drop below 1.
+            const uint32_t l = static_cast<uint32_t>(max(ll[x], l_lo));
+            const uint32_t qq[4] = {q[x].x, q[x].y, q[x].z, q[x].w};
+#pragma unroll
+            for (int v = 0; v < 4; ++v) {
+              const uint32_t d0 = __byte_perm(qq[v], 0xC0C0C0C0u, 0x4140) - thr[2 * v] - l;
+              const uint32_t d1 = __byte_perm(qq[v], 0xC0C0C0C0u, 0x4342) - thr[2 * v + 1] - l;
+              miss[v] |= half_signs(d0, d1) & (0x01010101u << (4 * y + x));
+            }
+            q[x] = load(cc[x]);
+          }
+        }
+        uint32_t in_row = 0xFFFFFFFFu;  // entries of the row
+        if (g < i || g + GRP > seg) {
+          const uint32_t up = min(max(static_cast<int>(seg) - static_cast<int>(h), 0), 8);
+          const uint32_t lo = min(max(static_cast<int>(i) - static_cast<int>(h), 0), 8);
+          in_row = (((1u << up) - 1u) & ~((1u << lo) - 1u)) * 0x01010101u;
+        }
+        uint32_t hits[4];
+#pragma unroll
+        for (int v = 0; v < 4; ++v) {
+          hits[v] = ~miss[v] & in_row;
+          if (SPAD == 0 || (SPAD % TILE) != 0 || a.samples != spad) {  // samples that do not exist
+            const int left = static_cast<int>(width) - static_cast<int>(sl + 4 * v);
+            hits[v] &= left >= 4 ? 0xFFFFFFFFu : left <= 0 ? 0u : (1u << (8 * left)) - 1u;
+          }
+        }
+        auto push = [&](uint32_t m, uint32_t v, uint32_t at) {
+          while (m) {
+            const uint32_t bit = __ffs(m) - 1;
+            m &= m - 1;
+            fs.queue[at++] =
+                static_cast<uint16_t>((h + (bit & 7u)) | (sl + 4 * v + (bit >> 3)) << 8);
+          }
+          return at;
+        };
+        const uint32_t mine =
+            __popc(hits[0]) + __popc(hits[1]) + __popc(hits[2]) + __popc(hits[3]);
+        const uint32_t incl = warp_prefix(mine, lane);
+        const uint32_t total = __shfl_sync(0xFFFFFFFFu, incl, 31);
+        if (count + total <= kQueue) {
+          uint32_t at = count + incl - mine;
+#pragma unroll
+          for (uint32_t v = 0; v < 4; ++v) at = push(hits[v], v, at);
+          count += total;
+        } else {
+          // More than the queue has room for: by quarters of at most 1024.
+#pragma unroll 1
+          for (uint32_t v = 0; v < 4; ++v) {
+            const uint32_t m = v == 0 ? hits[0] : v == 1 ? hits[1] : v == 2 ? hits[2] : hits[3];
+            const uint32_t in2 = warp_prefix(__popc(m), lane);
+            const uint32_t sum2 = __shfl_sync(0xFFFFFFFFu, in2, 31);
+            if (count + sum2 > kQueue) {
+              __syncwarp();
+              evaluate();
+            }
+            push(m, v, count + in2 - __popc(m));
+            count += sum2;
+          }
+        }
+        g += GRP;
+      }
+      __syncwarp();
+      evaluate();
+      if (ws + seg < row_end) refresh();  // the row goes on
+      i = seg;
+    }
+    if (k + 2 < nwin) {
+      const uint32_t ws2 = ws + 2 * kFWin;
+      issue_window<PACKED>(a, stg, wc.pk, b, ws2, min(kFWin, ce - ws2), bulk_ok, lane);
+    }
+  }
+  flush(min(row_end, ce));
+  while (r_next < r_stop) {  // trailing empty rows of the last chunk
+    row = r_next++;
+    row_end = ce;
+    head = false;
+    fresh = true;
+    flush(ce);
+  }
+  return true;
+}
+
+template <int LN, int SPAD, bool PACKED>
+__global__ void __launch_bounds__(kFilterBlock, kFilterBlocks) filter_kernel(const HashArgs a) {
+  __shared__ FilterStage<16 * LN> stage_all[kFilterBlock / 32];
+  PackedStageT<kFWin> *packed = nullptr;
+  if constexpr (PACKED) {
+    __shared__ PackedStageT<kFWin> packed_stage[kFilterBlock / 32];
+    packed = &packed_stage[threadIdx.x >> 5];
+  }
+  if (*a.status & kStatusBadIndptr) return;
+  FilterStage<16 * LN> &fs = stage_all[threadIdx.x >> 5];
+  WarpCtxT<kFWin> wc;
+  warp_ctx_init(wc, &fs.st, packed);
+  const uint32_t gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const uint32_t nw = (gridDim.x * blockDim.x) >> 5;
+  const uint32_t items = a.nchunks * a.ntiles;
+  for (uint32_t item = gw; item < items; item += nw) {
+    const uint32_t c = item / a.ntiles;
+    if (!filter_item<LN, SPAD, PACKED>(a, c, item - c * a.ntiles, wc, fs)) return;
+  }
+}
+
+template <int LN, int SPAD>
+__global__ void __launch_bounds__(kFilterBlock, kFilterBlocks) filter_batch_kernel(const BatchArgs b) {
+  __shared__ FilterStage<16 * LN> stage_all[kFilterBlock / 32];
+  __shared__ HashArgs views[kFilterBlock / 32];
+  if ((*b.base.status & kStatusBadIndptr) || !b.plan->filter) return;
+  FilterStage<16 * LN> &fs = stage_all[threadIdx.x >> 5];
+  WarpCtxT<kFWin> wc;
+  warp_ctx_init(wc, &fs.st);
+  HashArgs &view = views[threadIdx.x >> 5];
+  const uint32_t gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const uint32_t nw = (gridDim.x * blockDim.x) >> 5;
+  const uint32_t ntiles = b.ntiles[1];
+  const uint32_t chunk = b.plan->chunk;
+  const uint32_t items = b.plan->nchunks * ntiles;
+  for (uint32_t item = gw; item < items; item += nw) {
+    const uint32_t gc = item / ntiles;
+    const uint32_t m = b.chunk_owner[gc];
+    const uint32_t base = b.mats[m].chunk_base;
+    __syncwarp();
+    if (wc.lane == 0) view = matrix_view(b, b.mats[m], chunk);
+    __syncwarp();
+    if (!filter_item<LN, SPAD, false>(view, gc - base, item - gc * ntiles, wc, fs)) return;
+  }
+}
+
+using FilterFn = void (*)(const HashArgs);
+using FilterBatchFn = void (*)(const BatchArgs);
+
+FilterFn pick_filter(uint32_t s_pad, bool packed) {
+  if (s_pad == 128) return packed ? filter_kernel<8, 128, true> : filter_kernel<8, 128, false>;
+  if (s_pad == 256) return packed ? filter_kernel<8, 256, true> : filter_kernel<8, 256, false>;
+  switch (filter_lanes(s_pad)) {
+    case 8: return packed ? filter_kernel<8, 0, true> : filter_kernel<8, 0, false>;
+    case 4: return packed ? filter_kernel<4, 0, true> : filter_kernel<4, 0, false>;
+    default: return packed ? filter_kernel<2, 0, true> : filter_kernel<2, 0, false>;
+  }
+}
+
+FilterBatchFn pick_filter_batch(uint32_t s_pad) {
+  if (s_pad == 128) return filter_batch_kernel<8, 128>;
+  if (s_pad == 256) return filter_batch_kernel<8, 256>;
+  switch (filter_lanes(s_pad)) {
+    case 8: return filter_batch_kernel<8, 0>;
+    case 4: return filter_batch_kernel<4, 0>;
+    default: return filter_batch_kernel<2, 0>;
+  }
+}
+
+}  // namespace
+
+cudaError_t launch_filter(const HashArgs &a, const HashPlan &plan, cudaStream_t stream) {
+  pick_filter(a.s_pad, a.col_hi_bits != 0)<<<plan.grid, kFilterBlock, 0, stream>>>(a);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_filter_batch(const BatchArgs &b, const HashPlan &plan, cudaStream_t stream) {
+  pick_filter_batch(b.base.s_pad)<<<plan.grid, kFilterBlock, 0, stream>>>(b);
+  return cudaGetLastError();
+}
+
+int filter_blocks_per_sm(uint32_t s_pad) {
+  int n = 0;
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, pick_filter(s_pad, false), kFilterBlock, 0) !=
+      cudaSuccess) {
+    cudaGetLastError();
+    return 1;
+  }
+  return n > 0 ? n : 1;
+}
+
+}  // namespace mhb

@@ -35,93 +35,11 @@
 #include <cstdint>
 #include <cstdlib>
 
+#include "hash_device.cuh"
 #include "wmh_internal.h"
 
 namespace mhb {
 namespace {
-
-template <int SPL>
-struct Lanes {
-  float v[SPL];
-  __device__ __forceinline__ void load(const float *__restrict__ p) {
-    if constexpr (SPL == 4) {
-      const float4 x = __ldg(reinterpret_cast<const float4 *>(p));
-      v[0] = x.x; v[1] = x.y; v[2] = x.z; v[3] = x.w;
-    } else if constexpr (SPL == 2) {
-      const float2 x = __ldg(reinterpret_cast<const float2 *>(p));
-      v[0] = x.x; v[1] = x.y;
-    } else {
-      v[0] = __ldg(p);
-    }
-  }
-};
-
-// t of kernel.cu:103 exactly as the reference computes it: IEEE quotient,
-// rounded sum, floor.
-__device__ __forceinline__ float exact_t(float w, float r, float b) {
-  return floorf(__fadd_rn(__fdiv_rn(w, r), b));
-}
-
-// Margin of the fast t below, relative to |w/r| + |beta| + 1.
-constexpr float kTMargin = 0x1p-18f;
-
-// Fast t.  Only floor(v) with v = RN(RN(w/r) + beta) is needed, and it only
-// depends on the exact quotient when v lies close to an integer.  With
-// y = rcp.approx(r) (documented error 1 ulp; 2^-22 relative assumed) and
-// va = RN(RN(w*y) + beta):
-//   |va - v| <= |w/r| * 2^-20.6 + |beta| * 2^-23 < m,
-//   m = (|w*y| + |beta| + 1) * 2^-18,
-// so when va is more than m away from every integer, floor(va) = floor(v).
-// Returns false (t undecided) otherwise, and for every non-finite or
-// flushed case (w = +-inf/NaN, r = 0/denormal/huge, |va| >= 2^22: m >= 16).
-__device__ __forceinline__ bool fast_t(float w, float r, float b, float &t) {
-  float y;
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(r));
-  const float qa = __fmul_rn(w, y);
-  const float va = __fadd_rn(qa, b);
-  t = floorf(va);
-  const float f = __fsub_rn(va, t);  // exact for |va| >= 1; 1.0 or exact for va in (-1, 1)
-  const float m = __fmaf_rn(__fadd_rn(fabsf(qa), fabsf(b)), kTMargin, kTMargin);
-  return fabsf(__fsub_rn(f, 0.5f)) < __fsub_rn(0.5f, m);  // NaN -> false
-}
-
-// One (nnz, sample) evaluation, kernel.cu:101-109, given t: keeps the
-// minimum and the position `p` it came from.
-__device__ __forceinline__ void wmh_update(float t, float r, float c, float b, uint32_t p,
-                                           float &mn, uint32_t &pos) {
-  const float tb = __fsub_rn(t, b);
-  const float ln_a = __fsub_rn(__fmaf_rn(-tb, r, c), r);
-  const bool lt = ln_a < mn;
-  mn = lt ? ln_a : mn;
-  pos = lt ? p : pos;
-}
-
-// Column of relative position p in a packed CSR.
-__device__ __forceinline__ uint32_t packed_col(const HashArgs &a, uint32_t p) {
-  const uint32_t h = a.col_hi_bits == 4 ? (a.cols_hi[p >> 1] >> ((p & 1u) * 4)) & 15u
-                                        : a.cols_hi[p];
-  return static_cast<uint32_t>(a.cols_lo[p]) | (h << 16);
-}
-
-// The output pair of kernel.cu:108 for sample s whose minimum came from the
-// entry at relative position `pos`: k = cols[pos] and t recomputed from the
-// entry with the exact quotient.  Every evaluation used that same t (fast_t
-// only decides t when it equals the exact one), so tracking the position
-// instead of (k, t) changes nothing but the work per evaluation.
-// (uint32)(int32)t as kernel.cu:108; the GPU conversion saturates.
-// A position outside [0, nnz) (none found, or a partial that a failed launch
-// left unwritten) yields kNone and reads nothing.
-__device__ __forceinline__ uint2 resolve(const HashArgs &a, uint32_t pos, uint32_t s) {
-  if (pos >= a.nnz) return make_uint2(kNone, kNone);
-  const uint32_t k = a.col_hi_bits ? packed_col(a, pos) : a.cols[pos];
-  // An invalid column was evaluated as column 0 and failed the call: keep
-  // the parameter reads in bounds.
-  if (k >= a.dim) return make_uint2(kNone, kNone);
-  const float w = logf(a.weights[pos]);
-  const float *col = a.params + static_cast<size_t>(k) * 3 * a.s_pad + s;
-  const float t = exact_t(w, col[0], col[2 * static_cast<size_t>(a.s_pad)]);
-  return make_uint2(k, static_cast<uint32_t>(static_cast<int32_t>(t)));
-}
 
 // chunk_row[c] = first row whose first position is >= c*chunk (rows if none),
 // for the chunks whose first owned row is row i (i == rows: the chunks past
@@ -152,340 +70,6 @@ __device__ __forceinline__ void plan_row(const HashArgs &a, uint32_t i) {
 __global__ void plan_kernel(const HashArgs a) {
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i <= a.rows) plan_row(a, i);
-}
-
-template <int SPL>
-struct RowState {
-  float mn[SPL];
-  uint32_t pos[SPL];  // relative position of the minimum, kNone if none
-  __device__ __forceinline__ void reset() {
-#pragma unroll
-    for (int j = 0; j < SPL; ++j) {
-      mn[j] = FLT_MAX;
-      pos[j] = kNone;
-    }
-  }
-};
-
-template <int SPL>
-__device__ __forceinline__ void store_final(const HashArgs &a, uint32_t row, uint32_t s0,
-                                            const RowState<SPL> &st) {
-  uint32_t *o = a.out + (static_cast<size_t>(row) * a.samples + s0) * 2;
-#pragma unroll
-  for (int j = 0; j < SPL; ++j) {
-    if (s0 + j < a.samples) *reinterpret_cast<uint2 *>(o + 2 * j) = resolve(a, st.pos[j], s0 + j);
-  }
-}
-
-template <int SPL>
-__device__ __forceinline__ void store_partial(const HashArgs &a, uint32_t slot, uint32_t s0,
-                                              const RowState<SPL> &st) {
-  const size_t off = static_cast<size_t>(slot) * a.s_pad + s0;
-#pragma unroll
-  for (int j = 0; j < SPL; ++j) {
-    a.part_ln[off + j] = st.mn[j];
-    a.part_kt[off + j] = make_uint2(st.pos[j], 0u);
-  }
-}
-
-// ---- TMA bulk staging of the CSR (per warp, double-buffered) -------------
-
-constexpr uint32_t kWin = 256;  // CSR positions per staged window
-constexpr uint32_t kSpinLimit = 1u << 22;
-
-// One warp's staging area: two windows of weights (turned into ln w in
-// place) and column indices, each with its own transaction barrier.  Column
-// slots n and n + 1 of a window of n positions hold column 0, so the loop may
-// prefetch two positions past the window without a bounds branch (the row stride of c,
-// kWin + 4 words, keeps both windows 16-byte aligned for the bulk copies).
-struct alignas(16) WarpStage {
-  float w[2][kWin];
-  uint32_t c[2][kWin + 4];
-  unsigned long long bar[2];
-};
-
-// Landing area of packed columns (HashArgs::col_hi_bits != 0): the low 16
-// bits and the high nibbles or bytes of each window's columns, rebuilt into
-// WarpStage::c by finish_window.
-struct alignas(16) PackedStage {
-  uint16_t lo[2][kWin];
-  uint8_t hi[2][kWin];
-};
-
-
-__device__ __forceinline__ uint32_t smem_addr(const void *p) {
-  return static_cast<uint32_t>(__cvta_generic_to_shared(p));
-}
-
-__device__ __forceinline__ void mbar_init(unsigned long long *bar, uint32_t count) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_addr(bar)), "r"(count)
-               : "memory");
-}
-
-__device__ __forceinline__ void mbar_arrive_expect_tx(unsigned long long *bar, uint32_t bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_addr(bar)),
-               "r"(bytes)
-               : "memory");
-}
-
-__device__ __forceinline__ void mbar_arrive(unsigned long long *bar) {
-  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_addr(bar)) : "memory");
-}
-
-__device__ __forceinline__ bool mbar_try_wait(unsigned long long *bar, uint32_t parity) {
-  uint32_t ok;
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-      "selp.u32 %0, 1, 0, p;\n\t}"
-      : "=r"(ok)
-      : "r"(smem_addr(bar)), "r"(parity)
-      : "memory");
-  return ok != 0;
-}
-
-// Global -> this CTA's shared memory, completion counted on `bar`.  Both
-// addresses 16-byte aligned, bytes a multiple of 16.  No multicast.
-__device__ __forceinline__ void bulk_copy_g2s(void *dst, const void *src, uint32_t bytes,
-                                              unsigned long long *bar) {
-  asm volatile(
-      "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-          smem_addr(dst)),
-      "l"(src), "r"(bytes), "r"(smem_addr(bar))
-      : "memory");
-}
-
-// Positions of a window that arrive by bulk copy: a multiple of 4 (16 bytes
-// of weights and of columns), or of 32 with packed columns (16 bytes of high
-// nibbles); window starts are multiples of 32.
-template <bool PACKED>
-__device__ __forceinline__ uint32_t bulk_positions(uint32_t n, bool bulk_ok) {
-  return bulk_ok ? (n & (PACKED ? ~31u : ~3u)) : 0u;
-}
-
-// Lane 0 starts the copy of positions [ws, ws + n) into buffer `b`: the
-// 16-byte-aligned body by bulk copies, the ragged tail is left to
-// finish_window's plain loads.
-template <bool PACKED>
-__device__ __forceinline__ void issue_window(const HashArgs &a, WarpStage &st, PackedStage *pk,
-                                             uint32_t b, uint32_t ws, uint32_t n, bool bulk_ok,
-                                             uint32_t lane) {
-  // Order this warp's earlier generic accesses of the buffer before the
-  // asynchronous writes that are about to land in it.
-  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-  __syncwarp();
-  if (lane == 0) {
-    const uint32_t nb = bulk_positions<PACKED>(n, bulk_ok);
-    if (nb) {
-      if constexpr (PACKED) {
-        const uint32_t hi_bytes = a.col_hi_bits == 4 ? nb / 2 : nb;
-        const uint32_t hi_off = a.col_hi_bits == 4 ? ws / 2 : ws;
-        mbar_arrive_expect_tx(&st.bar[b], 6u * nb + hi_bytes);
-        bulk_copy_g2s(st.w[b], a.weights + ws, 4u * nb, &st.bar[b]);
-        bulk_copy_g2s(pk->lo[b], a.cols_lo + ws, 2u * nb, &st.bar[b]);
-        bulk_copy_g2s(pk->hi[b], a.cols_hi + hi_off, hi_bytes, &st.bar[b]);
-      } else {
-        mbar_arrive_expect_tx(&st.bar[b], 8u * nb);
-        bulk_copy_g2s(st.w[b], a.weights + ws, 4u * nb, &st.bar[b]);
-        bulk_copy_g2s(st.c[b], a.cols + ws, 4u * nb, &st.bar[b]);
-      }
-    } else {
-      mbar_arrive(&st.bar[b]);
-    }
-  }
-}
-
-// Waits for buffer `b` (bounded), loads the tail, turns weights into
-// ln(weight) in place -- once per nnz, lane-parallel -- and validates the
-// columns: a column >= dim flags kStatusBadColumn (the call then fails, its
-// hashes are not valid output) and is replaced by column 0, so the
-// evaluation loop reads only in-bounds parameters without a check per nnz.
-// Returns false if the copy did not complete within the spin limit.
-template <bool PACKED>
-__device__ __forceinline__ bool finish_window(const HashArgs &a, WarpStage &st, PackedStage *pk,
-                                              uint32_t b, uint32_t parity, uint32_t ws,
-                                              uint32_t n, bool bulk_ok, uint32_t lane) {
-  uint32_t spins = 0;
-  while (!mbar_try_wait(&st.bar[b], parity)) {
-    if (++spins > kSpinLimit) return false;
-  }
-  const uint32_t nb = bulk_positions<PACKED>(n, bulk_ok);
-  bool bad = false;
-  for (uint32_t i = lane; i < n; i += 32) {
-    float x;
-    uint32_t col;
-    if constexpr (PACKED) {
-      if (i < nb) {
-        x = st.w[b][i];
-        const uint32_t h = a.col_hi_bits == 4 ? (pk->hi[b][i >> 1] >> ((i & 1u) * 4)) & 15u
-                                              : pk->hi[b][i];
-        col = static_cast<uint32_t>(pk->lo[b][i]) | (h << 16);
-      } else {
-        x = __ldg(a.weights + ws + i);
-        col = packed_col(a, ws + i);
-      }
-    } else if (i < nb) {
-      x = st.w[b][i];
-      col = st.c[b][i];
-    } else if (a.host_csr) {  // mapped host memory: plain loads
-      x = a.weights[ws + i];
-      col = a.cols[ws + i];
-    } else {
-      x = __ldg(a.weights + ws + i);
-      col = __ldg(a.cols + ws + i);
-    }
-    if (col >= a.dim) {
-      bad = true;
-      col = 0;
-    }
-    st.c[b][i] = col;
-    st.w[b][i] = logf(x);
-  }
-  if (__any_sync(0xFFFFFFFFu, bad) && lane == 0) atomicOr(a.status, kStatusBadColumn);
-  if (lane == 0) st.c[b][n] = st.c[b][n + 1] = 0;  // the prefetch slots past the window
-  __syncwarp();
-  return true;
-}
-
-template <int SPL>
-struct Params {
-  Lanes<SPL> r, c, b;
-  __device__ __forceinline__ void load(const float *__restrict__ col_base, uint32_t s_pad) {
-    r.load(col_base);
-    c.load(col_base + s_pad);
-    b.load(col_base + 2 * s_pad);
-  }
-};
-
-// ---- Packed pairs of float32 (sm_100 f32x2 arithmetic) --------------------
-// One add/sub/mul/fma.rn.f32x2 applies the IEEE round-to-nearest operation
-// to both halves independently, so a pair computes exactly what two
-// __fadd_rn / __fsub_rn / __fmul_rn / __fmaf_rn calls compute, in one issue.
-struct F2 {
-  unsigned long long v;
-};
-__device__ __forceinline__ F2 f2(float lo, float hi) {
-  F2 r;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(lo), "f"(hi));
-  return r;
-}
-__device__ __forceinline__ void split(F2 x, float &lo, float &hi) {
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(x.v));
-}
-__device__ __forceinline__ F2 add2(F2 a, F2 b) {
-  F2 r;
-  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
-  return r;
-}
-__device__ __forceinline__ F2 sub2(F2 a, F2 b) {
-  F2 r;
-  asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
-  return r;
-}
-__device__ __forceinline__ F2 mul2(F2 a, F2 b) {
-  F2 r;
-  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
-  return r;
-}
-__device__ __forceinline__ F2 fma2(F2 a, F2 b, F2 c) {
-  F2 r;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
-  return r;
-}
-
-// Selects for samples j and j+1 given their ln_a pair (position p).
-template <int SPL>
-__device__ __forceinline__ void update_pair(F2 ln_a, uint32_t p, int j, RowState<SPL> &st) {
-  float l0, l1;
-  split(ln_a, l0, l1);
-  const bool lt0 = l0 < st.mn[j], lt1 = l1 < st.mn[j + 1];
-  st.mn[j] = lt0 ? l0 : st.mn[j];
-  st.pos[j] = lt0 ? p : st.pos[j];
-  st.mn[j + 1] = lt1 ? l1 : st.mn[j + 1];
-  st.pos[j + 1] = lt1 ? p : st.pos[j + 1];
-}
-
-template <int SPL>
-__device__ __forceinline__ void eval_all(const Params<SPL> &p, float w, uint32_t pos, bool active,
-                                         RowState<SPL> &st) {
-  float t[SPL];
-  bool undecided = false;
-  if constexpr (SPL % 2 == 0) {
-    // fast_t on sample pairs.  The bound is fast_t's; the limit 0.5 - m is
-    // one fma, (|qa| + |b|) * -2^-18 + (0.5 - 2^-18), whose single rounding
-    // (<= 2^-26) is covered by the additive 2^-18 in m.
-    const F2 ww = f2(w, w);
-#pragma unroll
-    for (int j = 0; j < SPL; j += 2) {
-      float y0, y1;
-      asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y0) : "f"(p.r.v[j]));
-      asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y1) : "f"(p.r.v[j + 1]));
-      const F2 qa = mul2(ww, f2(y0, y1));
-      const F2 va = add2(qa, f2(p.b.v[j], p.b.v[j + 1]));
-      float q0, q1;
-      split(qa, q0, q1);
-      float v0, v1;
-      split(va, v0, v1);
-      t[j] = floorf(v0);
-      t[j + 1] = floorf(v1);
-      const F2 fr = sub2(va, f2(t[j], t[j + 1]));
-      const F2 s = f2(__fadd_rn(fabsf(q0), fabsf(p.b.v[j])),
-                      __fadd_rn(fabsf(q1), fabsf(p.b.v[j + 1])));
-      const F2 lim = fma2(s, f2(-kTMargin, -kTMargin), f2(0.5f - kTMargin, 0.5f - kTMargin));
-      const F2 dv = sub2(fr, f2(0.5f, 0.5f));
-      float d0, d1, l0, l1;
-      split(dv, d0, d1);
-      split(lim, l0, l1);
-      undecided |= !(fabsf(d0) < l0) || !(fabsf(d1) < l1);  // NaN -> undecided
-    }
-  } else {
-#pragma unroll
-    for (int j = 0; j < SPL; ++j) undecided |= !fast_t(w, p.r.v[j], p.b.v[j], t[j]);
-  }
-  // Rare: some lane's t sits within the margin of an integer; the warp takes
-  // the exact quotient for all its samples (warp-uniform branch).
-  if (__any_sync(0xFFFFFFFFu, undecided && active)) {
-#pragma unroll
-    for (int j = 0; j < SPL; ++j) t[j] = exact_t(w, p.r.v[j], p.b.v[j]);
-  }
-  if constexpr (SPL % 2 == 0) {
-    // ln_a = fma(-(t - beta), r, ln_c) - r on pairs; beta - t is -(t - beta)
-    // exactly (round-to-nearest is symmetric).
-#pragma unroll
-    for (int j = 0; j < SPL; j += 2) {
-      const F2 rr = f2(p.r.v[j], p.r.v[j + 1]);
-      const F2 nb = sub2(f2(p.b.v[j], p.b.v[j + 1]), f2(t[j], t[j + 1]));
-      const F2 ln_a = sub2(fma2(nb, rr, f2(p.c.v[j], p.c.v[j + 1])), rr);
-      update_pair<SPL>(ln_a, pos, j, st);
-    }
-  } else {
-#pragma unroll
-    for (int j = 0; j < SPL; ++j)
-      wmh_update(t[j], p.r.v[j], p.c.v[j], p.b.v[j], pos, st.mn[j], st.pos[j]);
-  }
-}
-
-// Per-warp state of the hash kernels: the staging buffers, their barrier
-// phases and the launch-wide constants of the item loop.
-struct WarpCtx {
-  WarpStage *stg;
-  PackedStage *pk;  // packed-column landing area (packed kernels only)
-  uint32_t parity;  // bit b: phase parity to wait for on buffer b
-  uint32_t lane;
-};
-
-__device__ __forceinline__ void warp_ctx_init(WarpCtx &w, WarpStage *stage_all,
-                                              PackedStage *packed_all = nullptr) {
-  w.lane = threadIdx.x & 31u;
-  w.stg = &stage_all[threadIdx.x >> 5];
-  w.pk = packed_all ? &packed_all[threadIdx.x >> 5] : nullptr;
-  if (w.lane == 0) {
-    mbar_init(&w.stg->bar[0], 1);
-    mbar_init(&w.stg->bar[1], 1);
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-  }
-  __syncwarp();
-  w.parity = 0;
 }
 
 // Parameter sets a warp keeps in registers for register budget MINB
@@ -529,7 +113,7 @@ __device__ __forceinline__ bool hash_item(const HashArgs &a, uint32_t c, uint32_
     const bool active = s0 < spad;
     // Lanes past the last sample read the tile's first samples (in bounds)
     // and never store, so parameter loads need no branch.
-    const float *__restrict__ pbase = a.params + (active ? s0 : tile * (32u * SPL));
+    const float *__restrict__ pbase = a.params + param_index(active ? s0 : tile * (32u * SPL));
     const uint32_t cs = c * a.chunk;
     const uint32_t ce = cs + min(a.chunk, a.nnz - cs);  // no uint32 overflow near 2^32
     uint32_t r_next = a.chunk_row[c];
@@ -597,8 +181,8 @@ __device__ __forceinline__ bool hash_item(const HashArgs &a, uint32_t c, uint32_
         // and B position i + 1; positions up to n + 1 read the zero column
         // slots past the window.
         Params<SPL> A, B, C;
-        A.load(pbase + cl[0] * col_stride, spad);
-        B.load(pbase + cl[1] * col_stride, spad);
+        A.load(pbase + cl[0] * col_stride);
+        B.load(pbase + cl[1] * col_stride);
         uint32_t i = 0;
         while (i < n) {
           while (ws + i >= row_end) {
@@ -615,26 +199,26 @@ __device__ __forceinline__ bool hash_item(const HashArgs &a, uint32_t c, uint32_
           }
           const uint32_t seg = min(row_end - ws, n);
           while (i + 3 <= seg) {  // prefetches reach i + 4 <= n + 1
-            C.load(pbase + cl[i + 2] * col_stride, spad);
+            C.load(pbase + cl[i + 2] * col_stride);
             eval_all<SPL>(A, lw[i], ws + i, active, st);
-            A.load(pbase + cl[i + 3] * col_stride, spad);
+            A.load(pbase + cl[i + 3] * col_stride);
             eval_all<SPL>(B, lw[i + 1], ws + i + 1, active, st);
-            B.load(pbase + cl[i + 4] * col_stride, spad);
+            B.load(pbase + cl[i + 4] * col_stride);
             eval_all<SPL>(C, lw[i + 2], ws + i + 2, active, st);
             i += 3;
           }
           if (i + 2 == seg) {
-            C.load(pbase + cl[i + 2] * col_stride, spad);
+            C.load(pbase + cl[i + 2] * col_stride);
             eval_all<SPL>(A, lw[i], ws + i, active, st);
             eval_all<SPL>(B, lw[i + 1], ws + i + 1, active, st);
             i += 2;
             A = C;
-            B.load(pbase + cl[i + 1] * col_stride, spad);
+            B.load(pbase + cl[i + 1] * col_stride);
           } else if (i + 1 == seg) {
             eval_all<SPL>(A, lw[i], ws + i, active, st);
             i += 1;
             A = B;
-            B.load(pbase + cl[i + 1] * col_stride, spad);
+            B.load(pbase + cl[i + 1] * col_stride);
           }
         }
         if (k + 2 < nwin) {
@@ -645,7 +229,7 @@ __device__ __forceinline__ bool hash_item(const HashArgs &a, uint32_t c, uint32_
       }
       Params<SPL> A, B;
       uint32_t dA = cl[0], dB = 0;
-      A.load(pbase + dA * col_stride, spad);
+      A.load(pbase + dA * col_stride);
       uint32_t i = 0;
       while (i < n) {
         // Row boundaries (warp-uniform): finish rows, start the next owned one.
@@ -666,16 +250,16 @@ __device__ __forceinline__ bool hash_item(const HashArgs &a, uint32_t c, uint32_
         // evaluated, A for i+2 while B is evaluated.
         while (i + 1 < seg) {  // i + 2 <= n
           dB = cl[i + 1];
-          B.load(pbase + dB * col_stride, spad);
+          B.load(pbase + dB * col_stride);
           eval_all<SPL>(A, lw[i], ws + i, active, st);
           dA = cl[i + 2];
-          A.load(pbase + dA * col_stride, spad);
+          A.load(pbase + dA * col_stride);
           eval_all<SPL>(B, lw[i + 1], ws + i + 1, active, st);
           i += 2;
         }
         if (i < seg) {  // i + 1 <= n
           dB = cl[i + 1];
-          B.load(pbase + dB * col_stride, spad);
+          B.load(pbase + dB * col_stride);
           eval_all<SPL>(A, lw[i], ws + i, active, st);
           ++i;
           A = B;
@@ -705,14 +289,14 @@ __device__ __forceinline__ bool hash_item(const HashArgs &a, uint32_t c, uint32_
 template <int SPL, int MINB, int SPAD, bool PACKED>
 __global__ void __launch_bounds__(kHashBlock, MINB) hash_kernel(const HashArgs a) {
   __shared__ WarpStage stage_all[kHashBlock / 32];
-  PackedStage *packed_all = nullptr;
+  PackedStage *packed = nullptr;
   if constexpr (PACKED) {
     __shared__ PackedStage packed_stage[kHashBlock / 32];
-    packed_all = packed_stage;
+    packed = &packed_stage[threadIdx.x >> 5];
   }
   if (*a.status & kStatusBadIndptr) return;
   WarpCtx wc;
-  warp_ctx_init(wc, stage_all, packed_all);
+  warp_ctx_init(wc, &stage_all[threadIdx.x >> 5], packed);
   const uint32_t gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const uint32_t nw = (gridDim.x * blockDim.x) >> 5;
   const uint32_t items = a.nchunks * a.ntiles;
@@ -739,9 +323,10 @@ __device__ __forceinline__ void finalize_item(const HashArgs &a, uint32_t c, uin
   if (r1 <= r0) return;
   const uint32_t row = r1 - 1;
   const uint32_t end = a.indptr[row + 1] - base;
-  const uint32_t ce = c * a.chunk + min(a.chunk, a.nnz - c * a.chunk);
+  const uint32_t ce = chunk_begin(a, c + 1, base);
   if (end <= ce || s >= a.samples) return;
-  const uint32_t c_last = (end - 1) / a.chunk;
+  uint32_t c_last = (end - 1) / a.chunk;
+  if (chunk_begin(a, c_last, base) >= end) --c_last;  // starts at the next row
   const size_t stride = 2 * static_cast<size_t>(a.s_pad);  // one chunk's two slots
   size_t off = static_cast<size_t>(2 * c + 1) * a.s_pad + s;
   float mn = a.part_ln[off];
@@ -799,24 +384,6 @@ __global__ void finalize_kernel(const HashArgs a) {
 // slice of the chunk table and partials the item then works on exactly as a
 // single-matrix launch would: results equal one launch per matrix bit for bit
 // (a row's arg-min and its ties do not depend on how positions are cut).
-
-// HashArgs of matrix m inside batch b.
-__device__ __forceinline__ HashArgs matrix_view(const BatchArgs &b, const BatchMatrix &m,
-                                                uint32_t chunk) {
-  HashArgs v = b.base;
-  v.weights = m.weights;
-  v.cols = m.cols;
-  v.indptr = m.indptr;
-  v.out = m.out;
-  v.rows = m.rows;
-  v.nnz = m.nnz;
-  v.chunk = chunk;
-  v.nchunks = m.nchunks;
-  v.chunk_row = b.base.chunk_row + m.chunk_base;
-  v.part_ln = b.base.part_ln + static_cast<size_t>(2) * m.chunk_base * b.base.s_pad;
-  v.part_kt = b.base.part_kt + static_cast<size_t>(2) * m.chunk_base * b.base.s_pad;
-  return v;
-}
 
 constexpr int kSetupThreads = 1024;
 
@@ -878,12 +445,18 @@ __global__ void __launch_bounds__(kSetupThreads) batch_setup_kernel(const BatchA
   block_exclusive_scan(nonempty, &total_nonempty);
   __shared__ uint32_t s_chunk;
   if (t == 0) {
-    const uint64_t ntiles = b.base.ntiles;
-    uint64_t chunk = (total_nnz * ntiles + b.target_items - 1) / b.target_items;
+    const uint32_t f = b.filter_min_row && total_nnz >= total_rows * b.filter_min_row &&
+                       total_nnz >= b.filter_min_nnz;
+    b.plan->filter = f;
+    const uint64_t ntiles = b.ntiles[f], target = b.target_items[f], want = b.want_items[f];
+    uint64_t chunk = (total_nnz * ntiles + target - 1) / target;
     const uint64_t avg_row = total_rows ? (total_nnz + total_rows - 1) / total_rows : 1;
     chunk = max(chunk, min(4 * avg_row, static_cast<uint64_t>(1024)));
-    chunk = min(chunk, max(static_cast<uint64_t>(64),
-                           (total_nnz * ntiles + b.want_items - 1) / b.want_items));
+    if (f) {  // as make_plan: a row in pieces starts its search anew in each
+      chunk = max(chunk, min(avg_row, static_cast<uint64_t>(4096)));
+    } else {
+      chunk = min(chunk, max(static_cast<uint64_t>(64), (total_nnz * ntiles + want - 1) / want));
+    }
     // sum over matrices of ceil(nnz_m / chunk) <= total_nnz / chunk + nonempty
     const uint64_t avail = b.max_chunks > total_nonempty ? b.max_chunks - total_nonempty : 1;
     chunk = max(chunk, (total_nnz + avail - 1) / avail);
@@ -949,13 +522,13 @@ template <int SPL, int MINB, int SPAD>
 __global__ void __launch_bounds__(kHashBlock, MINB) hash_batch_kernel(const BatchArgs b) {
   __shared__ WarpStage stage_all[kHashBlock / 32];
   __shared__ HashArgs views[kHashBlock / 32];
-  if (*b.base.status & kStatusBadIndptr) return;
+  if ((*b.base.status & kStatusBadIndptr) || b.plan->filter) return;
   WarpCtx wc;
-  warp_ctx_init(wc, stage_all);
+  warp_ctx_init(wc, &stage_all[threadIdx.x >> 5]);
   HashArgs &view = views[threadIdx.x >> 5];
   const uint32_t gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const uint32_t nw = (gridDim.x * blockDim.x) >> 5;
-  const uint32_t ntiles = b.base.ntiles;
+  const uint32_t ntiles = b.ntiles[0];
   const uint32_t chunk = b.plan->chunk;
   const uint32_t items = b.plan->nchunks * ntiles;
   for (uint32_t item = gw; item < items; item += nw) {
@@ -1075,6 +648,7 @@ HashFn pick_hash(uint32_t spl, uint32_t minb, uint32_t s_pad, bool packed = fals
 }  // namespace
 
 cudaError_t launch_hash(const HashArgs &a, const HashPlan &plan, cudaStream_t stream) {
+  if (plan.filter) return launch_filter(a, plan, stream);
   const HashFn fn = pick_hash(plan.spl, plan.minb, a.s_pad, a.col_hi_bits != 0);
   if (!fn) return cudaErrorInvalidValue;
   fn<<<plan.grid, kHashBlock, 0, stream>>>(a);
@@ -1090,14 +664,18 @@ cudaError_t launch_finalize(const HashArgs &a, cudaStream_t stream) {
   return cudaGetLastError();
 }
 
-cudaError_t launch_batch(const BatchArgs &b, const HashPlan &plan, uint32_t plan_threads,
-                         cudaStream_t stream) {
-  const BatchFn fn = pick_batch(plan.spl, plan.minb, b.base.s_pad);
+cudaError_t launch_batch(const BatchArgs &b, const HashPlan &dense, const HashPlan &filtered,
+                         uint32_t plan_threads, cudaStream_t stream) {
+  const BatchFn fn = pick_batch(dense.spl, dense.minb, b.base.s_pad);
   if (!fn || b.count == 0 || b.max_chunks == 0) return cudaErrorInvalidValue;
   batch_setup_kernel<<<1, kSetupThreads, 0, stream>>>(b);
   if (plan_threads)
     batch_plan_kernel<<<(plan_threads + 255) / 256, 256, 0, stream>>>(b, plan_threads);
-  fn<<<plan.grid, kHashBlock, 0, stream>>>(b);
+  if (b.filter_min_row) {
+    const cudaError_t e = launch_filter_batch(b, filtered, stream);
+    if (e != cudaSuccess) return e;
+  }
+  fn<<<dense.grid, kHashBlock, 0, stream>>>(b);
   const uint64_t stiles = (b.base.samples + 31) / 32;
   uint64_t blocks = (static_cast<uint64_t>(b.max_chunks) * stiles + 7) / 8;
   blocks = std::min<uint64_t>(std::max<uint64_t>(blocks, 1), 8192);
@@ -1113,6 +691,10 @@ int hash_blocks_per_sm(uint32_t spl, uint32_t minb, uint32_t s_pad) {
     return 1;
   }
   return n > 0 ? n : 1;
+}
+
+int plan_blocks_per_sm(const HashPlan &plan, uint32_t s_pad) {
+  return plan.filter ? filter_blocks_per_sm(s_pad) : hash_blocks_per_sm(plan.spl, plan.minb, s_pad);
 }
 
 size_t hash_kernel_registers(uint32_t spl, uint32_t minb, uint32_t s_pad) {

@@ -113,7 +113,7 @@ extern "C" enum MHCUDAResult mhcuda_calc_device_noalloc(
   char *scratch = static_cast<char *>(noalloc_scratch_on(g.device));
   if (!scratch) return mhcudaRuntimeError;
   const cudaStream_t st = stream ? static_cast<cudaStream_t>(stream) : g.stream;
-  const int bps = mhb::hash_blocks_per_sm(plan.spl, plan.minb, s_pad);
+  const int bps = mhb::plan_blocks_per_sm(plan, s_pad);
   const uint64_t items = static_cast<uint64_t>(plan.nchunks) * plan.ntiles;
   const uint64_t want = (items + mhb::kHashBlock / 32 - 1) / (mhb::kHashBlock / 32);
   plan.grid = static_cast<uint32_t>(
@@ -124,6 +124,9 @@ extern "C" enum MHCUDAResult mhcuda_calc_device_noalloc(
   a.dim = g.dim;
   a.samples = g.samples;
   a.s_pad = s_pad;
+  a.bounds = g.bounds;
+  a.b_stride = mhb::bound_stride(s_pad);
+  a.snap_rows = plan.filter;
   a.weights = d_weights;
   a.cols = d_cols;
   a.indptr = d_rows;

@@ -305,8 +305,8 @@ MHCUDAResult MinhashCudaServer_::run_units(Lane &lane, const std::vector<Unit> &
   // even when rows are long (the plain plan keeps a few rows per chunk);
   // several lanes' launches overlap, so two are enough.
   mhb::HashPlan plan = mhb::plan_for_generator(units.front().req->gen, N, R,
-                                               high ? min_items_high : min_items_low);
-  const int bps = mhb::hash_blocks_per_sm(plan.spl, plan.minb, s_pad);
+                                               high ? min_items_high : min_items_low, !zc);
+  const int bps = mhb::plan_blocks_per_sm(plan, s_pad);
   // Keep the chunk table and partials inside the lane's fixed scratch:
   // nchunks*4 <= unit, 2*nchunks*s_pad*4 <= 4*unit, 2*nchunks*s_pad*8 <= 8*unit.
   const uint64_t max_chunks = std::max<uint64_t>(
@@ -321,7 +321,8 @@ MHCUDAResult MinhashCudaServer_::run_units(Lane &lane, const std::vector<Unit> &
   // blocks retire often and high-priority blocks get their SMs.
   {
     const uint64_t items = static_cast<uint64_t>(plan.nchunks) * plan.ntiles;
-    const uint64_t blocks = (items + 7) / 8;
+    const uint32_t warps = mhb::plan_block_warps(plan);
+    const uint64_t blocks = (items + warps - 1) / warps;
     const uint64_t resident = static_cast<uint64_t>(sm_count) * bps;
     plan.grid = static_cast<uint32_t>(std::max<uint64_t>(
         1, high ? std::min(blocks, resident) : std::min<uint64_t>(blocks, 1u << 30)));
@@ -331,6 +332,9 @@ MHCUDAResult MinhashCudaServer_::run_units(Lane &lane, const std::vector<Unit> &
   a.dim = g.dim;
   a.samples = g.samples;
   a.s_pad = s_pad;
+  a.bounds = g.bounds;
+  a.b_stride = mhb::bound_stride(s_pad);
+  a.snap_rows = plan.filter;
   a.weights = zc ? lane.mw : lane.w;
   a.cols = zc ? lane.mc : lane.c;
   a.indptr = zc ? lane.mip : lane.ip;

@@ -42,14 +42,27 @@ struct HashPlan {
   uint32_t nchunks;  // >= 1
   uint32_t spl;      // samples per lane in one item: 1, 2 or 4
   uint32_t minb;     // kernel variant: minimum resident blocks per SM (4; 3 or 2 for spl 4)
-  uint32_t ntiles;   // sample tiles of 32*spl samples
+  uint32_t ntiles;   // sample tiles of 32*spl samples (filter: filter_tile(s_pad))
   uint32_t grid;     // persistent grid (blocks of kHashBlock threads)
+  uint32_t filter;   // bound-filtered kernel (filter_kernels.cu) instead of the dense one
 };
 
 constexpr int kHashBlock = 256;
+constexpr int kFilterBlock = 128;
+
+// Row stride in bytes of the bound table (one byte per sample): whole
+// 32-byte sectors.
+constexpr uint32_t bound_stride(uint32_t s_pad) { return (s_pad + 31) & ~31u; }
+// Sample counts the filter kernels serve: below 32 the dense kernels read no
+// more sectors per entry than the bounds would add.
+constexpr uint32_t kFilterMinSamples = 32;
+// Lanes the filter kernels give one entry (16 samples each), and their sample
+// tile.
+constexpr uint32_t filter_lanes(uint32_t s_pad) { return s_pad > 64 ? 8 : s_pad > 32 ? 4 : 2; }
+constexpr uint32_t filter_tile(uint32_t s_pad) { return 16 * filter_lanes(s_pad); }
 
 struct HashArgs {
-  const float *params;       // [dim][3][s_pad]
+  const float *params;       // [dim][s_pad / 2][r r c c b b], see param_index
   uint32_t dim;
   uint32_t samples;
   uint32_t s_pad;
@@ -74,6 +87,11 @@ struct HashArgs {
   const uint16_t *cols_lo;
   const uint8_t *cols_hi;
   uint32_t col_hi_bits;
+  // Lower bounds of ln_c - r ([dim][b_stride] bytes, filter_kernels.cu), or
+  // nullptr when the generator has none.
+  const uint8_t *bounds;
+  uint32_t b_stride;
+  uint32_t snap_rows;  // chunks begin at rows where possible (chunk_begin); filtered launches
 };
 
 // One matrix of a device-resident batch (mhcuda_calc_batch_device).  The
@@ -94,6 +112,7 @@ struct BatchMatrix {
 struct BatchPlan {
   uint32_t chunk;    // positions per chunk, the same for every matrix
   uint32_t nchunks;  // chunks of all matrices
+  uint32_t filter;   // the bound-filtered launch does the work, not the dense one
 };
 
 struct BatchArgs {
@@ -105,8 +124,15 @@ struct BatchArgs {
   uint32_t max_chunks;    // chunk slots the scratch holds
   BatchPlan *plan;
   uint32_t *chunk_owner;  // [max_chunks] matrix of each batch chunk
-  uint64_t target_items;  // warp items to aim for (resident warps x waves)
-  uint64_t want_items;    // items per launch below which chunks shrink (resident warps x 8)
+  // [0] the dense kernel, [1] the filtered one:
+  uint64_t target_items[2];  // warp items to aim for (resident warps x waves)
+  uint64_t want_items[2];    // items per launch below which chunks shrink (resident warps x 8)
+  uint32_t ntiles[2];
+  // A batch is filtered when its mean row has this many entries and its
+  // entries reach filter_min_nnz; 0: never (then only the dense kernel is
+  // launched).
+  uint32_t filter_min_row;
+  uint64_t filter_min_nnz;
 };
 
 // Launchers (hash_kernels.cu).  All enqueue on `stream` and return the launch
@@ -116,22 +142,42 @@ cudaError_t launch_hash(const HashArgs &a, const HashPlan &plan, cudaStream_t st
 cudaError_t launch_finalize(const HashArgs &a, cudaStream_t stream);
 // A whole device-resident batch: setup (per-matrix nnz, chunk size, chunk
 // tables), plan, one persistent hash launch over all matrices' chunks and
-// finalize.  plan.spl/minb/ntiles/grid select the hash variant; plan_threads
-// is the sum of rows+1 over the matrices that have rows.
-cudaError_t launch_batch(const BatchArgs &b, const HashPlan &plan, uint32_t plan_threads,
-                         cudaStream_t stream);
+// finalize.  dense.spl/minb/grid select the dense variant; with
+// b.filter_min_row the filtered one (filtered.grid) is launched too and the
+// one that setup did not choose returns at once.  plan_threads is the sum of
+// rows+1 over the matrices that have rows.
+cudaError_t launch_batch(const BatchArgs &b, const HashPlan &dense, const HashPlan &filtered,
+                         uint32_t plan_threads, cudaStream_t stream);
+// The bound-filtered hash launches behind launch_hash / launch_batch, their
+// resident blocks per SM (filter_kernels.cu).
+cudaError_t launch_filter(const HashArgs &a, const HashPlan &plan, cudaStream_t stream);
+cudaError_t launch_filter_batch(const BatchArgs &b, const HashPlan &plan, cudaStream_t stream);
+int filter_blocks_per_sm(uint32_t s_pad);
 // Blocks per SM the hash kernel variant launched for (samples per lane,
 // register budget, s_pad) reaches, and its registers per thread.
 int hash_blocks_per_sm(uint32_t spl, uint32_t minb, uint32_t s_pad);
+// The same for the kernel a plan selects.
+int plan_blocks_per_sm(const HashPlan &plan, uint32_t s_pad);
+// Warps per block of that kernel.
+constexpr uint32_t plan_block_warps(const HashPlan &plan) {
+  return (plan.filter ? kFilterBlock : kHashBlock) / 32;
+}
 size_t hash_kernel_registers(uint32_t spl, uint32_t minb, uint32_t s_pad);
 
 // Parameter kernels (param_kernels.cu).
-enum class PairOp : int { kGamma = 0, kLogGamma = 1, kCopy = 2 };
-// params[d][which][s_base + s] = op(a[s*dim + d], b[s*dim + d]) for s < samples.
-cudaError_t launch_pack_params(const float *a, const float *b, PairOp op, uint32_t which,
-                               uint32_t dim, uint32_t s_base, uint32_t samples, uint32_t s_pad,
-                               float *params, cudaStream_t stream);
-// dst[s*dim + d] = params[d][which][s_base + s] for s < samples.
+// Blocks of sample rows in [samples][dim] order: the five uniform runs U1..U5
+// (draw), or r, ln_c and beta themselves.
+struct ParamSources {
+  const float *src[5];
+};
+// Fills samples [s_base, s_base + samples) of every column of the parameter
+// table and, if there is one, of the bound table (bound_byte).  parts: bits 0,
+// 1, 2 for r, ln_c, beta; the bound table is written when all are.
+cudaError_t launch_pack_params(const ParamSources &in, bool draw, uint32_t parts, uint32_t dim, uint32_t s_base,
+                               uint32_t samples, uint32_t s_pad, float *params, uint8_t *bounds,
+                               cudaStream_t stream);
+// dst[s*dim + d] = r, ln_c or beta (which 0, 1, 2) of column d, sample
+// s_base + s, for s < samples.
 cudaError_t launch_unpack_params(const float *params, uint32_t which, uint32_t dim,
                                  uint32_t s_base, uint32_t samples, uint32_t s_pad, float *dst,
                                  cudaStream_t stream);
@@ -175,6 +221,7 @@ class DeviceGuard {
 // engine.cu (engine.cu).
 struct GeneratorView {
   const float *params;
+  const uint8_t *bounds;  // nullptr: no bound table
   uint32_t dim;
   uint32_t samples;
   uint32_t s_pad;
@@ -186,7 +233,9 @@ struct GeneratorView {
 bool generator_view(const MinhashCudaGenerator_ *gen, GeneratorView *view);
 // The engine's work decomposition for `nnz` entries in `rows` rows, with at
 // least `min_items` warp items per resident warp where chunks allow.
+// allow_filter: false for a CSR in mapped host memory, which the filtered
+// kernels would read twice.
 HashPlan plan_for_generator(const MinhashCudaGenerator_ *gen, uint64_t nnz, uint64_t rows,
-                            uint32_t min_items = 8);
+                            uint32_t min_items = 8, bool allow_filter = true);
 
 }  // namespace mhb
