@@ -73,9 +73,9 @@ __device__ __forceinline__ uint32_t threshold(float mn) {
   return static_cast<uint32_t>(quant_up(mn) + kThrBias);
 }
 
-// Minima as ordered keys: (monotone image of ln_a, position).  The smallest
-// key is the smallest ln_a and, among equal ones, the earliest position: the
-// first strict minimum of kernel.cu:106, in whatever order it is combined.
+// Minima as (monotone image of ln_a, position).  The smallest pair is the
+// smallest ln_a and, among equal ones, the earliest position: the first strict
+// minimum of kernel.cu:106, in whatever order it is combined.
 __device__ __forceinline__ uint32_t ordered(float x) {
   const uint32_t u = __float_as_uint(__fadd_rn(x, 0.0f));  // -0 -> +0: equal as floats
   return u ^ (static_cast<uint32_t>(static_cast<int32_t>(u) >> 31) | 0x80000000u);
@@ -101,10 +101,16 @@ __device__ __forceinline__ uint32_t half_signs(uint32_t d0, uint32_t d1) {
   return r;
 }
 
-#ifndef FB
-#define FB 5
-#endif
-constexpr int kFilterBlocks = FB;
+// 20 warps per SM at 96 registers: 24 warps (80) and 16 (128) measured the
+// same or slower, 32 (64, with spills) 17% slower.
+constexpr int kFilterBlocks = 5;
+// Candidates evaluated at a time per lane; two sets of parameters in flight
+// leave the scan's registers unspilled (four: 6% slower on 1400-entry rows).
+constexpr uint32_t kEvalDepth = 2;
+// Queue length at which a batch is followed by an evaluation.  Fresh thresholds
+// pay: at 128 a 300-entry row has 13 candidates per sample, evaluated only at
+// the end of its windows 17.
+constexpr uint32_t kEvalAt = 128;
 constexpr uint32_t kFWin = 128;    // CSR positions per staged window
 constexpr uint32_t kQueue = 1024;  // candidates a warp holds
 
@@ -113,7 +119,8 @@ template <uint32_t TILE>
 struct alignas(16) FilterStage {
   WarpStageT<kFWin> st;
   int32_t l[kFWin];              // l of the window's entries in both halves (l * 65537)
-  unsigned long long key[TILE];  // running minima of the tile's samples
+  uint32_t val[TILE];            // running minima of the tile's samples (ordered)
+  uint32_t pos[TILE];            // and their positions
   uint16_t thr[TILE];            // their thresholds, m + kThrBias
   uint16_t queue[kQueue];        // candidates: window position | sample << 8
 };
@@ -136,9 +143,9 @@ __device__ __forceinline__ uint32_t warp_prefix(uint32_t x, uint32_t lane) {
 // LN lanes hold 16 samples each of one entry, so a tile is 16 * LN samples
 // and one warp load fetches the bytes of 32 / LN entries (16 per lane).  A
 // batch is 8 such loads, kept four ahead; its candidates go to a queue in
-// shared memory.  The queue is evaluated and the thresholds are updated at the
-// end of a window of 128 entries, four candidates per lane at a time so that
-// their parameter gathers overlap.
+// shared memory.  Once it holds 128, and at the end of a window or row, the
+// queue is evaluated, two candidates per lane at a time so that their
+// parameter gathers overlap, and the thresholds are updated.
 template <int LN, int SPAD, bool PACKED>
 __device__ __forceinline__ bool filter_item(const HashArgs &a, uint32_t c, uint32_t tile,
                                             WarpCtxT<kFWin> &wc, FilterStage<16 * LN> &fs) {
@@ -161,7 +168,7 @@ __device__ __forceinline__ bool filter_item(const HashArgs &a, uint32_t c, uint3
   const uint32_t width = min(TILE, a.samples - t0);  // samples of the tile that exist
   // Lanes past the last sample read the tile's first bytes; their candidate
   // bits are masked off.
-  const uint8_t *__restrict__ qbase = a.bounds + t0 + (t0 + sl < bstride ? sl : 0);
+  const uint32_t qoff = t0 + (t0 + sl < bstride ? sl : 0);
   const float *__restrict__ ptile = a.params + param_index(t0);
 
   const uint32_t cs = chunk_begin(a, c, base);
@@ -183,12 +190,12 @@ __device__ __forceinline__ bool filter_item(const HashArgs &a, uint32_t c, uint3
   uint32_t thr_guess = kThrOpen, thr_floor = 0;
   bool guessing = true;
 
-  // Thresholds from the keys, to shared memory and to the lanes that use them.
+  // Thresholds from the minima, to shared memory and to the lanes that use them.
   auto refresh = [&]() {
     uint32_t least = kThrOpen;
 #pragma unroll
     for (uint32_t v = 0; v < TILE / 32; ++v) {
-      const uint32_t hi = static_cast<uint32_t>(fs.key[v * 32 + lane] >> 32);
+      const uint32_t hi = fs.val[v * 32 + lane];
       const uint32_t t = max(min(thr_guess, threshold(unordered(hi))), thr_floor);
       fs.thr[v * 32 + lane] = static_cast<uint16_t>(t);
       least = min(least, t);
@@ -208,13 +215,13 @@ __device__ __forceinline__ bool filter_item(const HashArgs &a, uint32_t c, uint3
     for (uint32_t s1 = 0; s1 < width; s1 += 32) {
       const bool above =
           s1 + lane < width &&
-          threshold(unordered(static_cast<uint32_t>(fs.key[s1 + lane] >> 32))) > thr_guess;
+          threshold(unordered(fs.val[s1 + lane])) > thr_guess;
       uint32_t todo = __ballot_sync(0xFFFFFFFFu, above);
       while (todo) {
         const uint32_t s = s1 + __ffs(todo) - 1;
         todo &= todo - 1;
         ++failed;
-        unsigned long long best = fs.key[s];
+        unsigned long long best = static_cast<unsigned long long>(fs.val[s]) << 32 | fs.pos[s];
         for (uint32_t p = row_begin + lane; p < end; p += 32) {
           uint32_t col = PACKED ? packed_col(a, p) : a.cols[p];
           if (col >= a.dim) col = 0;
@@ -230,7 +237,10 @@ __device__ __forceinline__ bool filter_item(const HashArgs &a, uint32_t c, uint3
         for (int o = 16; o > 0; o >>= 1)
           best = min(best, __shfl_xor_sync(0xFFFFFFFFu, best, o));
         __syncwarp();
-        if (lane == 0) fs.key[s] = best;
+        if (lane == 0) {
+          fs.val[s] = static_cast<uint32_t>(best >> 32);
+          fs.pos[s] = static_cast<uint32_t>(best);
+        }
       }
     }
     // A table of other distributions, for which the guess does not hold.
@@ -244,11 +254,10 @@ __device__ __forceinline__ bool filter_item(const HashArgs &a, uint32_t c, uint3
     if (!fresh) rescan(end);
     const bool partial = head || row_end > ce;
     for (uint32_t s = lane; s < width; s += 32) {
-      const unsigned long long k = fresh ? make_key(FLT_MAX, kNone) : fs.key[s];
-      const uint32_t pos = static_cast<uint32_t>(k);
+      const uint32_t pos = fresh ? kNone : fs.pos[s];
       if (partial) {
         const size_t off = static_cast<size_t>(2 * c + (head ? 0 : 1)) * spad + t0 + s;
-        a.part_ln[off] = unordered(static_cast<uint32_t>(k >> 32));
+        a.part_ln[off] = fresh ? FLT_MAX : unordered(fs.val[s]);
         a.part_kt[off] = make_uint2(pos, 0u);
       } else {
         reinterpret_cast<uint2 *>(a.out)[static_cast<size_t>(row) * a.samples + t0 + s] =
@@ -291,30 +300,52 @@ __device__ __forceinline__ bool filter_item(const HashArgs &a, uint32_t c, uint3
     for (uint32_t i = n + lane; i < ((n + GRP - 1) & ~(GRP - 1)); i += 32) cl[i] = 0;
     __syncwarp();
 
-    // Evaluates the queued candidates, four per lane at a time.
+    // Evaluates queued candidates from the end, kEvalDepth per lane at a time,
+    // until at most `leave` are left.
     uint32_t count = 0;
-    auto evaluate = [&]() {
-      for (uint32_t at = 0; at < count; at += 128) {
-        uint32_t e[4];
-        float r[4], lc[4], be[4];
+    auto evaluate = [&](uint32_t leave) {
+      do {
+        const uint32_t from = count > 32 * kEvalDepth ? count - 32 * kEvalDepth : 0;
+        uint32_t e[kEvalDepth];
+        float r[kEvalDepth], lc[kEvalDepth], be[kEvalDepth];
 #pragma unroll
-        for (uint32_t j = 0; j < 4; ++j) {
-          // Lanes past the end repeat the last candidate: the same key again.
-          e[j] = fs.queue[min(at + 32 * j + lane, count - 1)];
+        for (uint32_t j = 0; j < kEvalDepth; ++j) {
+          // Lanes past the end repeat the last candidate's loads.
+          e[j] = fs.queue[min(from + 32 * j + lane, count - 1)];
           const float *p = ptile + static_cast<size_t>(cl[e[j] & 0xFFu]) * 3 * spad + param_index(e[j] >> 8);
           r[j] = __ldg(p);
           lc[j] = __ldg(p + 2);
           be[j] = __ldg(p + 4);
         }
+        // The minimum first, then the position of whoever holds it: the one
+        // lane that brought the value stores its own, equal values (ties,
+        // also with an earlier minimum) lower it to the earliest.
+        uint32_t x[kEvalDepth];
+        bool brought[kEvalDepth];
 #pragma unroll
-        for (uint32_t j = 0; j < 4; ++j) {
-          const uint32_t i = e[j] & 0xFFu;
-          const float x = exact_ln_a(lw[i], r[j], lc[j], be[j]);
-          if (at + 32 * j + lane < count && x < FLT_MAX) atomicMin(&fs.key[e[j] >> 8], make_key(x, ws + i));
+        for (uint32_t j = 0; j < kEvalDepth; ++j) {
+          const float ln_a = exact_ln_a(lw[e[j] & 0xFFu], r[j], lc[j], be[j]);
+          x[j] = from + 32 * j + lane < count && ln_a < FLT_MAX ? ordered(ln_a) : 0xFFFFFFFFu;
+          brought[j] = x[j] < atomicMin(&fs.val[e[j] >> 8], x[j]);
         }
-      }
-      count = 0;
-      __syncwarp();
+        __syncwarp();
+        bool tie = false;
+#pragma unroll
+        for (uint32_t j = 0; j < kEvalDepth; ++j) {
+          const bool holds = fs.val[e[j] >> 8] == x[j];
+          if (holds && brought[j]) fs.pos[e[j] >> 8] = ws + (e[j] & 0xFFu);
+          brought[j] = holds && !brought[j];
+          tie |= brought[j];
+        }
+        if (__any_sync(0xFFFFFFFFu, tie)) {
+          __syncwarp();
+#pragma unroll
+          for (uint32_t j = 0; j < kEvalDepth; ++j)
+            if (brought[j]) atomicMin(&fs.pos[e[j] >> 8], ws + (e[j] & 0xFFu));
+        }
+        __syncwarp();
+        count = from;
+      } while (count > leave);
     };
 
     uint32_t i = k == 0 ? cs - w0 : 0;
@@ -354,44 +385,68 @@ __device__ __forceinline__ bool filter_item(const HashArgs &a, uint32_t c, uint3
 #pragma unroll
         for (int v = 0; v < 8; ++v) thr[v] = thr_guess * 65537u;
 #pragma unroll
-        for (uint32_t v = 0; v < TILE / 32; ++v) fs.key[v * 32 + lane] = make_key(FLT_MAX, kNone);
+        for (uint32_t v = 0; v < TILE / 32; ++v) {
+          fs.val[v * 32 + lane] = ordered(FLT_MAX);
+          fs.pos[v * 32 + lane] = kNone;
+        }
         __syncwarp();
       }
       uint32_t g = i & ~(GRP - 1);
-      uint4 q[4];
+      uint4 q[4];  // bytes of four entries ahead
+      // The table is at most 2 GiB: 32-bit byte offsets.
       auto load = [&](uint32_t col) {
-        return __ldg(reinterpret_cast<const uint4 *>(qbase + static_cast<size_t>(col) * bstride));
+        return __ldg(reinterpret_cast<const uint4 *>(a.bounds + (col * bstride + qoff)));
       };
-      auto load4 = [&](uint32_t at) {
-        const uint4 cc = *reinterpret_cast<const uint4 *>(&cl[at]);
-        q[0] = load(cc.x); q[1] = load(cc.y); q[2] = load(cc.z); q[3] = load(cc.w);
-      };
-      load4(g + sub8);
+      {
+        const uint4 c0 = *reinterpret_cast<const uint4 *>(&cl[g + sub8]);
+        q[0] = load(c0.x);
+        q[1] = load(c0.y);
+        q[2] = load(c0.z);
+        q[3] = load(c0.w);
+      }
       while (g < seg) {
         const uint32_t h = g + sub8;
         const int32_t l_lo = (1 + 16384 - static_cast<int32_t>(thr_min)) * 65537;
         uint32_t miss[4] = {0, 0, 0, 0};  // byte j of [v], bit x: entry h + x cannot win 4v + j
+        // Entry h + x against the lane's 16 samples.
+        auto compare = [&](int x, int32_t lx) {
+          // l is kept above the value at which some T would drop below 1.
+          const uint32_t l = static_cast<uint32_t>(max(lx, l_lo));
+          const uint4 qx = q[x % 4];
+          const uint32_t qq[4] = {qx.x, qx.y, qx.z, qx.w};
 #pragma unroll
-        for (int y = 0; y < 2; ++y) {
-          const int4 l4 = *reinterpret_cast<const int4 *>(&fs.l[h + 4 * y]);
-          const int32_t ll[4] = {l4.x, l4.y, l4.z, l4.w};
-          // The loads four entries ahead; the last batch's repeat its own.
-          const uint32_t next = y == 0 ? h + 4 : g + GRP < seg ? h + GRP : h;
-          const uint4 c4 = *reinterpret_cast<const uint4 *>(&cl[next]);
-          const uint32_t cc[4] = {c4.x, c4.y, c4.z, c4.w};
-#pragma unroll
-          for (int x = 0; x < 4; ++x) {
-            // l is kept above the value at which some T would drop below 1.
-            const uint32_t l = static_cast<uint32_t>(max(ll[x], l_lo));
-            const uint32_t qq[4] = {q[x].x, q[x].y, q[x].z, q[x].w};
-#pragma unroll
-            for (int v = 0; v < 4; ++v) {
-              const uint32_t d0 = __byte_perm(qq[v], 0xC0C0C0C0u, 0x4140) - thr[2 * v] - l;
-              const uint32_t d1 = __byte_perm(qq[v], 0xC0C0C0C0u, 0x4342) - thr[2 * v + 1] - l;
-              miss[v] |= half_signs(d0, d1) & (0x01010101u << (4 * y + x));
-            }
-            q[x] = load(cc[x]);
+          for (int v = 0; v < 4; ++v) {
+            const uint32_t d0 = __byte_perm(qq[v], 0xC0C0C0C0u, 0x4140) - thr[2 * v] - l;
+            const uint32_t d1 = __byte_perm(qq[v], 0xC0C0C0C0u, 0x4342) - thr[2 * v + 1] - l;
+            miss[v] |= half_signs(d0, d1) & (0x01010101u << x);
           }
+        };
+        const int4 la = *reinterpret_cast<const int4 *>(&fs.l[h]);
+        const uint4 ca = *reinterpret_cast<const uint4 *>(&cl[h + 4]);
+        compare(0, la.x);
+        q[0] = load(ca.x);
+        compare(1, la.y);
+        q[1] = load(ca.y);
+        compare(2, la.z);
+        q[2] = load(ca.z);
+        compare(3, la.w);
+        q[3] = load(ca.w);
+        const int4 lb = *reinterpret_cast<const int4 *>(&fs.l[h + 4]);
+        if (g + GRP < seg) {  // with the loads of the next batch
+          const uint4 cb = *reinterpret_cast<const uint4 *>(&cl[h + GRP]);
+          compare(4, lb.x);
+          q[0] = load(cb.x);
+          compare(5, lb.y);
+          q[1] = load(cb.y);
+          compare(6, lb.z);
+          q[2] = load(cb.z);
+          compare(7, lb.w);
+          q[3] = load(cb.w);
+        } else {
+          compare(4, lb.x);
+          compare(5, lb.y);
+          compare(6, lb.z);
+          compare(7, lb.w);
         }
         uint32_t in_row = 0xFFFFFFFFu;  // entries of the row
         if (g < i || g + GRP > seg) {
@@ -409,11 +464,12 @@ __device__ __forceinline__ bool filter_item(const HashArgs &a, uint32_t c, uint3
           }
         }
         auto push = [&](uint32_t m, uint32_t v, uint32_t at) {
+          const uint32_t code = h | (sl + 4 * v) << 8;
           while (m) {
-            const uint32_t bit = __ffs(m) - 1;
-            m &= m - 1;
-            fs.queue[at++] =
-                static_cast<uint16_t>((h + (bit & 7u)) | (sl + 4 * v + (bit >> 3)) << 8);
+            uint32_t bit;  // the highest set bit: entry bit % 8, sample bit / 8
+            asm("bfind.u32 %0, %1;" : "=r"(bit) : "r"(m));
+            m ^= 1u << bit;
+            fs.queue[at++] = static_cast<uint16_t>(code + (bit & 7u) + (bit >> 3 << 8));
           }
           return at;
         };
@@ -426,6 +482,11 @@ __device__ __forceinline__ bool filter_item(const HashArgs &a, uint32_t c, uint3
 #pragma unroll
           for (uint32_t v = 0; v < 4; ++v) at = push(hits[v], v, at);
           count += total;
+          if (count >= kEvalAt) {
+            __syncwarp();
+            evaluate(32 * kEvalDepth - 1);
+            refresh();
+          }
         } else {
           // More than the queue has room for: by quarters of at most 1024.
 #pragma unroll 1
@@ -435,7 +496,7 @@ __device__ __forceinline__ bool filter_item(const HashArgs &a, uint32_t c, uint3
             const uint32_t sum2 = __shfl_sync(0xFFFFFFFFu, in2, 31);
             if (count + sum2 > kQueue) {
               __syncwarp();
-              evaluate();
+              evaluate(0);
             }
             push(m, v, count + in2 - __popc(m));
             count += sum2;
@@ -443,9 +504,11 @@ __device__ __forceinline__ bool filter_item(const HashArgs &a, uint32_t c, uint3
         }
         g += GRP;
       }
-      __syncwarp();
-      evaluate();
-      if (ws + seg < row_end) refresh();  // the row goes on
+      if (count) {
+        __syncwarp();
+        evaluate(0);
+        if (ws + seg < row_end) refresh();  // the row goes on
+      }
       i = seg;
     }
     if (k + 2 < nwin) {
