@@ -299,8 +299,19 @@ bool tuned_choice(const Gen *gen, uint64_t nnz, uint64_t rows, TuneChoice *out,
   return true;
 }
 
-constexpr uint32_t kFilterMinRow = 48;
-constexpr uint64_t kFilterMinEvals = 1ull << 29;
+// The filtered kernel evaluates 11-17 candidates per (row, sample) whatever the
+// row's length, the dense one every entry.  Measured on 8M entries in uniform
+// rows, 128 samples (ms, dense / filtered): rows of 60 entries 2.24 / 2.78, of
+// 80 2.15 / 2.23, of 100 2.11 / 1.94, of 120 2.07 / 1.76.
+constexpr uint32_t kFilterMinRow = 88;
+// Below it a launch is over before the chip is full: 30,000 entries in
+// 300-entry rows 31 / 34 us, 90,000 entries 69 / 51 us.
+constexpr uint64_t kFilterMinEvals = 1ull << 23;
+// Entries x tiles per resident warp below which tiles are made narrower: twice
+// the warps share a row, each with half the candidates, for a second pass over
+// the CSR.  3,000 rows of 1400 entries (1417 per warp): 485 us whole, 408
+// halved; 20,011 rows of 300 (2030 per warp): 481 whole, 567 halved.
+constexpr uint64_t kFilterShare = 1500;
 
 // Whether a launch takes the bound-filtered kernel (filter_kernels.cu).
 bool use_filter(const Gen *gen, uint64_t nnz, uint64_t rows, const TuneChoice *tuned) {
@@ -343,13 +354,15 @@ HashPlan make_plan(const Gen *gen, uint64_t nnz, uint64_t rows, const TuneChoice
   }
   p.spl = static_cast<uint32_t>(spl);
   p.minb = 4;
-  p.filter = allow_filter && use_filter(gen, nnz, rows, have_tuned ? &tuned : nullptr) ? 1u : 0u;
-  if (p.filter) p.spl = 4;
+  if (allow_filter && use_filter(gen, nnz, rows, have_tuned ? &tuned : nullptr)) {
+    p.filter = mhb::filter_lanes(s_pad);
+    p.spl = 4;
+  }
   if (p.spl == 4) {
     const int minb = env_int("MHCUDA_B200_MINB", have_tuned ? static_cast<int>(tuned.minb) : 4);
     p.minb = (minb == 3 || minb == 2) ? static_cast<uint32_t>(minb) : 4u;
   }
-  const uint32_t tile_w = p.filter ? mhb::filter_tile(s_pad) : 32u * p.spl;
+  const uint32_t tile_w = p.filter ? 16 * p.filter : 32u * p.spl;
   p.ntiles = (s_pad + tile_w - 1) / tile_w;
   const int bps = mhb::plan_blocks_per_sm(p, s_pad);
   const uint64_t resident_warps =
@@ -366,9 +379,15 @@ HashPlan make_plan(const Gen *gen, uint64_t nnz, uint64_t rows, const TuneChoice
   // resident warp even if rows then span chunks (their partials are merged
   // by finalize).
   if (p.filter) {
-    // A row in pieces starts its search anew in each: chunks of a mean row at
-    // least.
-    chunk = std::max<uint64_t>(chunk, std::min<uint64_t>(avg_row, 4096));
+    // Few entries per warp: narrower tiles before rows in pieces, each of which
+    // starts its search anew.
+    while (p.filter > 2 && nnz * p.ntiles < resident_warps * kFilterShare) {
+      p.filter /= 2;
+      p.ntiles = mhb::filter_tiles(s_pad, p.filter);
+    }
+    const mhb::FilterSplit sp = mhb::filter_split(nnz * p.ntiles, resident_warps, waves, avg_row);
+    chunk = sp.chunk;
+    p.snap = sp.snap;
   } else {
     const uint64_t want = resident_warps * std::max<uint32_t>(1, min_items);
     chunk = std::min<uint64_t>(chunk, std::max<uint64_t>(64, (nnz * p.ntiles + want - 1) / want));
@@ -398,14 +417,15 @@ MHCUDAResult prepare_launch(const Gen *gen, uint32_t rows, uint32_t nnz, const H
             mhcudaMemoryAllocationFailure);
   MHB_CHECK(gen, gen->d_part_kt.ensure(slots * gen->s_pad * sizeof(uint2)),
             mhcudaMemoryAllocationFailure);
-  MHB_CHECK(gen, gen->d_status.ensure(sizeof(uint32_t)), mhcudaMemoryAllocationFailure);
+  MHB_CHECK(gen, gen->d_status.ensure(2 * sizeof(uint32_t)), mhcudaMemoryAllocationFailure);
   a->params = gen->params;
   a->dim = gen->dim;
   a->samples = gen->samples;
   a->s_pad = gen->s_pad;
   a->bounds = gen->usable_bounds();
   a->b_stride = mhb::bound_stride(gen->s_pad);
-  a->snap_rows = plan.filter;
+  a->snap = plan.snap;
+  a->next_item = plan.filter ? gen->d_status.as<uint32_t>() + 1 : nullptr;
   a->rows = rows;
   a->nnz = nnz;
   a->chunk = plan.chunk;
@@ -693,7 +713,7 @@ MHCUDAResult calc_pipelined(const Gen *gen, const HostCsr &in, uint32_t length,
   const int forced = env_int("MHCUDA_B200_BLOCK_NNZ", 0);
   if (forced > 0) block_nnz = static_cast<uint64_t>(forced);
   const size_t row_bytes = static_cast<size_t>(gen->samples) * 2 * sizeof(uint32_t);
-  MHB_CHECK(gen, gen->d_status.ensure(sizeof(uint32_t)), mhcudaMemoryAllocationFailure);
+  MHB_CHECK(gen, gen->d_status.ensure(2 * sizeof(uint32_t)), mhcudaMemoryAllocationFailure);
   MHB_CHECK(gen, cudaMemsetAsync(gen->d_status.ptr, 0, sizeof(uint32_t), st), mhcudaRuntimeError);
   // The blocks are cut from one matrix: a variant the autotuner chose for the
   // whole matrix's shape applies to each of them (their own, smaller shape
@@ -1422,8 +1442,8 @@ enum MHCUDAResult mhcuda_calc_batch_device(const MinhashCudaGenerator *gen, uint
   // device from the batch's nnz (batch_setup_kernel).
   HashPlan vp = make_plan(gen, 1ull << 30, 1ull << 20, nullptr, 8, false);
   HashPlan fp = vp;
-  fp.filter = 1;
-  fp.ntiles = (gen->s_pad + mhb::filter_tile(gen->s_pad) - 1) / mhb::filter_tile(gen->s_pad);
+  fp.filter = mhb::filter_lanes(gen->s_pad);
+  fp.ntiles = mhb::filter_tiles(gen->s_pad, fp.filter);
   // Whether the batch is filtered is decided on the device too; a batch of few
   // rows is not worth the second launch that takes.
   const int force_filter = env_int("MHCUDA_B200_FILTER", -1);
@@ -1439,11 +1459,11 @@ enum MHCUDAResult mhcuda_calc_batch_device(const MinhashCudaGenerator *gen, uint
     const uint64_t warps =
         static_cast<uint64_t>(gen->sm_count) * bps * mhb::plan_block_warps(*plans[f]);
     resident_warps = std::max(resident_warps, warps);
-    b.target_items[f] = warps * static_cast<uint64_t>(waves);
-    b.want_items[f] = warps * 8;
+    b.warps[f] = warps;
     b.ntiles[f] = plans[f]->ntiles;
     plans[f]->grid = static_cast<uint32_t>(static_cast<uint64_t>(gen->sm_count) * bps);
   }
+  b.waves = static_cast<uint64_t>(waves);
   b.filter_min_row = !may_filter ? 0 : force_filter > 0 ? 1 : kFilterMinRow;
   b.filter_min_nnz = force_filter > 0 ? 0 : kFilterMinEvals / gen->s_pad;
   const uint64_t max_chunks64 = count + resident_warps * 8 + 1;
@@ -1452,6 +1472,7 @@ enum MHCUDAResult mhcuda_calc_batch_device(const MinhashCudaGenerator *gen, uint
   HashPlan big{};
   big.nchunks = max_chunks;
   HashArgs base{};
+  big.filter = may_filter;  // for next_item
   MHCUDAResult r = prepare_launch(gen, 0, 0, big, &base);
   if (r != mhcudaSuccess) return r;
   MHB_CHECK(gen, gen->d_chunk_owner.ensure(static_cast<size_t>(max_chunks) * 4),
@@ -1685,7 +1706,7 @@ enum MHCUDAResult mhcuda_calc_batch(const MinhashCudaGenerator *gen, uint32_t co
   const int forced = env_int("MHCUDA_B200_BLOCK_NNZ", 0);
   if (forced > 0) group_nnz = static_cast<uint64_t>(forced);
   const uint64_t group_rows = 1u << 20;
-  MHB_CHECK(gen, gen->d_status.ensure(sizeof(uint32_t)), mhcudaMemoryAllocationFailure);
+  MHB_CHECK(gen, gen->d_status.ensure(2 * sizeof(uint32_t)), mhcudaMemoryAllocationFailure);
   MHB_CHECK(gen, cudaMemsetAsync(gen->d_status.ptr, 0, sizeof(uint32_t), st), mhcudaRuntimeError);
   const unsigned nth = host_threads();
 

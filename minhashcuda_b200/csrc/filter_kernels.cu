@@ -527,6 +527,13 @@ __device__ __forceinline__ bool filter_item(const HashArgs &a, uint32_t c, uint3
   return true;
 }
 
+// The next item beyond each warp's first, taken in order of demand (lane 0
+// holds it): rows, and so items, differ in length, and the last items of a
+// launch go to the warps that are done.
+__device__ __forceinline__ uint32_t take_item(uint32_t *next_item, uint32_t lane) {
+  return lane == 0 ? atomicAdd(next_item, 1u) : 0u;
+}
+
 template <int LN, int SPAD, bool PACKED>
 __global__ void __launch_bounds__(kFilterBlock, kFilterBlocks) filter_kernel(const HashArgs a) {
   __shared__ FilterStage<16 * LN> stage_all[kFilterBlock / 32];
@@ -542,9 +549,11 @@ __global__ void __launch_bounds__(kFilterBlock, kFilterBlocks) filter_kernel(con
   const uint32_t gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const uint32_t nw = (gridDim.x * blockDim.x) >> 5;
   const uint32_t items = a.nchunks * a.ntiles;
-  for (uint32_t item = gw; item < items; item += nw) {
+  for (uint32_t item = gw; item < items;) {
+    const uint32_t next = take_item(a.next_item, wc.lane);  // in flight during this item
     const uint32_t c = item / a.ntiles;
     if (!filter_item<LN, SPAD, PACKED>(a, c, item - c * a.ntiles, wc, fs)) return;
+    item = nw + __shfl_sync(0xFFFFFFFFu, next, 0);
   }
 }
 
@@ -562,7 +571,8 @@ __global__ void __launch_bounds__(kFilterBlock, kFilterBlocks) filter_batch_kern
   const uint32_t ntiles = b.ntiles[1];
   const uint32_t chunk = b.plan->chunk;
   const uint32_t items = b.plan->nchunks * ntiles;
-  for (uint32_t item = gw; item < items; item += nw) {
+  for (uint32_t item = gw; item < items;) {
+    const uint32_t next = take_item(b.base.next_item, wc.lane);
     const uint32_t gc = item / ntiles;
     const uint32_t m = b.chunk_owner[gc];
     const uint32_t base = b.mats[m].chunk_base;
@@ -570,16 +580,19 @@ __global__ void __launch_bounds__(kFilterBlock, kFilterBlocks) filter_batch_kern
     if (wc.lane == 0) view = matrix_view(b, b.mats[m], chunk);
     __syncwarp();
     if (!filter_item<LN, SPAD, false>(view, gc - base, item - gc * ntiles, wc, fs)) return;
+    item = nw + __shfl_sync(0xFFFFFFFFu, next, 0);
   }
 }
 
 using FilterFn = void (*)(const HashArgs);
 using FilterBatchFn = void (*)(const BatchArgs);
 
-FilterFn pick_filter(uint32_t s_pad, bool packed) {
-  if (s_pad == 128) return packed ? filter_kernel<8, 128, true> : filter_kernel<8, 128, false>;
-  if (s_pad == 256) return packed ? filter_kernel<8, 256, true> : filter_kernel<8, 256, false>;
-  switch (filter_lanes(s_pad)) {
+FilterFn pick_filter(uint32_t s_pad, uint32_t lanes, bool packed) {
+  if (lanes == 8 && s_pad == 128)
+    return packed ? filter_kernel<8, 128, true> : filter_kernel<8, 128, false>;
+  if (lanes == 8 && s_pad == 256)
+    return packed ? filter_kernel<8, 256, true> : filter_kernel<8, 256, false>;
+  switch (lanes) {
     case 8: return packed ? filter_kernel<8, 0, true> : filter_kernel<8, 0, false>;
     case 4: return packed ? filter_kernel<4, 0, true> : filter_kernel<4, 0, false>;
     default: return packed ? filter_kernel<2, 0, true> : filter_kernel<2, 0, false>;
@@ -599,7 +612,7 @@ FilterBatchFn pick_filter_batch(uint32_t s_pad) {
 }  // namespace
 
 cudaError_t launch_filter(const HashArgs &a, const HashPlan &plan, cudaStream_t stream) {
-  pick_filter(a.s_pad, a.col_hi_bits != 0)<<<plan.grid, kFilterBlock, 0, stream>>>(a);
+  pick_filter(a.s_pad, plan.filter, a.col_hi_bits != 0)<<<plan.grid, kFilterBlock, 0, stream>>>(a);
   return cudaGetLastError();
 }
 
@@ -608,9 +621,9 @@ cudaError_t launch_filter_batch(const BatchArgs &b, const HashPlan &plan, cudaSt
   return cudaGetLastError();
 }
 
-int filter_blocks_per_sm(uint32_t s_pad) {
+int filter_blocks_per_sm(uint32_t s_pad, uint32_t lanes) {
   int n = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, pick_filter(s_pad, false), kFilterBlock, 0) !=
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, pick_filter(s_pad, lanes, false), kFilterBlock, 0) !=
       cudaSuccess) {
     cudaGetLastError();
     return 1;

@@ -60,16 +60,16 @@ __device__ __forceinline__ bool fast_t(float w, float r, float b, float &t) {
   return fabsf(__fsub_rn(f, 0.5f)) < __fsub_rn(0.5f, m);  // NaN -> false
 }
 
-// First position of chunk c (c == nchunks: nnz).  With snap_rows (the filtered
-// kernels, whose rows are dearer in pieces) that is the start of the next row
-// when it lies at most one chunk further, so only rows longer than a chunk
-// are cut; otherwise it is c * chunk.
+// First position of chunk c (c == nchunks: nnz): c * chunk or, when a row
+// starts at most `snap` positions further, that row's start (the filtered
+// kernels, whose rows are dearer in pieces).  Chunks inside a row that is kept
+// whole are empty.
 __device__ __forceinline__ uint32_t chunk_begin(const HashArgs &a, uint32_t c, uint32_t base) {
   if (c >= a.nchunks) return a.nnz;
   const uint32_t at = c * a.chunk;
-  if (!a.snap_rows) return at;
+  if (!a.snap) return at;
   const uint32_t e = a.indptr[a.chunk_row[c]] - base;
-  return e - at <= a.chunk ? e : at;
+  return e - at <= a.snap ? e : at;
 }
 
 // One (nnz, sample) evaluation, kernel.cu:101-109, given t: keeps the
@@ -484,7 +484,7 @@ __device__ __forceinline__ HashArgs matrix_view(const BatchArgs &b, const BatchM
   v.nnz = m.nnz;
   v.chunk = chunk;
   v.nchunks = m.nchunks;
-  v.snap_rows = b.plan->filter;
+  v.snap = b.plan->snap;
   v.chunk_row = b.base.chunk_row + m.chunk_base;
   v.part_ln = b.base.part_ln + static_cast<size_t>(2) * m.chunk_base * b.base.s_pad;
   v.part_kt = b.base.part_kt + static_cast<size_t>(2) * m.chunk_base * b.base.s_pad;

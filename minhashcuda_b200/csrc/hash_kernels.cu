@@ -69,6 +69,7 @@ __device__ __forceinline__ void plan_row(const HashArgs &a, uint32_t i) {
 
 __global__ void plan_kernel(const HashArgs a) {
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i == 0 && a.next_item) *a.next_item = 0;
   if (i <= a.rows) plan_row(a, i);
 }
 
@@ -326,7 +327,7 @@ __device__ __forceinline__ void finalize_item(const HashArgs &a, uint32_t c, uin
   const uint32_t ce = chunk_begin(a, c + 1, base);
   if (end <= ce || s >= a.samples) return;
   uint32_t c_last = (end - 1) / a.chunk;
-  if (chunk_begin(a, c_last, base) >= end) --c_last;  // starts at the next row
+  while (chunk_begin(a, c_last, base) >= end) --c_last;  // begins at the next row
   const size_t stride = 2 * static_cast<size_t>(a.s_pad);  // one chunk's two slots
   size_t off = static_cast<size_t>(2 * c + 1) * a.s_pad + s;
   float mn = a.part_ln[off];
@@ -448,12 +449,16 @@ __global__ void __launch_bounds__(kSetupThreads) batch_setup_kernel(const BatchA
     const uint32_t f = b.filter_min_row && total_nnz >= total_rows * b.filter_min_row &&
                        total_nnz >= b.filter_min_nnz;
     b.plan->filter = f;
-    const uint64_t ntiles = b.ntiles[f], target = b.target_items[f], want = b.want_items[f];
+    const uint64_t ntiles = b.ntiles[f], target = b.warps[f] * b.waves, want = b.warps[f] * 8;
     uint64_t chunk = (total_nnz * ntiles + target - 1) / target;
     const uint64_t avg_row = total_rows ? (total_nnz + total_rows - 1) / total_rows : 1;
     chunk = max(chunk, min(4 * avg_row, static_cast<uint64_t>(1024)));
-    if (f) {  // as make_plan: a row in pieces starts its search anew in each
-      chunk = max(chunk, min(avg_row, static_cast<uint64_t>(4096)));
+    b.plan->snap = 0;
+    if (f) {
+      const FilterSplit sp = filter_split(total_nnz * ntiles, b.warps[1], b.waves, avg_row);
+      chunk = sp.chunk;
+      b.plan->snap = sp.snap;
+      *b.base.next_item = 0;
     } else {
       chunk = min(chunk, max(static_cast<uint64_t>(64), (total_nnz * ntiles + want - 1) / want));
     }
@@ -694,7 +699,7 @@ int hash_blocks_per_sm(uint32_t spl, uint32_t minb, uint32_t s_pad) {
 }
 
 int plan_blocks_per_sm(const HashPlan &plan, uint32_t s_pad) {
-  return plan.filter ? filter_blocks_per_sm(s_pad) : hash_blocks_per_sm(plan.spl, plan.minb, s_pad);
+  return plan.filter ? filter_blocks_per_sm(s_pad, plan.filter) : hash_blocks_per_sm(plan.spl, plan.minb, s_pad);
 }
 
 size_t hash_kernel_registers(uint32_t spl, uint32_t minb, uint32_t s_pad) {

@@ -126,7 +126,6 @@ extern "C" enum MHCUDAResult mhcuda_calc_device_noalloc(
   a.s_pad = s_pad;
   a.bounds = g.bounds;
   a.b_stride = mhb::bound_stride(s_pad);
-  a.snap_rows = plan.filter;
   a.weights = d_weights;
   a.cols = d_cols;
   a.indptr = d_rows;

@@ -334,7 +334,8 @@ MHCUDAResult MinhashCudaServer_::run_units(Lane &lane, const std::vector<Unit> &
   a.s_pad = s_pad;
   a.bounds = g.bounds;
   a.b_stride = mhb::bound_stride(s_pad);
-  a.snap_rows = plan.filter;
+  a.snap = plan.snap;
+  a.next_item = plan.filter ? lane.status + 1 : nullptr;
   a.weights = zc ? lane.mw : lane.w;
   a.cols = zc ? lane.mc : lane.c;
   a.indptr = zc ? lane.mip : lane.ip;

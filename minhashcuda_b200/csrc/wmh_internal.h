@@ -42,9 +42,11 @@ struct HashPlan {
   uint32_t nchunks;  // >= 1
   uint32_t spl;      // samples per lane in one item: 1, 2 or 4
   uint32_t minb;     // kernel variant: minimum resident blocks per SM (4; 3 or 2 for spl 4)
-  uint32_t ntiles;   // sample tiles of 32*spl samples (filter: filter_tile(s_pad))
+  uint32_t ntiles;   // sample tiles of 32*spl samples (filter: of 16*filter)
   uint32_t grid;     // persistent grid (blocks of kHashBlock threads)
-  uint32_t filter;   // bound-filtered kernel (filter_kernels.cu) instead of the dense one
+  uint32_t filter;   // 0: the dense kernel; 8, 4, 2: the bound-filtered one
+                     // (filter_kernels.cu) with that many lanes per entry
+  uint32_t snap;     // HashArgs::snap
 };
 
 constexpr int kHashBlock = 256;
@@ -56,10 +58,28 @@ constexpr uint32_t bound_stride(uint32_t s_pad) { return (s_pad + 31) & ~31u; }
 // Sample counts the filter kernels serve: below 32 the dense kernels read no
 // more sectors per entry than the bounds would add.
 constexpr uint32_t kFilterMinSamples = 32;
-// Lanes the filter kernels give one entry (16 samples each), and their sample
-// tile.
+// Most lanes the filter kernels give one entry (16 samples each).
 constexpr uint32_t filter_lanes(uint32_t s_pad) { return s_pad > 64 ? 8 : s_pad > 32 ? 4 : 2; }
-constexpr uint32_t filter_tile(uint32_t s_pad) { return 16 * filter_lanes(s_pad); }
+constexpr uint32_t filter_tiles(uint32_t s_pad, uint32_t lanes) {
+  return (s_pad + 16 * lanes - 1) / (16 * lanes);
+}
+// Work division of a filtered launch over `total` = entries x sample tiles and
+// `warps` resident warps: positions per chunk and the snap distance.  Chunks
+// of a mean row, but eight or more per warp, 32 at least 128 positions long;
+// rows are kept whole up to a quarter of a warp's share.
+struct FilterSplit {
+  uint32_t chunk, snap;
+};
+__host__ __device__ inline FilterSplit filter_split(uint64_t total, uint64_t warps, uint64_t waves,
+                                                    uint64_t avg_row) {
+  const uint64_t share = total / warps;
+  uint64_t chunk = share / waves, whole = share / 8 < avg_row ? share / 8 : avg_row;
+  chunk = chunk > whole ? chunk : whole;
+  chunk = chunk < 128 ? 128 : chunk > (1u << 24) ? (1u << 24) : (chunk + 31) & ~31ull;
+  uint64_t snap = share / 4 < 8192 ? share / 4 : 8192;
+  snap = snap > chunk ? snap : chunk;
+  return FilterSplit{static_cast<uint32_t>(chunk), static_cast<uint32_t>(snap)};
+}
 
 struct HashArgs {
   const float *params;       // [dim][s_pad / 2][r r c c b b], see param_index
@@ -91,7 +111,11 @@ struct HashArgs {
   // nullptr when the generator has none.
   const uint8_t *bounds;
   uint32_t b_stride;
-  uint32_t snap_rows;  // chunks begin at rows where possible (chunk_begin); filtered launches
+  // Filtered launches: a chunk begins at the next row when that is at most
+  // `snap` positions away (chunk_begin); warps take items off *next_item,
+  // which the plan kernel sets to 0.  0 and nullptr for dense launches.
+  uint32_t snap;
+  uint32_t *next_item;
 };
 
 // One matrix of a device-resident batch (mhcuda_calc_batch_device).  The
@@ -113,6 +137,7 @@ struct BatchPlan {
   uint32_t chunk;    // positions per chunk, the same for every matrix
   uint32_t nchunks;  // chunks of all matrices
   uint32_t filter;   // the bound-filtered launch does the work, not the dense one
+  uint32_t snap;     // its HashArgs::snap
 };
 
 struct BatchArgs {
@@ -125,8 +150,8 @@ struct BatchArgs {
   BatchPlan *plan;
   uint32_t *chunk_owner;  // [max_chunks] matrix of each batch chunk
   // [0] the dense kernel, [1] the filtered one:
-  uint64_t target_items[2];  // warp items to aim for (resident warps x waves)
-  uint64_t want_items[2];    // items per launch below which chunks shrink (resident warps x 8)
+  uint64_t warps[2];   // resident warps
+  uint64_t waves;      // items per resident warp to aim for
   uint32_t ntiles[2];
   // A batch is filtered when its mean row has this many entries and its
   // entries reach filter_min_nnz; 0: never (then only the dense kernel is
@@ -152,7 +177,7 @@ cudaError_t launch_batch(const BatchArgs &b, const HashPlan &dense, const HashPl
 // resident blocks per SM (filter_kernels.cu).
 cudaError_t launch_filter(const HashArgs &a, const HashPlan &plan, cudaStream_t stream);
 cudaError_t launch_filter_batch(const BatchArgs &b, const HashPlan &plan, cudaStream_t stream);
-int filter_blocks_per_sm(uint32_t s_pad);
+int filter_blocks_per_sm(uint32_t s_pad, uint32_t lanes);
 // Blocks per SM the hash kernel variant launched for (samples per lane,
 // register budget, s_pad) reaches, and its registers per thread.
 int hash_blocks_per_sm(uint32_t spl, uint32_t minb, uint32_t s_pad);
