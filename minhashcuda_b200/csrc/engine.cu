@@ -301,9 +301,9 @@ bool tuned_choice(const Gen *gen, uint64_t nnz, uint64_t rows, TuneChoice *out,
 
 // The filtered kernel evaluates 11-17 candidates per (row, sample) whatever the
 // row's length, the dense one every entry.  Measured on 8M entries in uniform
-// rows, 128 samples (ms, dense / filtered): rows of 60 entries 2.24 / 2.78, of
-// 80 2.15 / 2.23, of 100 2.11 / 1.94, of 120 2.07 / 1.76.
-constexpr uint32_t kFilterMinRow = 88;
+// rows, 128 samples (ms, dense / filtered): rows of 60 entries 2.24 / 2.47, of
+// 80 2.15 / 1.97, of 100 2.11 / 1.72, of 120 2.07 / 1.6.
+constexpr uint32_t kFilterMinRow = 72;
 // Below it a launch is over before the chip is full: 30,000 entries in
 // 300-entry rows 31 / 34 us, 90,000 entries 69 / 51 us.
 constexpr uint64_t kFilterMinEvals = 1ull << 23;

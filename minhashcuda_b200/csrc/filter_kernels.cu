@@ -87,10 +87,14 @@ __device__ __forceinline__ unsigned long long make_key(float x, uint32_t pos) {
   return static_cast<unsigned long long>(ordered(x)) << 32 | pos;
 }
 
-// ln_a of one (entry, sample), kernel.cu:101-105.
-__device__ __forceinline__ float exact_ln_a(float w, float r, float c, float b) {
-  const float t = exact_t(w, r, b);
+// ln_a of one (entry, sample), kernel.cu:101-105, and its t.
+__device__ __forceinline__ float exact_ln_a(float w, float r, float c, float b, float &t) {
+  t = exact_t(w, r, b);
   return __fsub_rn(__fmaf_rn(-__fsub_rn(t, b), r, c), r);
+}
+// (uint32)(int32)t as kernel.cu:108; the conversion saturates.
+__device__ __forceinline__ uint32_t whole(float t) {
+  return static_cast<uint32_t>(static_cast<int32_t>(t));
 }
 
 // The sign bits of the four halves of (d0, d1), each spread over a byte (prmt
@@ -101,28 +105,36 @@ __device__ __forceinline__ uint32_t half_signs(uint32_t d0, uint32_t d1) {
   return r;
 }
 
-// 20 warps per SM at 96 registers: 24 warps (80) and 16 (128) measured the
-// same or slower, 32 (64, with spills) 17% slower.
-constexpr int kFilterBlocks = 5;
-// Candidates evaluated at a time per lane; two sets of parameters in flight
-// leave the scan's registers unspilled (four: 6% slower on 1400-entry rows).
+// 24 warps per SM at 80 registers, with the seldom used state of an item in
+// shared memory: 131,072 Zipf rows of 1400 entries take 7.3 ms, 7.7 with 20
+// warps (96 registers), 7.6 with 28 (72), 7.5 with 32 (64).
+constexpr int kFilterBlocks = 6;
+// Candidates evaluated at a time per lane: 1 / 2 / 3 take 7.9 / 7.3 / 7.8 ms
+// there, and 7.5 / 6.6 / 6.6 ms on 256 uneven matrices at 256 samples.
 constexpr uint32_t kEvalDepth = 2;
 // Queue length at which a batch is followed by an evaluation.  Fresh thresholds
 // pay: at 128 a 300-entry row has 13 candidates per sample, evaluated only at
 // the end of its windows 17.
 constexpr uint32_t kEvalAt = 128;
 constexpr uint32_t kFWin = 128;    // CSR positions per staged window
-constexpr uint32_t kQueue = 1024;  // candidates a warp holds
+// Candidates a warp holds: at least 127 left over and 512 more.  Shared memory
+// is taken from L1, which has to hold a candidate's sector between its three
+// loads: 1024 measured 4% slower on 1400-entry rows.
+constexpr uint32_t kQueue = 768;
 
 // One warp's shared memory; TILE samples per tile.
 template <uint32_t TILE>
 struct alignas(16) FilterStage {
   WarpStageT<kFWin> st;
   int32_t l[kFWin];              // l of the window's entries in both halves (l * 65537)
-  uint32_t val[TILE];            // running minima of the tile's samples (ordered)
-  uint32_t pos[TILE];            // and their positions
+  // The tile's samples: the running minimum (ordered), its position, and the
+  // pair it gives (kernel.cu:108).
+  uint32_t val[TILE], pos[TILE], k[TILE], t[TILE];
   uint16_t thr[TILE];            // their thresholds, m + kThrBias
   uint16_t queue[kQueue];        // candidates: window position | sample << 8
+  // Of the item, seldom read (registers are short): its chunk, the end of the
+  // rows it owns, and the first position of the current row in the chunk.
+  uint32_t chunk, r_stop, row_begin;
 };
 
 // Inclusive prefix sum over the warp.
@@ -174,8 +186,14 @@ __device__ __forceinline__ bool filter_item(const HashArgs &a, uint32_t c, uint3
   const uint32_t cs = chunk_begin(a, c, base);
   const uint32_t ce = chunk_begin(a, c + 1, base);
   uint32_t r_next = a.chunk_row[c];
-  const uint32_t r_stop = (c + 1 < a.nchunks) ? a.chunk_row[c + 1] : a.rows;
-  uint32_t row = kNone, row_end = cs, row_begin = cs;  // row_begin: its first position in the chunk
+  __syncwarp();
+  if (lane == 0) {
+    fs.chunk = c;
+    fs.r_stop = (c + 1 < a.nchunks) ? a.chunk_row[c + 1] : a.rows;
+    fs.row_begin = cs;
+  }
+  __syncwarp();
+  uint32_t row = kNone, row_end = cs;
   bool head = false, fresh = true;  // fresh: none of the row's entries has been looked at
   if (r_next > 0) {
     const uint32_t e = a.indptr[r_next] - base;
@@ -187,11 +205,12 @@ __device__ __forceinline__ bool filter_item(const HashArgs &a, uint32_t c, uint3
   }
   uint32_t thr[8];         // thresholds of the lane's 16 samples, two per register
   uint32_t thr_min = 0;    // the least of the tile's
-  uint32_t thr_guess = kThrOpen, thr_floor = 0;
+  uint32_t thr_guess = kThrOpen;
   bool guessing = true;
 
   // Thresholds from the minima, to shared memory and to the lanes that use them.
   auto refresh = [&]() {
+    const uint32_t thr_floor = thr_guess == kThrOpen ? 0 : thr_guess - kThrSpread;
     uint32_t least = kThrOpen;
 #pragma unroll
     for (uint32_t v = 0; v < TILE / 32; ++v) {
@@ -221,8 +240,9 @@ __device__ __forceinline__ bool filter_item(const HashArgs &a, uint32_t c, uint3
         const uint32_t s = s1 + __ffs(todo) - 1;
         todo &= todo - 1;
         ++failed;
+        uint32_t best_k = fs.k[s], best_t = fs.t[s];
         unsigned long long best = static_cast<unsigned long long>(fs.val[s]) << 32 | fs.pos[s];
-        for (uint32_t p = row_begin + lane; p < end; p += 32) {
+        for (uint32_t p = fs.row_begin + lane; p < end; p += 32) {
           uint32_t col = PACKED ? packed_col(a, p) : a.cols[p];
           if (col >= a.dim) col = 0;
           const float w = logf(a.weights[p]);
@@ -230,16 +250,24 @@ __device__ __forceinline__ bool filter_item(const HashArgs &a, uint32_t c, uint3
           const int m = quant_up(unordered(static_cast<uint32_t>(best >> 32)));
           if (static_cast<int>(byte) > max(m + quant_up(w) + 240, 0)) continue;
           const float *p3 = ptile + static_cast<size_t>(col) * 3 * spad + param_index(s);
-          const float x = exact_ln_a(w, __ldg(p3), __ldg(p3 + 2), __ldg(p3 + 4));
-          if (x < FLT_MAX) best = min(best, make_key(x, p));
+          float t;
+          const float x = exact_ln_a(w, __ldg(p3), __ldg(p3 + 2), __ldg(p3 + 4), t);
+          if (x < FLT_MAX && make_key(x, p) < best) {
+            best = make_key(x, p);
+            best_k = col;
+            best_t = whole(t);
+          }
         }
+        unsigned long long least = best;
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1)
-          best = min(best, __shfl_xor_sync(0xFFFFFFFFu, best, o));
+          least = min(least, __shfl_xor_sync(0xFFFFFFFFu, least, o));
         __syncwarp();
-        if (lane == 0) {
-          fs.val[s] = static_cast<uint32_t>(best >> 32);
-          fs.pos[s] = static_cast<uint32_t>(best);
+        if (best == least) {  // lanes that share it hold the same pair
+          fs.val[s] = static_cast<uint32_t>(least >> 32);
+          fs.pos[s] = static_cast<uint32_t>(least);
+          fs.k[s] = best_k;
+          fs.t[s] = best_t;
         }
       }
     }
@@ -254,14 +282,13 @@ __device__ __forceinline__ bool filter_item(const HashArgs &a, uint32_t c, uint3
     if (!fresh) rescan(end);
     const bool partial = head || row_end > ce;
     for (uint32_t s = lane; s < width; s += 32) {
-      const uint32_t pos = fresh ? kNone : fs.pos[s];
       if (partial) {
-        const size_t off = static_cast<size_t>(2 * c + (head ? 0 : 1)) * spad + t0 + s;
+        const size_t off = static_cast<size_t>(2 * fs.chunk + (head ? 0 : 1)) * spad + t0 + s;
         a.part_ln[off] = fresh ? FLT_MAX : unordered(fs.val[s]);
-        a.part_kt[off] = make_uint2(pos, 0u);
+        a.part_kt[off] = make_uint2(fresh ? kNone : fs.pos[s], 0u);
       } else {
         reinterpret_cast<uint2 *>(a.out)[static_cast<size_t>(row) * a.samples + t0 + s] =
-            resolve(a, pos, t0 + s);
+            fresh ? make_uint2(kNone, kNone) : make_uint2(fs.k[s], fs.t[s]);
       }
     }
     __syncwarp();
@@ -270,34 +297,38 @@ __device__ __forceinline__ bool filter_item(const HashArgs &a, uint32_t c, uint3
   // Windows start at multiples of 32 positions (16-byte aligned bulk copies
   // of every array), the first one possibly before the chunk.
   const uint32_t w0 = cs & ~31u;
-  const uint32_t nwin = ce > cs ? (ce - w0 + kFWin - 1) / kFWin : 0;
-  if (nwin > 0) issue_window<PACKED>(a, stg, wc.pk, 0, w0, min(kFWin, ce - w0), bulk_ok, lane);
-  if (nwin > 1)
-    issue_window<PACKED>(a, stg, wc.pk, 1, w0 + kFWin, min(kFWin, ce - w0 - kFWin), bulk_ok, lane);
-  auto drain_copies = [&](uint32_t from) {
-    for (uint32_t kk = from; kk < nwin && kk < from + 2; ++kk) {
-      const uint32_t bb = kk & 1u;
-      for (uint32_t spins = 0; !mbar_try_wait(&stg.bar[bb], (parity >> bb) & 1u);)
+  auto issue = [&](uint32_t at, uint32_t buf) {
+    if (at < ce) issue_window<PACKED>(a, stg, wc.pk, buf, at, min(kFWin, ce - at), bulk_ok, lane);
+  };
+  if (ce > cs) {
+    issue(w0, 0);
+    issue(w0 + kFWin, 1);
+  }
+  // Error exits wait (bounded) for the copies still in flight, those of the
+  // windows at `from` and behind it.
+  auto drain_copies = [&](uint32_t from, uint32_t buf) {
+    for (uint32_t kk = 0; kk < 2 && from < ce; ++kk, from += kFWin, buf ^= 1u) {
+      for (uint32_t spins = 0; !mbar_try_wait(&stg.bar[buf], (parity >> buf) & 1u);)
         if (++spins > kSpinLimit) break;
-      parity ^= 1u << bb;
+      parity ^= 1u << buf;
     }
   };
 
-  for (uint32_t k = 0; k < nwin; ++k) {
-    const uint32_t b = k & 1u;
-    const uint32_t ws = w0 + k * kFWin;
+  uint32_t b = 0;
+  uint32_t i = cs - w0;
+  for (uint32_t ws = w0; ws < ce && ce > cs; ws += kFWin, b ^= 1u, i = 0) {
     const uint32_t n = min(kFWin, ce - ws);
     if (!finish_window<PACKED>(a, stg, wc.pk, b, (parity >> b) & 1u, ws, n, bulk_ok, lane)) {
       if (lane == 0) atomicOr(a.status, kStatusStall);
-      drain_copies(k);
+      drain_copies(ws, b);
       return false;
     }
     parity ^= 1u << b;
     const float *__restrict__ lw = stg.w[b];
     uint32_t *__restrict__ cl = stg.c[b];
-    for (uint32_t i = lane; i < n; i += 32) fs.l[i] = quant_up(lw[i]) * 65537;
+    for (uint32_t p = lane; p < n; p += 32) fs.l[p] = quant_up(lw[p]) * 65537;
     // Entries past the window's end in its last batch: column 0, masked off.
-    for (uint32_t i = n + lane; i < ((n + GRP - 1) & ~(GRP - 1)); i += 32) cl[i] = 0;
+    for (uint32_t p = n + lane; p < ((n + GRP - 1) & ~(GRP - 1)); p += 32) cl[p] = 0;
     __syncwarp();
 
     // Evaluates queued candidates from the end, kEvalDepth per lane at a time,
@@ -317,49 +348,61 @@ __device__ __forceinline__ bool filter_item(const HashArgs &a, uint32_t c, uint3
           lc[j] = __ldg(p + 2);
           be[j] = __ldg(p + 4);
         }
-        // The minimum first, then the position of whoever holds it: the one
-        // lane that brought the value stores its own, equal values (ties,
-        // also with an earlier minimum) lower it to the earliest.
+        // The minimum first, then position and pair of whoever holds it: the one
+        // lane that brought the value stores its own; of equal values (ties, also
+        // with an earlier minimum) the earliest position stores over it.
         uint32_t x[kEvalDepth];
+        float t[kEvalDepth];
         bool brought[kEvalDepth];
 #pragma unroll
         for (uint32_t j = 0; j < kEvalDepth; ++j) {
-          const float ln_a = exact_ln_a(lw[e[j] & 0xFFu], r[j], lc[j], be[j]);
+          const float ln_a = exact_ln_a(lw[e[j] & 0xFFu], r[j], lc[j], be[j], t[j]);
           x[j] = from + 32 * j + lane < count && ln_a < FLT_MAX ? ordered(ln_a) : 0xFFFFFFFFu;
           brought[j] = x[j] < atomicMin(&fs.val[e[j] >> 8], x[j]);
         }
         __syncwarp();
+        auto store = [&](uint32_t j) {
+          fs.pos[e[j] >> 8] = ws + (e[j] & 0xFFu);
+          fs.k[e[j] >> 8] = cl[e[j] & 0xFFu];
+          fs.t[e[j] >> 8] = whole(t[j]);
+        };
         bool tie = false;
 #pragma unroll
         for (uint32_t j = 0; j < kEvalDepth; ++j) {
           const bool holds = fs.val[e[j] >> 8] == x[j];
-          if (holds && brought[j]) fs.pos[e[j] >> 8] = ws + (e[j] & 0xFFu);
+          if (holds && brought[j]) store(j);
           brought[j] = holds && !brought[j];
           tie |= brought[j];
         }
         if (__any_sync(0xFFFFFFFFu, tie)) {
           __syncwarp();
 #pragma unroll
+          for (uint32_t j = 0; j < kEvalDepth; ++j) {
+            const uint32_t pos = ws + (e[j] & 0xFFu);
+            if (brought[j]) brought[j] = pos < atomicMin(&fs.pos[e[j] >> 8], pos);
+          }
+          __syncwarp();
+#pragma unroll
           for (uint32_t j = 0; j < kEvalDepth; ++j)
-            if (brought[j]) atomicMin(&fs.pos[e[j] >> 8], ws + (e[j] & 0xFFu));
+            if (brought[j] && fs.pos[e[j] >> 8] == ws + (e[j] & 0xFFu)) store(j);
         }
         __syncwarp();
         count = from;
       } while (count > leave);
     };
 
-    uint32_t i = k == 0 ? cs - w0 : 0;
     while (i < n) {
       while (ws + i >= row_end) {
         flush(row_end);
-        if (r_next >= r_stop) {  // only reachable with inconsistent offsets
+        if (r_next >= fs.r_stop) {  // only reachable with inconsistent offsets
           if (lane == 0) atomicOr(a.status, kStatusBadIndptr);
-          drain_copies(k + 1);
+          drain_copies(ws + kFWin, b ^ 1u);
           return false;
         }
         row = r_next++;
-        row_begin = row_end;
-        row_end = a.indptr[row + 1] - base;
+        if (lane == 0) fs.row_begin = row_end;
+        __syncwarp();
+        row_end = a.indptr[row + 1] - a.indptr[0];
         head = false;
         fresh = true;
       }
@@ -368,18 +411,14 @@ __device__ __forceinline__ bool filter_item(const HashArgs &a, uint32_t c, uint3
         // First look at the row: no minima yet, thresholds at the guess.
         fresh = false;
         thr_guess = kThrOpen;
-        thr_floor = 0;
         if (guessing) {
           float sum = 0.0f;
           const uint32_t end = min(row_end, ce);
 #pragma unroll 8
-          for (uint32_t p = row_begin + lane; p < end; p += 32) sum += fmaxf(a.weights[p], 0.0f);
+          for (uint32_t p = fs.row_begin + lane; p < end; p += 32) sum += fmaxf(a.weights[p], 0.0f);
 #pragma unroll
           for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xFFFFFFFFu, sum, o);
-          if (sum > 0.0f && sum < FLT_MAX) {
-            thr_guess = threshold(__logf(kGuess / sum));
-            thr_floor = thr_guess - kThrSpread;
-          }
+          if (sum > 0.0f && sum < FLT_MAX) thr_guess = threshold(__logf(kGuess / sum));
         }
         thr_min = thr_guess;
 #pragma unroll
@@ -388,6 +427,8 @@ __device__ __forceinline__ bool filter_item(const HashArgs &a, uint32_t c, uint3
         for (uint32_t v = 0; v < TILE / 32; ++v) {
           fs.val[v * 32 + lane] = ordered(FLT_MAX);
           fs.pos[v * 32 + lane] = kNone;
+          fs.k[v * 32 + lane] = kNone;
+          fs.t[v * 32 + lane] = kNone;
         }
         __syncwarp();
       }
@@ -488,10 +529,13 @@ __device__ __forceinline__ bool filter_item(const HashArgs &a, uint32_t c, uint3
             refresh();
           }
         } else {
-          // More than the queue has room for: by quarters of at most 1024.
+          // More than the queue has room for: at most 512 at a time, four
+          // entries of four samples per lane.
 #pragma unroll 1
-          for (uint32_t v = 0; v < 4; ++v) {
-            const uint32_t m = v == 0 ? hits[0] : v == 1 ? hits[1] : v == 2 ? hits[2] : hits[3];
+          for (uint32_t part = 0; part < 8; ++part) {
+            const uint32_t v = part >> 1;
+            const uint32_t m = (v == 0 ? hits[0] : v == 1 ? hits[1] : v == 2 ? hits[2] : hits[3]) &
+                               (part & 1u ? 0xF0F0F0F0u : 0x0F0F0F0Fu);
             const uint32_t in2 = warp_prefix(__popc(m), lane);
             const uint32_t sum2 = __shfl_sync(0xFFFFFFFFu, in2, 31);
             if (count + sum2 > kQueue) {
@@ -511,13 +555,10 @@ __device__ __forceinline__ bool filter_item(const HashArgs &a, uint32_t c, uint3
       }
       i = seg;
     }
-    if (k + 2 < nwin) {
-      const uint32_t ws2 = ws + 2 * kFWin;
-      issue_window<PACKED>(a, stg, wc.pk, b, ws2, min(kFWin, ce - ws2), bulk_ok, lane);
-    }
+    issue(ws + 2 * kFWin, b);
   }
   flush(min(row_end, ce));
-  while (r_next < r_stop) {  // trailing empty rows of the last chunk
+  while (r_next < fs.r_stop) {  // trailing empty rows of the last chunk
     row = r_next++;
     row_end = ce;
     head = false;
