@@ -301,9 +301,9 @@ bool tuned_choice(const Gen *gen, uint64_t nnz, uint64_t rows, TuneChoice *out,
 
 // The filtered kernel evaluates 11-17 candidates per (row, sample) whatever the
 // row's length, the dense one every entry.  Measured on 8M entries in uniform
-// rows, 128 samples (ms, dense / filtered): rows of 60 entries 2.24 / 2.47, of
-// 80 2.15 / 1.97, of 100 2.11 / 1.72, of 120 2.07 / 1.6.
-constexpr uint32_t kFilterMinRow = 72;
+// rows, 128 samples (ms, dense / filtered): rows of 60 entries 1.99 / 2.52, of
+// 80 1.97 / 2.02, of 100 1.95 / 1.77, of 120 1.94 / 1.54.
+constexpr uint32_t kFilterMinRow = 88;
 // Below it a launch is over before the chip is full: 30,000 entries in
 // 300-entry rows 31 / 34 us, 90,000 entries 69 / 51 us.
 constexpr uint64_t kFilterMinEvals = 1ull << 23;
@@ -312,6 +312,11 @@ constexpr uint64_t kFilterMinEvals = 1ull << 23;
 // the CSR.  3,000 rows of 1400 entries (1417 per warp): 485 us whole, 408
 // halved; 20,011 rows of 300 (2030 per warp): 481 whole, 567 halved.
 constexpr uint64_t kFilterShare = 1500;
+
+// Mean rows below which the dense kernel keeps t with each minimum (RowState):
+// rows of 20 entries 2.64 -> 2.21 ms, of 60 2.27 -> 1.99, of 420 (heavy tail,
+// 256 samples) 6.14 -> 5.86; rows of 1400 Zipf entries 27.9 -> 28.5.
+constexpr uint64_t kKeepMaxRow = 512;
 
 // Whether a launch takes the bound-filtered kernel (filter_kernels.cu).
 bool use_filter(const Gen *gen, uint64_t nnz, uint64_t rows, const TuneChoice *tuned) {
@@ -392,6 +397,7 @@ HashPlan make_plan(const Gen *gen, uint64_t nnz, uint64_t rows, const TuneChoice
     const uint64_t want = resident_warps * std::max<uint32_t>(1, min_items);
     chunk = std::min<uint64_t>(chunk, std::max<uint64_t>(64, (nnz * p.ntiles + want - 1) / want));
   }
+  p.keep = !p.filter && avg_row < kKeepMaxRow;
   const int forced = env_int("MHCUDA_B200_CHUNK", 0);
   if (forced > 0) chunk = static_cast<uint64_t>(forced);
   chunk = std::max<uint64_t>(64, (chunk + 31) & ~31ull);
@@ -1441,6 +1447,7 @@ enum MHCUDAResult mhcuda_calc_batch_device(const MinhashCudaGenerator *gen, uint
   // Kernel variant as for one large launch; the chunk size is chosen on the
   // device from the batch's nnz (batch_setup_kernel).
   HashPlan vp = make_plan(gen, 1ull << 30, 1ull << 20, nullptr, 8, false);
+  vp.keep = 1;
   HashPlan fp = vp;
   fp.filter = mhb::filter_lanes(gen->s_pad);
   fp.ntiles = mhb::filter_tiles(gen->s_pad, fp.filter);

@@ -92,11 +92,6 @@ __device__ __forceinline__ float exact_ln_a(float w, float r, float c, float b, 
   t = exact_t(w, r, b);
   return __fsub_rn(__fmaf_rn(-__fsub_rn(t, b), r, c), r);
 }
-// (uint32)(int32)t as kernel.cu:108; the conversion saturates.
-__device__ __forceinline__ uint32_t whole(float t) {
-  return static_cast<uint32_t>(static_cast<int32_t>(t));
-}
-
 // The sign bits of the four halves of (d0, d1), each spread over a byte (prmt
 // with the replicate-sign bit of its selectors, which __byte_perm masks off).
 __device__ __forceinline__ uint32_t half_signs(uint32_t d0, uint32_t d1) {
@@ -285,7 +280,7 @@ __device__ __forceinline__ bool filter_item(const HashArgs &a, uint32_t c, uint3
       if (partial) {
         const size_t off = static_cast<size_t>(2 * fs.chunk + (head ? 0 : 1)) * spad + t0 + s;
         a.part_ln[off] = fresh ? FLT_MAX : unordered(fs.val[s]);
-        a.part_kt[off] = make_uint2(fresh ? kNone : fs.pos[s], 0u);
+        a.part_kt[off] = make_uint2(fresh ? kNone : fs.pos[s], fresh ? kNone : fs.t[s]);
       } else {
         reinterpret_cast<uint2 *>(a.out)[static_cast<size_t>(row) * a.samples + t0 + s] =
             fresh ? make_uint2(kNone, kNone) : make_uint2(fs.k[s], fs.t[s]);

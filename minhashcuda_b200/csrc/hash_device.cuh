@@ -72,17 +72,6 @@ __device__ __forceinline__ uint32_t chunk_begin(const HashArgs &a, uint32_t c, u
   return e - at <= a.snap ? e : at;
 }
 
-// One (nnz, sample) evaluation, kernel.cu:101-109, given t: keeps the
-// minimum and the position `p` it came from.
-__device__ __forceinline__ void wmh_update(float t, float r, float c, float b, uint32_t p,
-                                           float &mn, uint32_t &pos) {
-  const float tb = __fsub_rn(t, b);
-  const float ln_a = __fsub_rn(__fmaf_rn(-tb, r, c), r);
-  const bool lt = ln_a < mn;
-  mn = lt ? ln_a : mn;
-  pos = lt ? p : pos;
-}
-
 // Column of relative position p in a packed CSR.
 __device__ __forceinline__ uint32_t packed_col(const HashArgs &a, uint32_t p) {
   const uint32_t h = a.col_hi_bits == 4 ? (a.cols_hi[p >> 1] >> ((p & 1u) * 4)) & 15u
@@ -90,12 +79,16 @@ __device__ __forceinline__ uint32_t packed_col(const HashArgs &a, uint32_t p) {
   return static_cast<uint32_t>(a.cols_lo[p]) | (h << 16);
 }
 
+// (uint32)(int32)t as kernel.cu:108; the GPU conversion saturates.
+__device__ __forceinline__ uint32_t whole(float t) {
+  return static_cast<uint32_t>(static_cast<int32_t>(t));
+}
+
 // The output pair of kernel.cu:108 for sample s whose minimum came from the
 // entry at relative position `pos`: k = cols[pos] and t recomputed from the
 // entry with the exact quotient.  Every evaluation used that same t (fast_t
 // only decides t when it equals the exact one), so tracking the position
 // instead of (k, t) changes nothing but the work per evaluation.
-// (uint32)(int32)t as kernel.cu:108; the GPU conversion saturates.
 // A position outside [0, nnz) (none found, or a partial that a failed launch
 // left unwritten) yields kNone and reads nothing.
 __device__ __forceinline__ uint2 resolve(const HashArgs &a, uint32_t pos, uint32_t s) {
@@ -107,40 +100,72 @@ __device__ __forceinline__ uint2 resolve(const HashArgs &a, uint32_t pos, uint32
   const float w = logf(a.weights[pos]);
   const float *col = a.params + static_cast<size_t>(k) * 3 * a.s_pad + param_index(s);
   const float t = exact_t(w, col[0], col[4]);
-  return make_uint2(k, static_cast<uint32_t>(static_cast<int32_t>(t)));
+  return make_uint2(k, whole(t));
 }
 
-template <int SPL>
+// KEEP: the minimum's t is kept beside its position (one select per
+// evaluation, a register per sample), so that the end of a row does not
+// recompute it: three gathers, a logarithm and a division per (row, sample).
+template <int SPL, bool KEEP>
 struct RowState {
   float mn[SPL];
   uint32_t pos[SPL];  // relative position of the minimum, kNone if none
+  float t[KEEP ? SPL : 1];
   __device__ __forceinline__ void reset() {
 #pragma unroll
     for (int j = 0; j < SPL; ++j) {
       mn[j] = FLT_MAX;
       pos[j] = kNone;
+      if constexpr (KEEP) t[j] = 0.0f;
     }
+  }
+  // One (nnz, sample) evaluation, kernel.cu:106-109, given ln_a.
+  __device__ __forceinline__ void update(int j, float ln_a, float tj, uint32_t p) {
+    const bool lt = ln_a < mn[j];
+    mn[j] = lt ? ln_a : mn[j];
+    pos[j] = lt ? p : pos[j];
+    if constexpr (KEEP) t[j] = lt ? tj : t[j];
   }
 };
 
-template <int SPL>
+// win: the staged columns of the positions from `ws` on.
+template <int SPL, bool KEEP>
 __device__ __forceinline__ void store_final(const HashArgs &a, uint32_t row, uint32_t s0,
-                                            const RowState<SPL> &st) {
+                                            const RowState<SPL, KEEP> &st,
+                                            const uint32_t *__restrict__ win, uint32_t ws) {
   uint32_t *o = a.out + (static_cast<size_t>(row) * a.samples + s0) * 2;
 #pragma unroll
   for (int j = 0; j < SPL; ++j) {
-    if (s0 + j < a.samples) *reinterpret_cast<uint2 *>(o + 2 * j) = resolve(a, st.pos[j], s0 + j);
+    uint2 kt;
+    if constexpr (KEEP) {
+      kt = make_uint2(kNone, kNone);
+      if (st.pos[j] < a.nnz) {
+        const uint32_t k = st.pos[j] >= ws ? win[st.pos[j] - ws]
+                           : a.col_hi_bits ? packed_col(a, st.pos[j])
+                                           : a.cols[st.pos[j]];
+        kt = make_uint2(k, whole(st.t[j]));
+      }
+    } else {
+      kt = resolve(a, st.pos[j], s0 + j);
+    }
+    if (s0 + j < a.samples) *reinterpret_cast<uint2 *>(o + 2 * j) = kt;
   }
 }
 
-template <int SPL>
+template <int SPL, bool KEEP>
 __device__ __forceinline__ void store_partial(const HashArgs &a, uint32_t slot, uint32_t s0,
-                                              const RowState<SPL> &st) {
+                                              const RowState<SPL, KEEP> &st) {
   const size_t off = static_cast<size_t>(slot) * a.s_pad + s0;
 #pragma unroll
   for (int j = 0; j < SPL; ++j) {
+    uint32_t t;
+    if constexpr (KEEP) {
+      t = whole(st.t[j]);
+    } else {
+      t = resolve(a, st.pos[j], s0 + j).y;
+    }
     a.part_ln[off + j] = st.mn[j];
-    a.part_kt[off + j] = make_uint2(st.pos[j], 0u);
+    a.part_kt[off + j] = make_uint2(st.pos[j], t);
   }
 }
 
@@ -373,21 +398,9 @@ __device__ __forceinline__ F2 fma2(F2 a, F2 b, F2 c) {
   return r;
 }
 
-// Selects for samples j and j+1 given their ln_a pair (position p).
-template <int SPL>
-__device__ __forceinline__ void update_pair(F2 ln_a, uint32_t p, int j, RowState<SPL> &st) {
-  float l0, l1;
-  split(ln_a, l0, l1);
-  const bool lt0 = l0 < st.mn[j], lt1 = l1 < st.mn[j + 1];
-  st.mn[j] = lt0 ? l0 : st.mn[j];
-  st.pos[j] = lt0 ? p : st.pos[j];
-  st.mn[j + 1] = lt1 ? l1 : st.mn[j + 1];
-  st.pos[j + 1] = lt1 ? p : st.pos[j + 1];
-}
-
-template <int SPL>
+template <int SPL, bool KEEP>
 __device__ __forceinline__ void eval_all(const Params<SPL> &p, float w, uint32_t pos, bool active,
-                                         RowState<SPL> &st) {
+                                         RowState<SPL, KEEP> &st) {
   float t[SPL];
   bool undecided = false;
   if constexpr (SPL % 2 == 0) {
@@ -436,12 +449,17 @@ __device__ __forceinline__ void eval_all(const Params<SPL> &p, float w, uint32_t
       const F2 rr = f2(p.r.v[j], p.r.v[j + 1]);
       const F2 nb = sub2(f2(p.b.v[j], p.b.v[j + 1]), f2(t[j], t[j + 1]));
       const F2 ln_a = sub2(fma2(nb, rr, f2(p.c.v[j], p.c.v[j + 1])), rr);
-      update_pair<SPL>(ln_a, pos, j, st);
+      float l0, l1;
+      split(ln_a, l0, l1);
+      st.update(j, l0, t[j], pos);
+      st.update(j + 1, l1, t[j + 1], pos);
     }
   } else {
 #pragma unroll
-    for (int j = 0; j < SPL; ++j)
-      wmh_update(t[j], p.r.v[j], p.c.v[j], p.b.v[j], pos, st.mn[j], st.pos[j]);
+    for (int j = 0; j < SPL; ++j) {
+      const float tb = __fsub_rn(t[j], p.b.v[j]);
+      st.update(j, __fsub_rn(__fmaf_rn(-tb, p.r.v[j], p.c.v[j]), p.r.v[j]), t[j], pos);
+    }
   }
 }
 

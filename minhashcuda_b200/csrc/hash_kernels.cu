@@ -93,7 +93,7 @@ __host__ __device__ constexpr int param_depth(int minb) { return minb == 2 ? 3 :
 // wide multiply-add and immediate load offsets.
 // DEPTH: parameter sets in registers, 2 (the next position is loaded while
 // one is evaluated) or 3 (the next two are), see param_depth.
-template <int SPL, int SPAD, bool PACKED, int DEPTH>
+template <int SPL, int SPAD, bool PACKED, int DEPTH, bool KEEP>
 __device__ __forceinline__ bool hash_item(const HashArgs &a, uint32_t c, uint32_t tile,
                                           WarpCtx &wc) {
   const uint32_t lane = wc.lane;
@@ -132,17 +132,19 @@ __device__ __forceinline__ bool hash_item(const HashArgs &a, uint32_t c, uint32_
         head = true;
       }
     }
-    RowState<SPL> st;
+    RowState<SPL, KEEP> st;
     st.reset();
+    const uint32_t *win = stg.c[0];  // the window last staged and its first position
+    uint32_t win_at = cs;
 
     auto flush = [&]() {
       if (row == kNone || !active) return;
       if (head) {
-        store_partial<SPL>(a, 2 * c, s0, st);
+        store_partial(a, 2 * c, s0, st);
       } else if (row_end > ce) {
-        store_partial<SPL>(a, 2 * c + 1, s0, st);
+        store_partial(a, 2 * c + 1, s0, st);
       } else {
-        store_final<SPL>(a, row, s0, st);
+        store_final(a, row, s0, st, win, win_at);
       }
     };
 
@@ -174,6 +176,8 @@ __device__ __forceinline__ bool hash_item(const HashArgs &a, uint32_t c, uint32_
       parity ^= 1u << b;
       const float *__restrict__ lw = stg.w[b];
       const uint32_t *__restrict__ cl = stg.c[b];
+      win = stg.c[b];
+      win_at = ws;
 
       // Columns in the window are < dim, and slots n and n + 1 hold column 0
       // (finish_window).
@@ -201,22 +205,22 @@ __device__ __forceinline__ bool hash_item(const HashArgs &a, uint32_t c, uint32_
           const uint32_t seg = min(row_end - ws, n);
           while (i + 3 <= seg) {  // prefetches reach i + 4 <= n + 1
             C.load(pbase + cl[i + 2] * col_stride);
-            eval_all<SPL>(A, lw[i], ws + i, active, st);
+            eval_all(A, lw[i], ws + i, active, st);
             A.load(pbase + cl[i + 3] * col_stride);
-            eval_all<SPL>(B, lw[i + 1], ws + i + 1, active, st);
+            eval_all(B, lw[i + 1], ws + i + 1, active, st);
             B.load(pbase + cl[i + 4] * col_stride);
-            eval_all<SPL>(C, lw[i + 2], ws + i + 2, active, st);
+            eval_all(C, lw[i + 2], ws + i + 2, active, st);
             i += 3;
           }
           if (i + 2 == seg) {
             C.load(pbase + cl[i + 2] * col_stride);
-            eval_all<SPL>(A, lw[i], ws + i, active, st);
-            eval_all<SPL>(B, lw[i + 1], ws + i + 1, active, st);
+            eval_all(A, lw[i], ws + i, active, st);
+            eval_all(B, lw[i + 1], ws + i + 1, active, st);
             i += 2;
             A = C;
             B.load(pbase + cl[i + 1] * col_stride);
           } else if (i + 1 == seg) {
-            eval_all<SPL>(A, lw[i], ws + i, active, st);
+            eval_all(A, lw[i], ws + i, active, st);
             i += 1;
             A = B;
             B.load(pbase + cl[i + 1] * col_stride);
@@ -252,16 +256,16 @@ __device__ __forceinline__ bool hash_item(const HashArgs &a, uint32_t c, uint32_
         while (i + 1 < seg) {  // i + 2 <= n
           dB = cl[i + 1];
           B.load(pbase + dB * col_stride);
-          eval_all<SPL>(A, lw[i], ws + i, active, st);
+          eval_all(A, lw[i], ws + i, active, st);
           dA = cl[i + 2];
           A.load(pbase + dA * col_stride);
-          eval_all<SPL>(B, lw[i + 1], ws + i + 1, active, st);
+          eval_all(B, lw[i + 1], ws + i + 1, active, st);
           i += 2;
         }
         if (i < seg) {  // i + 1 <= n
           dB = cl[i + 1];
           B.load(pbase + dB * col_stride);
-          eval_all<SPL>(A, lw[i], ws + i, active, st);
+          eval_all(A, lw[i], ws + i, active, st);
           ++i;
           A = B;
           dA = dB;
@@ -287,7 +291,7 @@ __device__ __forceinline__ bool hash_item(const HashArgs &a, uint32_t c, uint32_
 }
 
 // PACKED: the columns arrive as cols_lo/cols_hi (HashArgs::col_hi_bits).
-template <int SPL, int MINB, int SPAD, bool PACKED>
+template <int SPL, int MINB, int SPAD, bool PACKED, bool KEEP>
 __global__ void __launch_bounds__(kHashBlock, MINB) hash_kernel(const HashArgs a) {
   __shared__ WarpStage stage_all[kHashBlock / 32];
   PackedStage *packed = nullptr;
@@ -303,7 +307,7 @@ __global__ void __launch_bounds__(kHashBlock, MINB) hash_kernel(const HashArgs a
   const uint32_t items = a.nchunks * a.ntiles;
   for (uint32_t item = gw; item < items; item += nw) {
     const uint32_t c = item / a.ntiles;
-    if (!hash_item<SPL, SPAD, PACKED, param_depth(MINB)>(a, c, item - c * a.ntiles, wc)) return;
+    if (!hash_item<SPL, SPAD, PACKED, param_depth(MINB), KEEP>(a, c, item - c * a.ntiles, wc)) return;
   }
 }
 
@@ -331,34 +335,40 @@ __device__ __forceinline__ void finalize_item(const HashArgs &a, uint32_t c, uin
   const size_t stride = 2 * static_cast<size_t>(a.s_pad);  // one chunk's two slots
   size_t off = static_cast<size_t>(2 * c + 1) * a.s_pad + s;
   float mn = a.part_ln[off];
-  uint32_t kp = a.part_kt[off].x;
+  uint2 kt = a.part_kt[off];  // position and t
   off = static_cast<size_t>(2 * (c + 1)) * a.s_pad + s;
   uint32_t cc = c + 1;
   for (; cc + kFinalizeUnroll - 1 <= c_last; cc += kFinalizeUnroll) {
     float m[kFinalizeUnroll];
-    uint32_t k[kFinalizeUnroll];
+    uint2 k[kFinalizeUnroll];
 #pragma unroll
     for (uint32_t u = 0; u < kFinalizeUnroll; ++u) {
       m[u] = a.part_ln[off + u * stride];
-      k[u] = a.part_kt[off + u * stride].x;
+      k[u] = a.part_kt[off + u * stride];
     }
 #pragma unroll
     for (uint32_t u = 0; u < kFinalizeUnroll; ++u) {
       const bool lt = m[u] < mn;
       mn = lt ? m[u] : mn;
-      kp = lt ? k[u] : kp;
+      kt.x = lt ? k[u].x : kt.x;
+      kt.y = lt ? k[u].y : kt.y;
     }
     off += kFinalizeUnroll * stride;
   }
   for (; cc <= c_last; ++cc, off += stride) {
     const float m2 = a.part_ln[off];
-    const uint32_t k2 = a.part_kt[off].x;
+    const uint2 k2 = a.part_kt[off];
     const bool lt = m2 < mn;
     mn = lt ? m2 : mn;
-    kp = lt ? k2 : kp;
+    kt = lt ? k2 : kt;
   }
   uint32_t *o = a.out + (static_cast<size_t>(row) * a.samples + s) * 2;
-  *reinterpret_cast<uint2 *>(o) = resolve(a, kp, s);
+  if (kt.x >= a.nnz) {
+    kt = make_uint2(kNone, kNone);
+  } else {
+    kt.x = a.col_hi_bits ? packed_col(a, kt.x) : a.cols[kt.x];
+  }
+  *reinterpret_cast<uint2 *>(o) = kt;
 }
 
 __global__ void finalize_kernel(const HashArgs a) {
@@ -523,7 +533,7 @@ __global__ void batch_plan_kernel(const BatchArgs b, uint32_t plan_threads) {
 // The matrix view of an item is kept in shared memory, one per warp: its
 // fields are read where the item needs them (per row or window), so the
 // evaluation loop's registers are the single-matrix kernel's.
-template <int SPL, int MINB, int SPAD>
+template <int SPL, int MINB, int SPAD, bool KEEP>
 __global__ void __launch_bounds__(kHashBlock, MINB) hash_batch_kernel(const BatchArgs b) {
   __shared__ WarpStage stage_all[kHashBlock / 32];
   __shared__ HashArgs views[kHashBlock / 32];
@@ -543,7 +553,7 @@ __global__ void __launch_bounds__(kHashBlock, MINB) hash_batch_kernel(const Batc
     __syncwarp();
     if (wc.lane == 0) view = matrix_view(b, b.mats[m], chunk);
     __syncwarp();
-    if (!hash_item<SPL, SPAD, false, param_depth(MINB)>(view, gc - base, item - gc * ntiles, wc))
+    if (!hash_item<SPL, SPAD, false, param_depth(MINB), KEEP>(view, gc - base, item - gc * ntiles, wc))
       return;
   }
 }
@@ -586,75 +596,52 @@ namespace {
 using HashFn = void (*)(const HashArgs);
 using BatchFn = void (*)(const BatchArgs);
 
-BatchFn pick_batch(uint32_t spl, uint32_t minb, uint32_t s_pad) {
-  switch (spl * 100000 + minb * 10000 + s_pad) {
-    case 440128: return hash_batch_kernel<4, 4, 128>;
-    case 430128: return hash_batch_kernel<4, 3, 128>;
-    case 420128: return hash_batch_kernel<4, 2, 128>;
-    case 440256: return hash_batch_kernel<4, 4, 256>;
-    case 430256: return hash_batch_kernel<4, 3, 256>;
-    case 420256: return hash_batch_kernel<4, 2, 256>;
-    case 240064: return hash_batch_kernel<2, 4, 64>;
-    default: break;
-  }
-  switch (spl * 10 + minb) {
-    case 44: return hash_batch_kernel<4, 4, 0>;
-    case 43: return hash_batch_kernel<4, 3, 0>;
-    case 42: return hash_batch_kernel<4, 2, 0>;
-    case 24: return hash_batch_kernel<2, 4, 0>;
-    case 14: return hash_batch_kernel<1, 4, 0>;
-    default: return nullptr;
-  }
-}
-
 // Instantiated (samples per lane, minimum resident blocks per SM) variants,
-// with s_pad compiled in for the common sample counts.
-HashFn pick_hash(uint32_t spl, uint32_t minb, uint32_t s_pad, bool packed = false) {
-  if (packed) {
-    switch (spl * 100000 + minb * 10000 + s_pad) {
-      case 440128: return hash_kernel<4, 4, 128, true>;
-      case 430128: return hash_kernel<4, 3, 128, true>;
-      case 420128: return hash_kernel<4, 2, 128, true>;
-      case 440256: return hash_kernel<4, 4, 256, true>;
-      case 430256: return hash_kernel<4, 3, 256, true>;
-      case 420256: return hash_kernel<4, 2, 256, true>;
-      case 240064: return hash_kernel<2, 4, 64, true>;
-      default: break;
-    }
-    switch (spl * 10 + minb) {
-      case 44: return hash_kernel<4, 4, 0, true>;
-      case 43: return hash_kernel<4, 3, 0, true>;
-      case 42: return hash_kernel<4, 2, 0, true>;
-      case 24: return hash_kernel<2, 4, 0, true>;
-      case 14: return hash_kernel<1, 4, 0, true>;
-      default: return nullptr;
-    }
+// with s_pad compiled in for the common sample counts.  The 4-block ones come
+// with and without KEEP.
+#define MHB_PICK(KERNEL, ...)                                      \
+  switch (spl * 100000 + minb * 10000 + s_pad) {                   \
+    case 440128: return KERNEL<4, 4, 128, __VA_ARGS__ KEEP>;       \
+    case 440256: return KERNEL<4, 4, 256, __VA_ARGS__ KEEP>;       \
+    case 240064: return KERNEL<2, 4, 64, __VA_ARGS__ KEEP>;        \
+    case 430128: return KERNEL<4, 3, 128, __VA_ARGS__ false>;      \
+    case 420128: return KERNEL<4, 2, 128, __VA_ARGS__ false>;      \
+    case 430256: return KERNEL<4, 3, 256, __VA_ARGS__ false>;      \
+    case 420256: return KERNEL<4, 2, 256, __VA_ARGS__ false>;      \
+    default: break;                                                \
+  }                                                                \
+  switch (spl * 10 + minb) {                                       \
+    case 44: return KERNEL<4, 4, 0, __VA_ARGS__ KEEP>;             \
+    case 24: return KERNEL<2, 4, 0, __VA_ARGS__ KEEP>;             \
+    case 14: return KERNEL<1, 4, 0, __VA_ARGS__ KEEP>;             \
+    case 43: return KERNEL<4, 3, 0, __VA_ARGS__ false>;            \
+    case 42: return KERNEL<4, 2, 0, __VA_ARGS__ false>;            \
+    default: return nullptr;                                       \
   }
-  switch (spl * 100000 + minb * 10000 + s_pad) {
-    case 440128: return hash_kernel<4, 4, 128, false>;
-    case 430128: return hash_kernel<4, 3, 128, false>;
-    case 420128: return hash_kernel<4, 2, 128, false>;
-    case 440256: return hash_kernel<4, 4, 256, false>;
-    case 430256: return hash_kernel<4, 3, 256, false>;
-    case 420256: return hash_kernel<4, 2, 256, false>;
-    case 240064: return hash_kernel<2, 4, 64, false>;
-    default: break;
-  }
-  switch (spl * 10 + minb) {
-    case 44: return hash_kernel<4, 4, 0, false>;
-    case 43: return hash_kernel<4, 3, 0, false>;
-    case 42: return hash_kernel<4, 2, 0, false>;
-    case 24: return hash_kernel<2, 4, 0, false>;
-    case 14: return hash_kernel<1, 4, 0, false>;
-    default: return nullptr;
-  }
+#define MHB_COMMA ,
+
+template <bool KEEP>
+BatchFn pick_batch(uint32_t spl, uint32_t minb, uint32_t s_pad) {
+  MHB_PICK(hash_batch_kernel)
+}
+template <bool PACKED, bool KEEP>
+HashFn pick_hash(uint32_t spl, uint32_t minb, uint32_t s_pad) {
+  MHB_PICK(hash_kernel, PACKED MHB_COMMA)
+}
+#undef MHB_COMMA
+#undef MHB_PICK
+
+HashFn pick_hash(uint32_t spl, uint32_t minb, uint32_t s_pad, bool packed, bool keep) {
+  if (packed)
+    return keep ? pick_hash<true, true>(spl, minb, s_pad) : pick_hash<true, false>(spl, minb, s_pad);
+  return keep ? pick_hash<false, true>(spl, minb, s_pad) : pick_hash<false, false>(spl, minb, s_pad);
 }
 
 }  // namespace
 
 cudaError_t launch_hash(const HashArgs &a, const HashPlan &plan, cudaStream_t stream) {
   if (plan.filter) return launch_filter(a, plan, stream);
-  const HashFn fn = pick_hash(plan.spl, plan.minb, a.s_pad, a.col_hi_bits != 0);
+  const HashFn fn = pick_hash(plan.spl, plan.minb, a.s_pad, a.col_hi_bits != 0, plan.keep != 0);
   if (!fn) return cudaErrorInvalidValue;
   fn<<<plan.grid, kHashBlock, 0, stream>>>(a);
   return cudaGetLastError();
@@ -671,7 +658,8 @@ cudaError_t launch_finalize(const HashArgs &a, cudaStream_t stream) {
 
 cudaError_t launch_batch(const BatchArgs &b, const HashPlan &dense, const HashPlan &filtered,
                          uint32_t plan_threads, cudaStream_t stream) {
-  const BatchFn fn = pick_batch(dense.spl, dense.minb, b.base.s_pad);
+  const BatchFn fn = dense.keep ? pick_batch<true>(dense.spl, dense.minb, b.base.s_pad)
+                                : pick_batch<false>(dense.spl, dense.minb, b.base.s_pad);
   if (!fn || b.count == 0 || b.max_chunks == 0) return cudaErrorInvalidValue;
   batch_setup_kernel<<<1, kSetupThreads, 0, stream>>>(b);
   if (plan_threads)
@@ -689,7 +677,7 @@ cudaError_t launch_batch(const BatchArgs &b, const HashPlan &dense, const HashPl
 }
 
 int hash_blocks_per_sm(uint32_t spl, uint32_t minb, uint32_t s_pad) {
-  const HashFn fn = pick_hash(spl, minb, s_pad);
+  const HashFn fn = pick_hash(spl, minb, s_pad, false, false);
   int n = 0;
   if (!fn || cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, fn, kHashBlock, 0) != cudaSuccess) {
     cudaGetLastError();
@@ -703,7 +691,7 @@ int plan_blocks_per_sm(const HashPlan &plan, uint32_t s_pad) {
 }
 
 size_t hash_kernel_registers(uint32_t spl, uint32_t minb, uint32_t s_pad) {
-  const HashFn fn = pick_hash(spl, minb, s_pad);
+  const HashFn fn = pick_hash(spl, minb, s_pad, false, false);
   cudaFuncAttributes attr{};
   if (!fn || cudaFuncGetAttributes(&attr, fn) != cudaSuccess) return 0;
   return attr.numRegs;

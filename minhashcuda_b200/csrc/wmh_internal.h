@@ -47,6 +47,7 @@ struct HashPlan {
   uint32_t filter;   // 0: the dense kernel; 8, 4, 2: the bound-filtered one
                      // (filter_kernels.cu) with that many lanes per entry
   uint32_t snap;     // HashArgs::snap
+  uint32_t keep;     // dense, 4 blocks per SM: t kept per minimum (RowState)
 };
 
 constexpr int kHashBlock = 256;
@@ -96,7 +97,7 @@ struct HashArgs {
   uint32_t ntiles;
   uint32_t *chunk_row;       // [nchunks] first row owned by each chunk
   float *part_ln;            // [2*nchunks][s_pad] partial minima
-  uint2 *part_kt;            // [2*nchunks][s_pad] partial (position of the minimum, 0)
+  uint2 *part_kt;            // [2*nchunks][s_pad] partial (position of the minimum, its t)
   uint32_t *out;             // [rows][samples][2]
   uint32_t *status;          // device status word
   uint32_t host_csr;         // weights/cols/indptr/out are mapped host memory
