@@ -14,6 +14,7 @@
 #include <algorithm>
 #include <atomic>
 #include <cinttypes>
+#include <condition_variable>
 #include <cstdarg>
 #include <cstdio>
 #include <cstdlib>
@@ -21,6 +22,7 @@
 #include <memory>
 #include <mutex>
 #include <string>
+#include <system_error>
 #include <thread>
 #include <unordered_map>
 #include <vector>
@@ -499,26 +501,97 @@ unsigned host_threads() {
   return forced > 0 ? static_cast<unsigned>(forced) : std::min(16u, hw);
 }
 
+// The host threads of one mhcuda_calc / mhcuda_calc_batch call, for staging
+// copies and conversions: started by its first parallel section and joined at
+// its end, since a section comes with every row block.  On a 16-core host the
+// sections of 14 blocks (40,000 rows of 1400 entries, pageable) each spent
+// about a third of their time starting and joining threads.
+class HostPool {
+ public:
+  HostPool() : n_(host_threads()) {}
+  HostPool(const HostPool &) = delete;
+  HostPool &operator=(const HostPool &) = delete;
+  ~HostPool() {
+    {
+      std::lock_guard<std::mutex> lock(mu_);
+      stop_ = true;
+    }
+    go_.notify_all();
+    for (auto &t : threads_) t.join();
+  }
+  unsigned threads() const { return n_; }
+  // Runs f(0) .. f(parts - 1) on the pool's threads and the caller's.
+  template <typename F>
+  void run(size_t parts, const F &f) {
+    if (parts > 1) start();
+    if (parts <= 1 || threads_.empty()) {
+      for (size_t p = 0; p < parts; ++p) f(p);
+      return;
+    }
+    {
+      std::lock_guard<std::mutex> lock(mu_);
+      job_ = [](const void *c, size_t p) { (*static_cast<const F *>(c))(p); };
+      ctx_ = &f;
+      parts_ = parts;
+      next_ = 0;
+      working_ = threads_.size();
+      ++round_;
+    }
+    go_.notify_all();
+    for (size_t p; (p = next_.fetch_add(1)) < parts;) f(p);
+    std::unique_lock<std::mutex> lock(mu_);
+    done_.wait(lock, [&] { return working_ == 0; });
+  }
+
+ private:
+  void start() {
+    try {
+      while (threads_.size() + 1 < n_) threads_.emplace_back([this]() { work(); });
+    } catch (const std::system_error &) {  // the threads there are do the work
+      n_ = static_cast<unsigned>(threads_.size()) + 1;
+    }
+  }
+  void work() {
+    uint64_t seen = 0;
+    std::unique_lock<std::mutex> lock(mu_);
+    for (;;) {
+      go_.wait(lock, [&] { return stop_ || round_ != seen; });
+      if (stop_) return;
+      seen = round_;
+      lock.unlock();
+      for (size_t p; (p = next_.fetch_add(1)) < parts_;) job_(ctx_, p);
+      lock.lock();
+      if (--working_ == 0) done_.notify_one();
+    }
+  }
+  unsigned n_;
+  std::vector<std::thread> threads_;
+  std::mutex mu_;
+  std::condition_variable go_, done_;
+  void (*job_)(const void *, size_t) = nullptr;
+  const void *ctx_ = nullptr;
+  size_t parts_ = 0;
+  std::atomic<size_t> next_{0};
+  size_t working_ = 0;
+  uint64_t round_ = 0;
+  bool stop_ = false;
+};
+
 // memcpy split over a few threads for large blocks (host bandwidth for the
 // pinned staging of pageable caller buffers).
-void par_memcpy(void *dst, const void *src, size_t bytes) {
+void par_memcpy(HostPool &pool, void *dst, const void *src, size_t bytes) {
   const size_t kSplit = static_cast<size_t>(8) << 20;
-  const unsigned n = bytes < kSplit ? 1u : host_threads();
+  const unsigned n = bytes < kSplit ? 1u : pool.threads();
   if (n == 1) {
     stream_copy(dst, src, bytes);
     return;
   }
   const size_t part = (((bytes + n - 1) / n) + 4095) & ~static_cast<size_t>(4095);
-  std::vector<std::thread> pool;
-  for (unsigned t = 0; t < n; ++t) {
+  pool.run((bytes + part - 1) / part, [=](size_t t) {
     const size_t off = t * part;
-    if (off >= bytes) break;
-    const size_t len = std::min(part, bytes - off);
-    pool.emplace_back([=]() {
-      stream_copy(static_cast<char *>(dst) + off, static_cast<const char *>(src) + off, len);
-    });
-  }
-  for (auto &th : pool) th.join();
+    stream_copy(static_cast<char *>(dst) + off, static_cast<const char *>(src) + off,
+                std::min(part, bytes - off));
+  });
 }
 
 // Creates the copy streams and slot events of the pipelines on first use.
@@ -554,24 +627,18 @@ struct HostCsr {
   bool native() const { return !w64 && cols64 == 0; }
 };
 
-// Runs f(begin, end) over [0, n), split over up to 8 host threads once n
+// Runs f(begin, end) over [0, n), split over the pool's threads once n
 // reaches `split`.
 template <typename F>
-void par_for(size_t n, size_t split, F f) {
-  const unsigned k = n < split ? 1u : host_threads();
+void par_for(HostPool &pool, size_t n, size_t split, F f) {
+  const unsigned k = n < split ? 1u : pool.threads();
   if (k == 1) {
     if (n) f(size_t{0}, n);
     return;
   }
   const size_t part = (((n + k - 1) / k) + 1023) & ~static_cast<size_t>(1023);
-  std::vector<std::thread> pool;
-  for (unsigned t = 0; t < k; ++t) {
-    const size_t b = t * part;
-    if (b >= n) break;
-    const size_t e = std::min(n, b + part);
-    pool.emplace_back([=]() { f(b, e); });
-  }
-  for (auto &th : pool) th.join();
+  pool.run((n + part - 1) / part,
+           [&](size_t t) { f(t * part, std::min(n, t * part + part)); });
 }
 
 // Stages entries [b0, b0 + n) of the caller's weights and columns into the
@@ -579,24 +646,24 @@ void par_for(size_t n, size_t split, F f) {
 // to nearest; a 64-bit column outside [0, 2^32) becomes 0xFFFFFFFF, which no
 // dim admits, so the device check rejects it instead of a wrapped value
 // passing.
-void stage_weights(const HostCsr &in, uint64_t b0, size_t n, float *w) {
+void stage_weights(HostPool &pool, const HostCsr &in, uint64_t b0, size_t n, float *w) {
   constexpr size_t kSplit = size_t{2} << 20;
   if (in.w64) {
     const double *src = static_cast<const double *>(in.weights) + b0;
-    par_for(n, kSplit, [=](size_t b, size_t e) { mhb::convert_f64_to_f32(w + b, src + b, e - b); });
+    par_for(pool, n, kSplit, [=](size_t b, size_t e) { mhb::convert_f64_to_f32(w + b, src + b, e - b); });
   } else {
-    par_memcpy(w, static_cast<const float *>(in.weights) + b0, n * sizeof(float));
+    par_memcpy(pool, w, static_cast<const float *>(in.weights) + b0, n * sizeof(float));
   }
 }
 
-void stage_cols(const HostCsr &in, uint64_t b0, size_t n, uint32_t *c) {
+void stage_cols(HostPool &pool, const HostCsr &in, uint64_t b0, size_t n, uint32_t *c) {
   constexpr size_t kSplit = size_t{2} << 20;
   if (in.cols64) {
     // int64 and uint64 alike: a negative int64 has its high bits set.
     const uint64_t *src = static_cast<const uint64_t *>(in.cols) + b0;
-    par_for(n, kSplit, [=](size_t b, size_t e) { mhb::convert_i64_to_u32(c + b, src + b, e - b); });
+    par_for(pool, n, kSplit, [=](size_t b, size_t e) { mhb::convert_i64_to_u32(c + b, src + b, e - b); });
   } else {
-    par_memcpy(c, static_cast<const uint32_t *>(in.cols) + b0, n * sizeof(uint32_t));
+    par_memcpy(pool, c, static_cast<const uint32_t *>(in.cols) + b0, n * sizeof(uint32_t));
   }
 }
 
@@ -604,12 +671,12 @@ void stage_cols(const HostCsr &in, uint64_t b0, size_t n, uint32_t *c) {
 // arrays (mhb::pack_cols, split over host threads at even entries).  Returns
 // false if some column needs more than 16 + hi_bits bits; the block then
 // crosses the link unpacked.
-bool stage_packed_cols(const HostCsr &in, uint64_t b0, size_t n, uint16_t *lo, uint8_t *hi,
-                       int hi_bits) {
+bool stage_packed_cols(HostPool &pool, const HostCsr &in, uint64_t b0, size_t n, uint16_t *lo,
+                       uint8_t *hi, int hi_bits) {
   constexpr size_t kSplit = size_t{2} << 20;
   const uint32_t *src = static_cast<const uint32_t *>(in.cols) + b0;
   std::atomic<bool> fits{true};
-  par_for(n, kSplit, [&, src, lo, hi](size_t b, size_t e) {
+  par_for(pool, n, kSplit, [&, src, lo, hi](size_t b, size_t e) {
     if (!mhb::pack_cols(src + b, e - b, lo + b, hi + (hi_bits == 4 ? b / 2 : b), hi_bits))
       fits.store(false, std::memory_order_relaxed);
   });
@@ -727,11 +794,12 @@ MHCUDAResult calc_pipelined(const Gen *gen, const HostCsr &in, uint32_t length,
   TuneChoice whole{};
   const TuneChoice *force = tuned_choice(gen, nnz, length, &whole, true) ? &whole : nullptr;
 
+  HostPool pool;
   // Finishes a slot: waits for its hashes and moves staged ones to the caller.
   auto retire = [&](Gen::Slot &sl) -> MHCUDAResult {
     if (!sl.busy) return mhcudaSuccess;
     MHB_CHECK(gen, cudaEventSynchronize(sl.d2h), mhcudaMemoryCopyError);
-    if (sl.pending_out) par_memcpy(sl.pending_out, sl.hout.ptr, sl.pending_bytes);
+    if (sl.pending_out) par_memcpy(pool, sl.pending_out, sl.hout.ptr, sl.pending_bytes);
     sl.pending_out = nullptr;
     sl.busy = false;
     return mhcudaSuccess;
@@ -830,7 +898,7 @@ MHCUDAResult calc_pipelined(const Gen *gen, const HostCsr &in, uint32_t length,
     const size_t hi_bytes = pack_bits == 4 ? (static_cast<size_t>(n) + 1) / 2 : n;
     const bool packed =
         pack_bits && n &&
-        stage_packed_cols(in, b0, n, sl.hc.as<uint16_t>(), sl.hc.as<uint8_t>() + hi_off, pack_bits);
+        stage_packed_cols(pool, in, b0, n, sl.hc.as<uint16_t>(), sl.hc.as<uint8_t>() + hi_off, pack_bits);
     if (pin_in) {
       src_w = static_cast<const float *>(in.weights) + b0;
       src_c = static_cast<const uint32_t *>(in.cols) + b0;
@@ -838,8 +906,8 @@ MHCUDAResult calc_pipelined(const Gen *gen, const HostCsr &in, uint32_t length,
       MHB_CHECK(gen, sl.hw.ensure(static_cast<size_t>(n) * 4), mhcudaMemoryAllocationFailure);
       MHB_CHECK(gen, sl.hip.ensure((static_cast<size_t>(len) + 1) * 4),
                 mhcudaMemoryAllocationFailure);
-      stage_weights(in, b0, n, static_cast<float *>(sl.hw.ptr));
-      if (!packed) stage_cols(in, b0, n, static_cast<uint32_t *>(sl.hc.ptr));
+      stage_weights(pool, in, b0, n, static_cast<float *>(sl.hw.ptr));
+      if (!packed) stage_cols(pool, in, b0, n, static_cast<uint32_t *>(sl.hc.ptr));
       memcpy(sl.hip.ptr, src_i, (static_cast<size_t>(len) + 1) * 4);
       src_w = sl.hw.ptr;
       src_c = sl.hc.ptr;
@@ -1715,7 +1783,8 @@ enum MHCUDAResult mhcuda_calc_batch(const MinhashCudaGenerator *gen, uint32_t co
   const uint64_t group_rows = 1u << 20;
   MHB_CHECK(gen, gen->d_status.ensure(2 * sizeof(uint32_t)), mhcudaMemoryAllocationFailure);
   MHB_CHECK(gen, cudaMemsetAsync(gen->d_status.ptr, 0, sizeof(uint32_t), st), mhcudaRuntimeError);
-  const unsigned nth = host_threads();
+  HostPool pool;
+  const unsigned nth = pool.threads();
 
   // A slot's staged hashes go back to their matrices once its copy is done.
   struct Pending {
@@ -1731,14 +1800,10 @@ enum MHCUDAResult mhcuda_calc_batch(const MinhashCudaGenerator *gen, uint32_t co
     std::vector<size_t> off(pd.last - pd.first + 1, 0);
     for (uint32_t i = pd.first; i < pd.last; ++i)
       off[i - pd.first + 1] = off[i - pd.first] + lengths[i] * row_bytes;
-    std::vector<std::thread> pool;
-    for (unsigned t = 0; t < nth; ++t) {
-      pool.emplace_back([&, t]() {
-        for (uint32_t i = pd.first + t; i < pd.last; i += nth)
-          if (lengths[i]) stream_copy(outputs[i], src + off[i - pd.first], lengths[i] * row_bytes);
-      });
-    }
-    for (auto &th : pool) th.join();
+    pool.run(nth, [&](size_t t) {
+      for (uint32_t i = pd.first + static_cast<uint32_t>(t); i < pd.last; i += nth)
+        if (lengths[i]) stream_copy(outputs[i], src + off[i - pd.first], lengths[i] * row_bytes);
+    });
     sl.busy = false;
     return mhcudaSuccess;
   };
@@ -1826,22 +1891,18 @@ enum MHCUDAResult mhcuda_calc_batch(const MinhashCudaGenerator *gen, uint32_t co
     float *sw = sl.hw.as<float>();
     uint32_t *sc = sl.hc.as<uint32_t>(), *si = sl.hip.as<uint32_t>();
     {
-      std::vector<std::thread> pool;
-      for (unsigned t = 0; t < nth; ++t) {
-        pool.emplace_back([&, t]() {
-          for (uint32_t i = m0 + t; i < m1; i += nth) {
-            const uint64_t len = lengths[i];
-            if (!len) continue;
-            const uint32_t b = rows[i][0];
-            const uint64_t po = moff[i - m0], ro = roff[i - m0];
-            stream_copy(sw + po, weights[i] + b, nnz_of[i] * 4);
-            stream_copy(sc + po, cols[i] + b, nnz_of[i] * 4);
-            for (uint64_t x = 0; x < len; ++x)
-              si[ro + x] = static_cast<uint32_t>(po + (rows[i][x] - b));
-          }
-        });
-      }
-      for (auto &th : pool) th.join();
+      pool.run(nth, [&](size_t t) {
+        for (uint32_t i = m0 + static_cast<uint32_t>(t); i < m1; i += nth) {
+          const uint64_t len = lengths[i];
+          if (!len) continue;
+          const uint32_t b = rows[i][0];
+          const uint64_t po = moff[i - m0], ro = roff[i - m0];
+          stream_copy(sw + po, weights[i] + b, nnz_of[i] * 4);
+          stream_copy(sc + po, cols[i] + b, nnz_of[i] * 4);
+          for (uint64_t x = 0; x < len; ++x)
+            si[ro + x] = static_cast<uint32_t>(po + (rows[i][x] - b));
+        }
+      });
     }
     si[R] = N;
     MHB_CHECK(gen, cudaMemcpyAsync(sl.ip.ptr, si, (static_cast<size_t>(R) + 1) * 4,
