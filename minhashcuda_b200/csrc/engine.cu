@@ -304,11 +304,15 @@ bool tuned_choice(const Gen *gen, uint64_t nnz, uint64_t rows, TuneChoice *out,
 // The filtered kernel evaluates 11-17 candidates per (row, sample) whatever the
 // row's length, the dense one every entry.  Measured on 8M entries in uniform
 // rows, 128 samples (ms, dense / filtered): rows of 60 entries 1.99 / 2.52, of
-// 80 1.97 / 2.02, of 100 1.95 / 1.77, of 120 1.94 / 1.54.
-constexpr uint32_t kFilterMinRow = 88;
+// 80 1.97 / 2.02, of 100 1.95 / 1.77, of 120 1.94 / 1.54; 13,003 heavy-tailed
+// rows of 101 on average at 200 samples 652 / 661 us.
+constexpr uint32_t kFilterMinRow = 104;
 // Below it a launch is over before the chip is full: 30,000 entries in
 // 300-entry rows 31 / 34 us, 90,000 entries 69 / 51 us.
 constexpr uint64_t kFilterMinEvals = 1ull << 23;
+// Dense launches under 2^26 evaluations with fewer 64-entry items than this
+// take one sample per lane, for more items.
+constexpr uint64_t kSmallItems = 9472;  // two per resident warp
 // Entries x tiles per resident warp below which tiles are made narrower: twice
 // the warps share a row, each with half the candidates, for a second pass over
 // the CSR.  3,000 rows of 1400 entries (1417 per warp): 485 us whole, 408
@@ -317,7 +321,9 @@ constexpr uint64_t kFilterShare = 1500;
 
 // Mean rows below which the dense kernel keeps t with each minimum (RowState):
 // rows of 20 entries 2.64 -> 2.21 ms, of 60 2.27 -> 1.99, of 420 (heavy tail,
-// 256 samples) 6.14 -> 5.86; rows of 1400 Zipf entries 27.9 -> 28.5.
+// 256 samples) 6.14 -> 5.86; rows of 1400 Zipf entries 27.9 -> 28.5.  With one
+// sample per lane only tiny launches do (one 300-entry row 21.9 -> 17.8 us
+// alone); others lose (400,000 rows of 20 at 32 samples 0.84 -> 0.99 ms).
 constexpr uint64_t kKeepMaxRow = 512;
 
 // Whether a launch takes the bound-filtered kernel (filter_kernels.cu).
@@ -331,8 +337,10 @@ bool use_filter(const Gen *gen, uint64_t nnz, uint64_t rows, const TuneChoice *t
 
 // min_items: items per resident warp the chunk is capped to give (8 for the
 // engine's own calls; the server asks for 2, its launches overlap).
+// least_chunk: shortest chunk of a tiny launch, a multiple of 8 (of 32 where
+// the columns may be packed).
 HashPlan make_plan(const Gen *gen, uint64_t nnz, uint64_t rows, const TuneChoice *force = nullptr,
-                   uint32_t min_items = 8, bool allow_filter = true) {
+                   uint32_t min_items = 8, bool allow_filter = true, uint32_t least_chunk = 32) {
   HashPlan p{};
   const uint32_t s_pad = gen->s_pad;
   TuneChoice tuned{};
@@ -350,14 +358,10 @@ HashPlan make_plan(const Gen *gen, uint64_t nnz, uint64_t rows, const TuneChoice
     // logf share); narrow tiles give small inputs more warps.  Keep lane
     // utilisation of the last tile >= 3/4.
     const uint64_t evals = nnz * static_cast<uint64_t>(gen->samples);
-    spl = 4;
-    auto util = [&](int s) {
-      const uint32_t w = 32u * s;
-      const uint32_t tiles = (s_pad + w - 1) / w;
-      return static_cast<double>(s_pad) / (static_cast<double>(tiles) * w);
-    };
-    if (util(4) < 0.75) spl = util(2) >= 0.75 ? 2 : 1;
-    if (evals < (1ull << 26) && spl > 1) spl = 1;  // small inputs: more items
+    spl = mhb::tile_fills(s_pad, 4) ? 4 : mhb::tile_fills(s_pad, 2) ? 2 : 1;
+    // Small inputs: more items, unless there are chunks enough as it is.
+    const uint32_t tiles = (s_pad + 32 * spl - 1) / (32 * spl);
+    if (evals < (1ull << 26) && nnz / 64 * tiles < kSmallItems) spl = 1;
   }
   p.spl = static_cast<uint32_t>(spl);
   p.minb = 4;
@@ -378,6 +382,7 @@ HashPlan make_plan(const Gen *gen, uint64_t nnz, uint64_t rows, const TuneChoice
       1, env_int("MHCUDA_B200_WAVES", have_tuned ? static_cast<int>(tuned.waves) : 32));
   const uint64_t target_items = resident_warps * waves;
   uint64_t chunk = (nnz * p.ntiles + target_items - 1) / target_items;
+  bool tiny = false;
   // Rows shorter than a chunk finish inside it; aim for a few rows per chunk.
   const uint64_t avg_row = rows ? (nnz + rows - 1) / rows : 1;
   chunk = std::max<uint64_t>(chunk, std::min<uint64_t>(4 * avg_row, 1024));
@@ -398,11 +403,20 @@ HashPlan make_plan(const Gen *gen, uint64_t nnz, uint64_t rows, const TuneChoice
   } else {
     const uint64_t want = resident_warps * std::max<uint32_t>(1, min_items);
     chunk = std::min<uint64_t>(chunk, std::max<uint64_t>(64, (nnz * p.ntiles + want - 1) / want));
+    // Too few entries for 8 per warp: one item per resident warp.  The time of
+    // such a launch is its longest chain of dependent gathers: one 300-entry row
+    // at 128 samples takes 8.2 us in chunks of 64 entries, 6.2 in 32s, 4.85 in 8s
+    // (a launch among others; 30.5, 23.8 and 21.2 alone).
+    if (nnz * p.ntiles <= 8 * resident_warps) {
+      tiny = true;
+      chunk = std::max<uint64_t>(
+          least_chunk, (((nnz * p.ntiles + resident_warps - 1) / resident_warps) + 7) & ~7ull);
+    }
   }
-  p.keep = !p.filter && avg_row < kKeepMaxRow;
+  p.keep = !p.filter && p.minb == 4 && (p.spl > 1 || tiny) && avg_row < kKeepMaxRow;
   const int forced = env_int("MHCUDA_B200_CHUNK", 0);
   if (forced > 0) chunk = static_cast<uint64_t>(forced);
-  chunk = std::max<uint64_t>(64, (chunk + 31) & ~31ull);
+  if (!tiny || forced > 0) chunk = std::max<uint64_t>(64, (chunk + 31) & ~31ull);
   chunk = std::min<uint64_t>(chunk, 1u << 24);
   p.chunk = static_cast<uint32_t>(chunk);
   const uint64_t nchunks = nnz == 0 ? 1 : (nnz + chunk - 1) / chunk;
@@ -433,6 +447,7 @@ MHCUDAResult prepare_launch(const Gen *gen, uint32_t rows, uint32_t nnz, const H
   a->bounds = gen->usable_bounds();
   a->b_stride = mhb::bound_stride(gen->s_pad);
   a->snap = plan.snap;
+  a->part_t = plan.filter || plan.keep;
   a->next_item = plan.filter ? gen->d_status.as<uint32_t>() + 1 : nullptr;
   a->rows = rows;
   a->nnz = nnz;
@@ -448,9 +463,7 @@ MHCUDAResult prepare_launch(const Gen *gen, uint32_t rows, uint32_t nnz, const H
 
 MHCUDAResult enqueue_hash(const Gen *gen, const HashArgs &a, const HashPlan &plan,
                           cudaStream_t stream, bool clear_status = true) {
-  if (clear_status)
-    MHB_CHECK(gen, cudaMemsetAsync(a.status, 0, sizeof(uint32_t), stream), mhcudaRuntimeError);
-  MHB_CHECK(gen, mhb::launch_plan(a, stream), mhcudaRuntimeError);
+  MHB_CHECK(gen, mhb::launch_plan(a, stream, clear_status), mhcudaRuntimeError);
   std::pair<cudaEvent_t, cudaEvent_t> *ev = nullptr;
   if (gen->profiling) {
     if (gen->prof_used == gen->prof_events.size()) {
@@ -1351,7 +1364,7 @@ enum MHCUDAResult mhcuda_calc(const MinhashCudaGenerator *gen, const float *weig
                                    cudaMemcpyHostToDevice, st),
               mhcudaMemoryCopyError);
   }
-  const HashPlan plan = make_plan(gen, nnz, length);
+  const HashPlan plan = make_plan(gen, nnz, length, nullptr, 8, true, 8);
   HashArgs a{};
   MHCUDAResult r = prepare_launch(gen, length, nnz, plan, &a);
   if (r != mhcudaSuccess) return r;
@@ -1430,7 +1443,7 @@ enum MHCUDAResult mhcuda_calc_device(const MinhashCudaGenerator *gen, const floa
   std::lock_guard<std::mutex> lock(gen->mu);
   MHB_ON_DEVICE(gen);
   const cudaStream_t st = stream ? static_cast<cudaStream_t>(stream) : gen->stream;
-  const HashPlan plan = make_plan(gen, nnz, length);
+  const HashPlan plan = make_plan(gen, nnz, length, nullptr, 8, true, 8);
   HashArgs a{};
   MHCUDAResult r = prepare_launch(gen, length, nnz, plan, &a);
   if (r != mhcudaSuccess) return r;
@@ -1515,7 +1528,6 @@ enum MHCUDAResult mhcuda_calc_batch_device(const MinhashCudaGenerator *gen, uint
   // Kernel variant as for one large launch; the chunk size is chosen on the
   // device from the batch's nnz (batch_setup_kernel).
   HashPlan vp = make_plan(gen, 1ull << 30, 1ull << 20, nullptr, 8, false);
-  vp.keep = 1;
   HashPlan fp = vp;
   fp.filter = mhb::filter_lanes(gen->s_pad);
   fp.ntiles = mhb::filter_tiles(gen->s_pad, fp.filter);
@@ -1524,6 +1536,8 @@ enum MHCUDAResult mhcuda_calc_batch_device(const MinhashCudaGenerator *gen, uint
   const int force_filter = env_int("MHCUDA_B200_FILTER", -1);
   const bool may_filter = gen->usable_bounds() && force_filter != 0 &&
                           (force_filter > 0 || plan_threads >= 4096);
+  // The dense launch of a batch that may be filtered hashes short rows.
+  vp.keep = may_filter && vp.spl > 1 && vp.minb == 4;
   TuneChoice tc{};
   const int waves = std::max(1, env_int("MHCUDA_B200_WAVES", static_cast<int>(tc.waves)));
   mhb::BatchArgs b{};
@@ -1548,8 +1562,10 @@ enum MHCUDAResult mhcuda_calc_batch_device(const MinhashCudaGenerator *gen, uint
   big.nchunks = max_chunks;
   HashArgs base{};
   big.filter = may_filter;  // for next_item
+  big.keep = vp.keep;
   MHCUDAResult r = prepare_launch(gen, 0, 0, big, &base);
   if (r != mhcudaSuccess) return r;
+  base.part_t = vp.keep;  // a filtered batch has it too (matrix_view)
   MHB_CHECK(gen, gen->d_chunk_owner.ensure(static_cast<size_t>(max_chunks) * 4),
             mhcudaMemoryAllocationFailure);
   MHB_CHECK(gen, gen->d_batch_plan.ensure(sizeof(mhb::BatchPlan)), mhcudaMemoryAllocationFailure);

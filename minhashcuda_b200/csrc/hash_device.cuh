@@ -158,12 +158,8 @@ __device__ __forceinline__ void store_partial(const HashArgs &a, uint32_t slot, 
   const size_t off = static_cast<size_t>(slot) * a.s_pad + s0;
 #pragma unroll
   for (int j = 0; j < SPL; ++j) {
-    uint32_t t;
-    if constexpr (KEEP) {
-      t = whole(st.t[j]);
-    } else {
-      t = resolve(a, st.pos[j], s0 + j).y;
-    }
+    uint32_t t = 0;  // without KEEP the merge recomputes it (HashArgs::part_t)
+    if constexpr (KEEP) t = whole(st.t[j]);
     a.part_ln[off + j] = st.mn[j];
     a.part_kt[off + j] = make_uint2(st.pos[j], t);
   }
@@ -503,6 +499,7 @@ __device__ __forceinline__ HashArgs matrix_view(const BatchArgs &b, const BatchM
   v.chunk = chunk;
   v.nchunks = m.nchunks;
   v.snap = b.plan->snap;
+  v.part_t = b.base.part_t || b.plan->filter;
   v.chunk_row = b.base.chunk_row + m.chunk_base;
   v.part_ln = b.base.part_ln + static_cast<size_t>(2) * m.chunk_base * b.base.s_pad;
   v.part_kt = b.base.part_kt + static_cast<size_t>(2) * m.chunk_base * b.base.s_pad;

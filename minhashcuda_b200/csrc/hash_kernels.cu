@@ -67,8 +67,14 @@ __device__ __forceinline__ void plan_row(const HashArgs &a, uint32_t i) {
   (void)start;
 }
 
-__global__ void plan_kernel(const HashArgs a) {
+// clear: the launch's one block clears the status word first, in place of a
+// memset of its own (launches of few rows are bound by their launch count).
+__global__ void plan_kernel(const HashArgs a, bool clear) {
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (clear) {
+    if (threadIdx.x == 0) *a.status = 0;
+    __syncthreads();
+  }
   if (i == 0 && a.next_item) *a.next_item = 0;
   if (i <= a.rows) plan_row(a, i);
 }
@@ -363,7 +369,9 @@ __device__ __forceinline__ void finalize_item(const HashArgs &a, uint32_t c, uin
     kt = lt ? k2 : kt;
   }
   uint32_t *o = a.out + (static_cast<size_t>(row) * a.samples + s) * 2;
-  if (kt.x >= a.nnz) {
+  if (!a.part_t) {
+    kt = resolve(a, kt.x, s);
+  } else if (kt.x >= a.nnz) {
     kt = make_uint2(kNone, kNone);
   } else {
     kt.x = a.col_hi_bits ? packed_col(a, kt.x) : a.cols[kt.x];
@@ -475,7 +483,12 @@ __global__ void __launch_bounds__(kSetupThreads) batch_setup_kernel(const BatchA
     // sum over matrices of ceil(nnz_m / chunk) <= total_nnz / chunk + nonempty
     const uint64_t avail = b.max_chunks > total_nonempty ? b.max_chunks - total_nonempty : 1;
     chunk = max(chunk, (total_nnz + avail - 1) / avail);
-    chunk = max(static_cast<uint64_t>(64), (chunk + 31) & ~static_cast<uint64_t>(31));
+    if (!f && total_nnz * ntiles <= 8 * b.warps[0]) {  // tiny, as in make_plan
+      const uint64_t one = (total_nnz * ntiles + b.warps[0] - 1) / b.warps[0];
+      chunk = max(static_cast<uint64_t>(8), (one + 7) & ~static_cast<uint64_t>(7));
+    } else {
+      chunk = max(static_cast<uint64_t>(64), (chunk + 31) & ~static_cast<uint64_t>(31));
+    }
     if (chunk > (1u << 24)) {
       chunk = 1u << 24;
       if (total_nnz / chunk + total_nonempty > b.max_chunks) atomicOr(b.base.status, kStatusBadIndptr);
@@ -584,10 +597,14 @@ __global__ void logf_kernel(const float *in, float *out, size_t n) {
 
 }  // namespace
 
-cudaError_t launch_plan(const HashArgs &a, cudaStream_t stream) {
-  const uint32_t threads = 256;
-  const uint32_t blocks = (a.rows + 1 + threads - 1) / threads;
-  plan_kernel<<<blocks, threads, 0, stream>>>(a);
+cudaError_t launch_plan(const HashArgs &a, cudaStream_t stream, bool clear_status) {
+  const uint32_t threads = clear_status && a.rows < 1024 ? 1024 : 256;
+  const uint32_t blocks = a.rows / threads + 1;
+  if (clear_status && blocks > 1) {
+    const cudaError_t e = cudaMemsetAsync(a.status, 0, sizeof(uint32_t), stream);
+    if (e != cudaSuccess) return e;
+  }
+  plan_kernel<<<blocks, threads, 0, stream>>>(a, clear_status && blocks == 1);
   return cudaGetLastError();
 }
 

@@ -79,12 +79,8 @@ extern "C" enum MHCUDAResult mhcuda_calc_device_noalloc(
 
   // Work decomposition that fits the fixed scratch.
   const uint32_t s_pad = g.s_pad;
-  auto util = [&](uint32_t spl) {
-    const uint32_t w = 32u * spl, tiles = (s_pad + w - 1) / w;
-    return static_cast<double>(s_pad) / (static_cast<double>(tiles) * w);
-  };
   mhb::HashPlan plan{};
-  plan.spl = util(4) >= 0.75 ? 4 : (util(2) >= 0.75 ? 2 : 1);
+  plan.spl = mhb::tile_fills(s_pad, 4) ? 4 : mhb::tile_fills(s_pad, 2) ? 2 : 1;
   plan.minb = 4;
   plan.ntiles = (s_pad + 32u * plan.spl - 1) / (32u * plan.spl);
   const uint64_t per_chunk = 4 + 2 * static_cast<uint64_t>(s_pad) * (sizeof(float) + sizeof(uint2));

@@ -8,9 +8,8 @@
 // device-wide synchronisation.  Here one pass reads a block of sample rows of
 // all five uniform runs (or of the three assigned arrays) in [samples][dim]
 // order, applies the same float operations (each rounded to float as in the
-// reference: -logf(a*b), then logf of that), and writes whole columns of the
-// table -- 12 contiguous bytes per sample, in pairs r r c c b b -- and of the
-// byte table of bounds through shared-memory tiles, so reads and writes are
+// reference: -logf(a*b), then logf of that), and writes columns of the table
+// (12 contiguous bytes per sample, in pairs r r c c b b) and of the byte table of bounds through shared-memory tiles, so reads and writes are
 // coalesced and neither table is read back.
 #include <cstdint>
 

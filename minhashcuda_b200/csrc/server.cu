@@ -336,6 +336,7 @@ MHCUDAResult MinhashCudaServer_::run_units(Lane &lane, const std::vector<Unit> &
   a.b_stride = mhb::bound_stride(s_pad);
   a.snap = plan.snap;
   a.next_item = plan.filter ? lane.status + 1 : nullptr;
+  a.part_t = plan.filter || plan.keep;
   a.weights = zc ? lane.mw : lane.w;
   a.cols = zc ? lane.mc : lane.c;
   a.indptr = zc ? lane.mip : lane.ip;

@@ -29,7 +29,8 @@ inline uint32_t padded_samples(uint32_t samples) { return (samples + 3u) & ~3u; 
 // Work decomposition of one hash launch.
 //
 // The CSR's nnz positions [0, nnz) (relative to indptr[0]) are cut into
-// `nchunks` chunks of `chunk` positions (a multiple of 32).  A row belongs to
+// `nchunks` chunks of `chunk` positions (a multiple of 32; of 8 in tiny
+// launches, whose columns are never packed).  A row belongs to
 // the chunk holding its first position (trailing empty rows to the last
 // chunk).  A warp hashes one (chunk, sample-tile) item: it finishes every row
 // that lies inside the chunk and leaves a partial arg-min for the row that
@@ -38,7 +39,7 @@ inline uint32_t padded_samples(uint32_t samples) { return (samples + 3u) & ~3u; 
 // partials of every row that crosses a chunk boundary, earlier positions
 // winning ties exactly as the reference's strict '<' scan does.
 struct HashPlan {
-  uint32_t chunk;    // positions per chunk, multiple of 32
+  uint32_t chunk;    // positions per chunk, multiple of 32 (of 8 in tiny launches)
   uint32_t nchunks;  // >= 1
   uint32_t spl;      // samples per lane in one item: 1, 2 or 4
   uint32_t minb;     // kernel variant: minimum resident blocks per SM (4; 3 or 2 for spl 4)
@@ -53,6 +54,10 @@ struct HashPlan {
 constexpr int kHashBlock = 256;
 constexpr int kFilterBlock = 128;
 
+// True when tiles of 32 * spl samples are at least three quarters full.
+constexpr bool tile_fills(uint32_t s_pad, uint32_t spl) {
+  return 4 * s_pad >= 3 * ((s_pad + 32 * spl - 1) / (32 * spl)) * (32 * spl);
+}
 // Row stride in bytes of the bound table (one byte per sample): whole
 // 32-byte sectors.
 constexpr uint32_t bound_stride(uint32_t s_pad) { return (s_pad + 31) & ~31u; }
@@ -97,7 +102,7 @@ struct HashArgs {
   uint32_t ntiles;
   uint32_t *chunk_row;       // [nchunks] first row owned by each chunk
   float *part_ln;            // [2*nchunks][s_pad] partial minima
-  uint2 *part_kt;            // [2*nchunks][s_pad] partial (position of the minimum, its t)
+  uint2 *part_kt;            // [2*nchunks][s_pad] partial (position of the minimum, its t or 0)
   uint32_t *out;             // [rows][samples][2]
   uint32_t *status;          // device status word
   uint32_t host_csr;         // weights/cols/indptr/out are mapped host memory
@@ -117,6 +122,7 @@ struct HashArgs {
   // which the plan kernel sets to 0.  0 and nullptr for dense launches.
   uint32_t snap;
   uint32_t *next_item;
+  uint32_t part_t;           // partials carry t (filtered and KEEP launches)
 };
 
 // One matrix of a device-resident batch (mhcuda_calc_batch_device).  The
@@ -163,7 +169,7 @@ struct BatchArgs {
 
 // Launchers (hash_kernels.cu).  All enqueue on `stream` and return the launch
 // error, if any.
-cudaError_t launch_plan(const HashArgs &a, cudaStream_t stream);
+cudaError_t launch_plan(const HashArgs &a, cudaStream_t stream, bool clear_status = false);
 cudaError_t launch_hash(const HashArgs &a, const HashPlan &plan, cudaStream_t stream);
 cudaError_t launch_finalize(const HashArgs &a, cudaStream_t stream);
 // A whole device-resident batch: setup (per-matrix nnz, chunk size, chunk
