@@ -131,7 +131,8 @@ def measured_peaks():
     return 6650.0, "fallback"
 
 
-KERNEL_SOURCE = os.path.join(ROOT, "minhashcuda_b200", "csrc", "hash_kernels.cu")
+KERNEL_SOURCES = [os.path.join(ROOT, "minhashcuda_b200", "csrc", f)
+                  for f in ("hash_kernels.cu", "filter_kernels.cu", "hash_device.cuh")]
 PROFILE_JSON = os.path.join(ROOT, "profiles", "hash_kernel_traffic.json")
 SMS = 148
 ISSUE_PER_SM_CLK = 4 * 32  # four schedulers, one warp-instruction (32 threads) per clock each
@@ -139,13 +140,27 @@ ISSUE_PER_SM_CLK = 4 * 32  # four schedulers, one warp-instruction (32 threads) 
 
 def kernel_source_sha16():
     import hashlib
-    with open(KERNEL_SOURCE, "rb") as f:
-        return hashlib.sha256(f.read()).hexdigest()[:16]
+    h = hashlib.sha256()
+    for p in KERNEL_SOURCES:
+        with open(p, "rb") as f:
+            h.update(f.read())
+    return h.hexdigest()[:16]
+
+
+def filtered(nnz, rows, samples):
+    """Whether the engine's rule gives a launch of this size the bound-filtered
+    kernel (make_plan's use_filter in engine.cu; the tuner agrees on these
+    workloads)."""
+    forced = os.environ.get("MHCUDA_B200_FILTER")
+    if forced is not None:
+        return forced != "0"
+    return samples > 28 and nnz >= 104 * rows and nnz * samples >= 1 << 23
 
 
 def kernel_profile(variant):
-    """Counters ncu measured for the hash kernel variant `variant` (e.g.
-    "spl4_minb3") on a 20,000-row case of the large workload
+    """Counters ncu measured for the hash kernel variant `variant` (the
+    filtered kernel's "filter" and "filter_uniform", or a dense one's, e.g.
+    "spl4_minb3") on a small case of its workload
     (profiles/hash_kernel_traffic.json), and whether they were taken on the
     kernel source this run built."""
     if not os.path.exists(PROFILE_JSON):
@@ -169,8 +184,9 @@ def hash_roofline(nnz, R, S, kernel_ms, sm_mhz, peak, peak_kind, profile, profil
     over the measured HBM bandwidth; issue (ncu thread-instructions per eval
     over 148 SMs x 128 thread-instructions per clock at the run's median SM
     clock); and the FP32 issue floor of 8 operations per eval.  `bound` is the
-    one closest to its peak; the algorithmic bytes 12NS + 8N + 4(R+1) + 8RS
-    are kept beside them (their rate exceeds HBM when hot columns hit L2)."""
+    one closest to its peak; the bytes of evaluating every entry, 12NS + 8N +
+    4(R+1) + 8RS, are kept beside them (their rate exceeds HBM: the filtered
+    kernel reads one byte per entry and sample and evaluates few of them)."""
     t = kernel_ms / 1e3
     evals = nnz * S
     alg = 12 * nnz * S + 8 * nnz + 4 * (R + 1) + 8 * R * S
@@ -325,7 +341,8 @@ def extra_uniform(lib, local, peak, peak_kind):
     workload (12,000,000 dims x 128 samples, 18.4 GB of parameters, uniform
     columns, so the gathers find nothing in L2), device-resident, one
     mhcuda_calc_device per step, the hash kernel timed with the events the
-    library records around it."""
+    library records around it; its DRAM traffic is ncu's bytes per eval of a
+    smaller block, scaled."""
     import torch
     from minhashcuda_b200 import synth
     w = synth.WORKLOADS["streamed"]
@@ -360,11 +377,14 @@ def extra_uniform(lib, local, peak, peak_kind):
     lib.mhcuda_fini(gen)
     kernel_ms = hm.value / max(1, nl.value)
     alg = 12 * nnz * S + 8 * nnz + 4 * (rows + 1) + 8 * rows * S
-    gbs = alg / (kernel_ms / 1e3) / 1e9
+    prof, current = kernel_profile("filter_uniform") if filtered(nnz, rows, S) else (None, False)
+    traffic = prof["dram_bytes_per_eval"] * nnz * S if prof else None
+    gbs = (traffic or alg) / (kernel_ms / 1e3) / 1e9
     del ip, cols, wts, out
     _free_cuda()
     return {"bound": "hbm", "achieved": gbs, "peak": peak, "unit": "GB/s", "frac": gbs / peak,
-            "traffic": None, "kernel": "hash_kernel", "kernel_ms": kernel_ms,
+            "traffic": traffic, "kernel": "filter_kernel" if prof else "hash_kernel",
+            "kernel_ms": kernel_ms, "profile_matches_built_kernel": current,
             "algorithmic_bytes": alg, "peak_source": f"{peak_kind} hbm_gbs (MEASURED_PEAKS.json)",
             "value": nnz * S / (e0.elapsed_time(e1) / 5 / 1e3), "unit_value": UNIT,
             "workload": f"streamed block: {rows} rows x {w.dim} dims, {S} samples, {nnz} nnz, "
@@ -1163,7 +1183,9 @@ def main():
 
     hash_ms_launch = hash_ms.value / max(1, launches.value)
     peak, peak_kind = measured_peaks()
-    if tuned:
+    if w.name == "large" and filtered(nnz, R, S):
+        variant = "filter"
+    elif tuned:
         variant = f"spl{tuned['samples_per_lane']}_minb{tuned['min_blocks_per_sm']}"
     else:
         variant = f"spl{os.environ.get('MHCUDA_B200_SPL', '4')}_minb" \

@@ -9,8 +9,8 @@
  * Semantics on this engine:
  *  - One generator lives on exactly one CUDA device (the lowest set bit of
  *    the `devices` mask that names a present device; mask 0 means device 0).
- *  - Parameters are kept on the device as one [dim][3][samples] table
- *    (r, ln_c, beta per column); the host-facing layout stays row-major
+ *  - Parameters are kept on the device as one table with all samples of a
+ *    column together (r, ln_c, beta); the host-facing layout stays row-major
  *    [samples][dim] float32 for retrieve/assign.
  *  - All calls are synchronous: results are valid when the call returns.
  *  - One generator is not re-entrant; calls on one generator are serialised

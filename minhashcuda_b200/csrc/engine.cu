@@ -1051,7 +1051,9 @@ MHCUDAResult init_params(Gen *gen, uint32_t seed) {
       if (g) curandDestroyGenerator(g);
     return code;
   };
-  for (uint64_t k = 0; k < 5; ++k) {
+  // All runs in one block: one generator draws them one after the other.
+  const bool single = whole && rows >= S;
+  for (uint64_t k = 0; k < (single ? 1u : 5u); ++k) {
     if (curandCreateGenerator(&rng[k], CURAND_RNG_PSEUDO_DEFAULT) != CURAND_STATUS_SUCCESS) {
       rng[k] = nullptr;
       return finish(mhcudaRuntimeError);
@@ -1069,10 +1071,13 @@ MHCUDAResult init_params(Gen *gen, uint32_t seed) {
         if (!(parts >> (k / 2) & 1u)) continue;  // U1, U2: r; U3, U4: ln_c; U5: beta
         float *u = buf.as<float>() + static_cast<size_t>(whole ? k : k % 2) * block;
         in.src[k] = u;
+        if (single) continue;
         if (curandGenerateUniform(rng[k], u, static_cast<size_t>(cnt) * D) !=
             CURAND_STATUS_SUCCESS)
           return finish(mhcudaRuntimeError);
       }
+      if (single && curandGenerateUniform(rng[0], buf.as<float>(), 5 * block) != CURAND_STATUS_SUCCESS)
+        return finish(mhcudaRuntimeError);
       if (mhb::launch_pack_params(in, true, parts, D, s0, cnt, P, gen->params, gen->bounds,
                                   gen->stream) != cudaSuccess)
         return finish(mhcudaRuntimeError);
@@ -1535,7 +1540,7 @@ enum MHCUDAResult mhcuda_calc_batch_device(const MinhashCudaGenerator *gen, uint
   // rows is not worth the second launch that takes.
   const int force_filter = env_int("MHCUDA_B200_FILTER", -1);
   const bool may_filter = gen->usable_bounds() && force_filter != 0 &&
-                          (force_filter > 0 || plan_threads >= 4096);
+                          (force_filter > 0 || plan_threads >= 512);
   // The dense launch of a batch that may be filtered hashes short rows.
   vp.keep = may_filter && vp.spl > 1 && vp.minb == 4;
   TuneChoice tc{};

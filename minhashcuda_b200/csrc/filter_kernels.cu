@@ -22,9 +22,21 @@
 // e^kGuess.  Samples that end above the guess are found at the end of the row
 // and scanned again without it (rescan).  With the generator's distributions
 // (r ~ Gamma(2), c ~ Gamma(2)) the share of entries whose c * e^-r lies below
-// x is x * (ln(1/x) + 0.42), which makes about 19 candidates per sample of a
-// 1400-entry row and 14 of a 200-entry one; with the running minimum alone
-// they are 29 and 17, and a row's first entries all pass.
+// x is x * (ln(1/x) + 0.42); counted on the device, 17 candidates per sample
+// are evaluated in a 1400-entry row, 13 in one of 300 (42 in the former
+// without the guess, when a row's first entries all pass).
+//
+// What bounds it.  Per entry a 128-byte line of bounds and per candidate a
+// 12-byte triple in a 32- or 64-byte sector somewhere in the table.  On uniform
+// columns over 12M that is HBM: 3.9 bytes per eval (12 in the dense kernel) at
+// 86% of the measured copy rate.  On Zipf columns, whose bounds stay in L2 (0.73
+// bytes per eval from HBM), it is the warps' waits for gathers at 5 instructions
+// per eval and 54% of the issue slots; candidates take a third of the time.
+// Against the dense kernels, device-resident, same box: 524,288 Zipf rows of
+// 1400 entries 98.1 -> 27.7 ms (3.4e12 evals/s), 131,072 ragged rows over 12M
+// columns 16.0 -> 5.3 ms, 256 uneven matrices at 256 samples 12.8 -> 5.9 ms,
+// 20,011 rows of 300 entries 855 -> 418 us.  use_filter in engine.cu says which
+// launches come here.
 //
 // Rounding.  In float32 the computed ln_a may lie below the real
 // ln_c - r - w by at most 2^-24 * (6|w| + 5 r (1 + |beta|) + 3|ln_c|) (one
@@ -56,6 +68,8 @@ namespace {
 constexpr int kLimit = 8191;  // |m|, |l| are clamped to it
 constexpr int kThrBias = 241 + 16384;
 constexpr uint32_t kThrOpen = kLimit + kThrBias;  // every entry passes
+// 7 was the fastest of 5 (20% slower on 1400-entry rows: one sample in 150 is
+// scanned again), 7, 8 and 10 (8% slower on 200-entry rows: more candidates).
 constexpr float kGuess = 7.0f;
 // A threshold is kept within this of the row's guess (3 in ln_a).  The few
 // samples with a lower minimum let a few entries more pass; the lower end of
@@ -148,9 +162,10 @@ __device__ __forceinline__ uint32_t warp_prefix(uint32_t x, uint32_t lane) {
 // starts soon enough (chunk_begin).
 //
 // LN lanes hold 16 samples each of one entry, so a tile is 16 * LN samples
-// and one warp load fetches the bytes of 32 / LN entries (16 per lane).  A
-// batch is 8 such loads, kept four ahead; its candidates go to a queue in
-// shared memory.  Once it holds 128, and at the end of a window or row, the
+// and one warp load fetches the bytes of 32 / LN entries (16 per lane; with 4
+// samples per lane addresses and loads cost four times as much per sample).  A
+// batch is 8 such loads, kept four ahead (eight ahead measured the same); its
+// candidates go to a queue in shared memory.  Once it holds 128, and at the end of a window or row, the
 // queue is evaluated, two candidates per lane at a time so that their
 // parameter gathers overlap, and the thresholds are updated.
 template <int LN, int SPAD, bool PACKED>

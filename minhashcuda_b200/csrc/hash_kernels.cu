@@ -12,8 +12,9 @@
 // (the form the reference build evaluates; pinned on a B200 by the tests).
 //
 // Layout and mapping (B200-first, not the reference's):
-//  - parameters are [dim][3][s_pad]: one nnz's r / ln_c / beta for a tile of
-//    32*SPL samples are three fully coalesced warp loads (SPL=4: 3 x 512 B),
+//  - a column's parameters are contiguous, in sample pairs (r r c c b b): one
+//    nnz's for a tile of 32*SPL samples are three vector loads per lane over
+//    one contiguous block (SPL=4: 1536 B),
 //  - a warp owns one (chunk, sample tile) item; each lane keeps SPL running
 //    minima in registers (no shared-memory spill as in kernel.cu:72-74),
 //    each with the position of its entry; (k, t) are recovered once per

@@ -117,3 +117,13 @@ def test_packed_columns_and_batches(dim, monkeypatch):
         np.testing.assert_array_equal(eng.calc_csr(m), want)
     if dim == 900:
         check(m, samples, params)
+
+
+@pytest.mark.parametrize("samples", [100, 128, 200])
+def test_full_width_tiles(samples):
+    """Enough entries per warp for the widest tiles (smaller inputs get
+    narrower ones), long rows kept whole and cut."""
+    rng = np.random.default_rng(samples)
+    dim = 9000
+    m = random_csr(rng, 4400, dim, 1100, long_rows=[(3, 9000), (1700, 8000), (4399, 9000)])
+    check(m, samples, gamma_params(rng, dim, samples))
