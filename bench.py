@@ -169,7 +169,7 @@ def kernel_profile(variant):
     v = d.get("variants", {}).get(variant)
     if v is None:
         return None, False
-    v = dict(v, captured_case=d.get("captured_case"), variant=variant)
+    v = dict({"captured_case": d.get("captured_case")}, **v, variant=variant)
     return v, d.get("source_sha16") == kernel_source_sha16()
 
 
@@ -190,7 +190,9 @@ def hash_roofline(nnz, R, S, kernel_ms, sm_mhz, peak, peak_kind, profile, profil
     t = kernel_ms / 1e3
     evals = nnz * S
     alg = 12 * nnz * S + 8 * nnz + 4 * (R + 1) + 8 * R * S
-    out = {"kernel": "hash_kernel", "kernel_ms": kernel_ms, "algorithmic_bytes": alg,
+    variant = (profile or {}).get("variant", "")
+    out = {"kernel": "filter_kernel" if variant.startswith("filter") else "hash_kernel",
+           "kernel_ms": kernel_ms, "algorithmic_bytes": alg,
            "algorithmic_gbs": alg / t / 1e9, "algorithmic_frac": alg / t / 1e9 / peak,
            "peak_source": f"{peak_kind} hbm_gbs (MEASURED_PEAKS.json)", "sm_mhz": sm_mhz}
     cands = {}

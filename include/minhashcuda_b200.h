@@ -32,7 +32,8 @@ enum MHCUDAResult mhcuda_calc_device(
     uint32_t nnz, uint32_t *d_output, void *stream);
 
 /* Autotuner: times the hash kernel's variants (samples per lane 1/2/4,
- * register budget, chunk granularity) on this device-resident CSR (same
+ * register budget, chunk granularity; the bound-filtered kernel, reported as
+ * 4 samples per lane and 4 blocks) on this device-resident CSR (same
  * arguments as mhcuda_calc_device; d_output receives the hashes), keeps the
  * fastest for launches of the same shape class (log2 of nnz and of the mean
  * row length) on this generator, and returns it in choice[3] = {samples per

@@ -39,8 +39,8 @@ ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 NVCC_FLAGS = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC", "-ccbin", HOST_CXX,
               "-I" + INCLUDE, "--expt-relaxed-constexpr"]
 
-ENGINE_SOURCES = ["hash_kernels.cu", "filter_kernels.cu", "param_kernels.cu", "engine.cu", "noalloc.cu", "server.cu",
-                  "lsh.cu", "host_copy.cc"]
+ENGINE_SOURCES = ["hash_kernels.cu", "filter_kernels.cu", "param_kernels.cu", "engine.cu",
+                  "noalloc.cu", "server.cu", "lsh.cu", "host_copy.cc"]
 HEADERS = ["wmh_internal.h", "hash_device.cuh"]
 
 EXT_SUFFIX = sysconfig.get_config_var("EXT_SUFFIX") or ".so"

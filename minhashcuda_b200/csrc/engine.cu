@@ -1076,7 +1076,8 @@ MHCUDAResult init_params(Gen *gen, uint32_t seed) {
             CURAND_STATUS_SUCCESS)
           return finish(mhcudaRuntimeError);
       }
-      if (single && curandGenerateUniform(rng[0], buf.as<float>(), 5 * block) != CURAND_STATUS_SUCCESS)
+      if (single &&
+          curandGenerateUniform(rng[0], buf.as<float>(), 5 * block) != CURAND_STATUS_SUCCESS)
         return finish(mhcudaRuntimeError);
       if (mhb::launch_pack_params(in, true, parts, D, s0, cnt, P, gen->params, gen->bounds,
                                   gen->stream) != cudaSuccess)

@@ -252,7 +252,9 @@ __device__ __forceinline__ bool filter_item(const HashArgs &a, uint32_t c, uint3
         ++failed;
         uint32_t best_k = fs.k[s], best_t = fs.t[s];
         unsigned long long best = static_cast<unsigned long long>(fs.val[s]) << 32 | fs.pos[s];
-        for (uint32_t p = fs.row_begin + lane; p < end; p += 32) {
+        const uint32_t begin = fs.row_begin, len = end - begin;  // p + 32 could wrap near 2^32
+        for (uint32_t o = lane; o < len; o += 32) {
+          const uint32_t p = begin + o;
           uint32_t col = PACKED ? packed_col(a, p) : a.cols[p];
           if (col >= a.dim) col = 0;
           const float w = logf(a.weights[p]);
@@ -307,17 +309,18 @@ __device__ __forceinline__ bool filter_item(const HashArgs &a, uint32_t c, uint3
   // Windows start at multiples of 32 positions (16-byte aligned bulk copies
   // of every array), the first one possibly before the chunk.
   const uint32_t w0 = cs & ~31u;
+  // Offsets from w0, which stay far from 2^32 where positions may not.
+  const uint32_t span = ce > cs ? ce - w0 : 0;
   auto issue = [&](uint32_t at, uint32_t buf) {
-    if (at < ce) issue_window<PACKED>(a, stg, wc.pk, buf, at, min(kFWin, ce - at), bulk_ok, lane);
+    if (at < span)
+      issue_window<PACKED>(a, stg, wc.pk, buf, w0 + at, min(kFWin, span - at), bulk_ok, lane);
   };
-  if (ce > cs) {
-    issue(w0, 0);
-    issue(w0 + kFWin, 1);
-  }
+  issue(0, 0);
+  issue(kFWin, 1);
   // Error exits wait (bounded) for the copies still in flight, those of the
-  // windows at `from` and behind it.
+  // windows at offset `from` and behind it.
   auto drain_copies = [&](uint32_t from, uint32_t buf) {
-    for (uint32_t kk = 0; kk < 2 && from < ce; ++kk, from += kFWin, buf ^= 1u) {
+    for (uint32_t kk = 0; kk < 2 && from < span; ++kk, from += kFWin, buf ^= 1u) {
       for (uint32_t spins = 0; !mbar_try_wait(&stg.bar[buf], (parity >> buf) & 1u);)
         if (++spins > kSpinLimit) break;
       parity ^= 1u << buf;
@@ -326,11 +329,12 @@ __device__ __forceinline__ bool filter_item(const HashArgs &a, uint32_t c, uint3
 
   uint32_t b = 0;
   uint32_t i = cs - w0;
-  for (uint32_t ws = w0; ws < ce && ce > cs; ws += kFWin, b ^= 1u, i = 0) {
-    const uint32_t n = min(kFWin, ce - ws);
+  for (uint32_t off = 0; off < span; off += kFWin, b ^= 1u, i = 0) {
+    const uint32_t ws = w0 + off;
+    const uint32_t n = min(kFWin, span - off);
     if (!finish_window<PACKED>(a, stg, wc.pk, b, (parity >> b) & 1u, ws, n, bulk_ok, lane)) {
       if (lane == 0) atomicOr(a.status, kStatusStall);
-      drain_copies(ws, b);
+      drain_copies(off, b);
       return false;
     }
     parity ^= 1u << b;
@@ -406,7 +410,7 @@ __device__ __forceinline__ bool filter_item(const HashArgs &a, uint32_t c, uint3
         flush(row_end);
         if (r_next >= fs.r_stop) {  // only reachable with inconsistent offsets
           if (lane == 0) atomicOr(a.status, kStatusBadIndptr);
-          drain_copies(ws + kFWin, b ^ 1u);
+          drain_copies(off + kFWin, b ^ 1u);
           return false;
         }
         row = r_next++;
@@ -423,9 +427,10 @@ __device__ __forceinline__ bool filter_item(const HashArgs &a, uint32_t c, uint3
         thr_guess = kThrOpen;
         if (guessing) {
           float sum = 0.0f;
-          const uint32_t end = min(row_end, ce);
+          const uint32_t len = min(row_end, ce) - fs.row_begin;
+          const float *__restrict__ weights = a.weights + fs.row_begin;
 #pragma unroll 8
-          for (uint32_t p = fs.row_begin + lane; p < end; p += 32) sum += fmaxf(a.weights[p], 0.0f);
+          for (uint32_t o = lane; o < len; o += 32) sum += fmaxf(weights[o], 0.0f);
 #pragma unroll
           for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xFFFFFFFFu, sum, o);
           if (sum > 0.0f && sum < FLT_MAX) thr_guess = threshold(__logf(kGuess / sum));
@@ -565,7 +570,7 @@ __device__ __forceinline__ bool filter_item(const HashArgs &a, uint32_t c, uint3
       }
       i = seg;
     }
-    issue(ws + 2 * kFWin, b);
+    issue(off + 2 * kFWin, b);
   }
   flush(min(row_end, ce));
   while (r_next < fs.r_stop) {  // trailing empty rows of the last chunk

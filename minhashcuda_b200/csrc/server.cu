@@ -305,7 +305,8 @@ MHCUDAResult MinhashCudaServer_::run_units(Lane &lane, const std::vector<Unit> &
   // even when rows are long (the plain plan keeps a few rows per chunk);
   // several lanes' launches overlap, so two are enough.
   mhb::HashPlan plan = mhb::plan_for_generator(units.front().req->gen, N, R,
-                                               high ? min_items_high : min_items_low, !zc);
+                                               high ? min_items_high : min_items_low,
+                                               !zc && g.bounds != nullptr);
   const int bps = mhb::plan_blocks_per_sm(plan, s_pad);
   // Keep the chunk table and partials inside the lane's fixed scratch:
   // nchunks*4 <= unit, 2*nchunks*s_pad*4 <= 4*unit, 2*nchunks*s_pad*8 <= 8*unit.
