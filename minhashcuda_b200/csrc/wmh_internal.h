@@ -70,9 +70,10 @@ constexpr uint32_t filter_tiles(uint32_t s_pad, uint32_t lanes) {
   return (s_pad + 16 * lanes - 1) / (16 * lanes);
 }
 // Work division of a filtered launch over `total` = entries x sample tiles and
-// `warps` resident warps: positions per chunk and the snap distance.  Chunks
-// of a mean row, but eight or more per warp, 32 at least 128 positions long;
-// rows are kept whole up to a quarter of a warp's share.
+// `warps` resident warps: positions per chunk and the snap distance.  `waves`
+// chunks per warp, but none shorter than a mean row as long as that leaves
+// eight per warp, nor than 128 positions; rows are kept whole up to a quarter
+// of a warp's share.
 struct FilterSplit {
   uint32_t chunk, snap;
 };
