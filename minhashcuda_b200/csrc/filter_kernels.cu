@@ -61,13 +61,10 @@ namespace {
 // when byte <= m + l + 240, m = ceil(20 * threshold), l = ceil(20 * w_i).
 // Two samples share a register as 16-bit halves; the halves' signed sums are
 // formed by one 32-bit addition each because the biased total
-//     D = (0xC000 + byte) - (m + 241 + 16384) - l = 0x8000 + byte - T,
-//     T = m + l + 241,
+//     D = filter_diff(byte, m, l) = 0x8000 + byte - T,  T = m + l + 241,
 // stays within 16 bits; bit 15 of D is clear exactly when byte < T.
 
-constexpr int kLimit = 8191;  // |m|, |l| are clamped to it
-constexpr int kThrBias = 241 + 16384;
-constexpr uint32_t kThrOpen = kLimit + kThrBias;  // every entry passes
+constexpr uint32_t kThrOpen = kThrLimit + kThrBias;  // every entry passes
 // 7 was the fastest of 5 (20% slower on 1400-entry rows: one sample in 150 is
 // scanned again), 7, 8 and 10 (8% slower on 200-entry rows: more candidates).
 constexpr float kGuess = 7.0f;
@@ -77,14 +74,16 @@ constexpr float kGuess = 7.0f;
 // with the least minimum.
 constexpr uint32_t kThrSpread = 60;
 
-// ceil(20 * x) clamped; 0.01 covers the product's rounding.
+// ceil(20 * x); 0.01 covers the product's rounding.  NaN gives 0, infinities
+// the ends of int.
 __device__ __forceinline__ int quant_up(float x) {
-  return min(max(__float2int_ru(__fmaf_rn(x, kBoundScale, 0.01f)), -kLimit - 1), kLimit);
+  return __float2int_ru(__fmaf_rn(x, kBoundScale, 0.01f));
 }
-// Finite minima above 400 (no table of the generator's gives one) keep the
-// threshold open, so the upper clamp of m never hides a candidate.
+// m and l (the clamps' reasons are at their definitions).
+__device__ __forceinline__ int quant_min(float mn) { return clamp_min(quant_up(mn)); }
+__device__ __forceinline__ int quant_weight(float w) { return clamp_weight(quant_up(w)); }
 __device__ __forceinline__ uint32_t threshold(float mn) {
-  return static_cast<uint32_t>(quant_up(mn) + kThrBias);
+  return static_cast<uint32_t>(quant_min(mn) + kThrBias);
 }
 
 // Minima as (monotone image of ln_a, position).  The smallest pair is the
@@ -259,8 +258,8 @@ __device__ __forceinline__ bool filter_item(const HashArgs &a, uint32_t c, uint3
           if (col >= a.dim) col = 0;
           const float w = logf(a.weights[p]);
           const uint32_t byte = a.bounds[static_cast<size_t>(col) * bstride + t0 + s];
-          const int m = quant_up(unordered(static_cast<uint32_t>(best >> 32)));
-          if (static_cast<int>(byte) > max(m + quant_up(w) + 240, 0)) continue;
+          const int m = quant_min(unordered(static_cast<uint32_t>(best >> 32)));
+          if (static_cast<int>(byte) > max(m + quant_weight(w) + 240, 0)) continue;
           const float *p3 = ptile + static_cast<size_t>(col) * 3 * spad + param_index(s);
           float t;
           const float x = exact_ln_a(w, __ldg(p3), __ldg(p3 + 2), __ldg(p3 + 4), t);
@@ -340,7 +339,7 @@ __device__ __forceinline__ bool filter_item(const HashArgs &a, uint32_t c, uint3
     parity ^= 1u << b;
     const float *__restrict__ lw = stg.w[b];
     uint32_t *__restrict__ cl = stg.c[b];
-    for (uint32_t p = lane; p < n; p += 32) fs.l[p] = quant_up(lw[p]) * 65537;
+    for (uint32_t p = lane; p < n; p += 32) fs.l[p] = quant_weight(lw[p]) * 65537;
     // Entries past the window's end in its last batch: column 0, masked off.
     for (uint32_t p = n + lane; p < ((n + GRP - 1) & ~(GRP - 1)); p += 32) cl[p] = 0;
     __syncwarp();

@@ -69,6 +69,25 @@ constexpr uint32_t filter_lanes(uint32_t s_pad) { return s_pad > 64 ? 8 : s_pad 
 constexpr uint32_t filter_tiles(uint32_t s_pad, uint32_t lanes) {
   return (s_pad + 16 * lanes - 1) / (16 * lanes);
 }
+// Threshold arithmetic of the filter kernels (filter_kernels.cu): m is a
+// sample's threshold and l an entry's ln(weight), both in steps of 1/20 and
+// rounded up, clamped to what 16 bits hold.
+constexpr int kThrLimit = 8191;
+constexpr int kThrBias = 241 + 16384;
+// Below -8192: a threshold of -409.6 lets a few entries more pass.  Above 8191:
+// finite weights (l >= -2080) all pass there, as they have to; no value of the
+// generator's tables is above 400.
+constexpr int clamp_min(int q) { return q < -kThrLimit - 1 ? -kThrLimit - 1 : q < kThrLimit ? q : kThrLimit; }
+// Below: only weights of 0, which never win.  Above: only infinite weights,
+// whose ln_a of -inf wins whatever the threshold: l + m has to pass byte 255 at
+// m = -8192 too, hence the 256 more.
+constexpr int clamp_weight(int q) {
+  return q < -kThrLimit - 1 ? -kThrLimit - 1 : q < kThrLimit + 256 ? q : kThrLimit + 256;
+}
+// The 16-bit difference whose bit 15 is clear when the entry passes.
+constexpr uint32_t filter_diff(uint32_t byte, int m, int l) {
+  return 0xC000u + byte - static_cast<uint32_t>(m + kThrBias) - static_cast<uint32_t>(l);
+}
 // Work division of a filtered launch over `total` = entries x sample tiles and
 // `warps` resident warps: positions per chunk and the snap distance.  `waves`
 // chunks per warp, but none shorter than a mean row as long as that leaves
