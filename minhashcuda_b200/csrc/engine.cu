@@ -187,6 +187,8 @@ struct MinhashCudaGenerator_ {
   // when there is none.  bounds_ok: it belongs to the current parameters.
   uint8_t *bounds = nullptr;
   mutable std::atomic<bool> bounds_ok{false};
+  // They are worth using without being asked to (mhb::bounds_fit).
+  mutable std::atomic<bool> bounds_fit{false};
   const uint8_t *usable_bounds() const { return bounds_ok.load() ? bounds : nullptr; }
   cudaStream_t stream = nullptr;
 
@@ -331,6 +333,7 @@ bool use_filter(const Gen *gen, uint64_t nnz, uint64_t rows, const TuneChoice *t
   if (!gen->usable_bounds()) return false;
   const int forced = env_int("MHCUDA_B200_FILTER", -1);
   if (forced >= 0) return forced != 0;
+  if (!gen->bounds_fit) return false;
   if (tuned) return tuned->filter;
   return nnz >= kFilterMinRow * rows && nnz * gen->s_pad >= kFilterMinEvals;
 }
@@ -1080,12 +1083,13 @@ MHCUDAResult init_params(Gen *gen, uint32_t seed) {
           curandGenerateUniform(rng[0], buf.as<float>(), 5 * block) != CURAND_STATUS_SUCCESS)
         return finish(mhcudaRuntimeError);
       if (mhb::launch_pack_params(in, true, parts, D, s0, cnt, P, gen->params, gen->bounds,
-                                  gen->stream) != cudaSuccess)
+                                  nullptr, gen->stream) != cudaSuccess)
         return finish(mhcudaRuntimeError);
     }
   }
   if (cudaStreamSynchronize(gen->stream) != cudaSuccess) return finish(mhcudaRuntimeError);
   gen->bounds_ok = gen->bounds && whole;
+  gen->bounds_fit = true;
   return finish(mhcudaSuccess);
 }
 
@@ -1311,8 +1315,15 @@ enum MHCUDAResult mhcuda_assign_random_vars(const MinhashCudaGenerator *gen, con
   gen->bounds_ok = false;
   // Without room for a block of each array, one array at a time and no bounds.
   DevBuf tmp;
-  const bool whole = tmp.ensure(3 * block * sizeof(float)) == cudaSuccess;
+  std::vector<uint32_t> counts(static_cast<size_t>(S) * mhb::kFitCuts);
+  const size_t count_bytes = counts.size() * sizeof(uint32_t);
+  const bool whole = tmp.ensure(3 * block * sizeof(float) + count_bytes) == cudaSuccess;
   if (!whole) MHB_CHECK(gen, tmp.ensure(block * sizeof(float)), mhcudaMemoryAllocationFailure);
+  uint32_t *d_counts = nullptr;
+  if (whole && gen->bounds) {
+    d_counts = reinterpret_cast<uint32_t *>(tmp.as<float>() + 3 * block);
+    MHB_CHECK(gen, cudaMemsetAsync(d_counts, 0, count_bytes, gen->stream), mhcudaRuntimeError);
+  }
   for (uint32_t parts : whole ? std::vector<uint32_t>{7u} : std::vector<uint32_t>{1u, 2u, 4u}) {
     for (uint32_t s0 = 0; s0 < S; s0 += rows) {
       const uint32_t cnt = std::min(rows, S - s0);
@@ -1327,12 +1338,17 @@ enum MHCUDAResult mhcuda_assign_random_vars(const MinhashCudaGenerator *gen, con
                   mhcudaMemoryCopyError);
       }
       MHB_CHECK(gen, mhb::launch_pack_params(in, false, parts, D, s0, cnt, gen->s_pad,
-                                             gen->params, gen->bounds, gen->stream),
+                                             gen->params, gen->bounds, d_counts, gen->stream),
                 mhcudaRuntimeError);
     }
   }
+  if (d_counts)
+    MHB_CHECK(gen, cudaMemcpyAsync(counts.data(), d_counts, count_bytes, cudaMemcpyDeviceToHost,
+                                   gen->stream),
+              mhcudaMemoryCopyError);
   MHB_CHECK(gen, cudaStreamSynchronize(gen->stream), mhcudaMemoryCopyError);
-  gen->bounds_ok = gen->bounds && whole;
+  gen->bounds_fit = d_counts && mhb::bounds_fit(counts.data(), D, S);
+  gen->bounds_ok = d_counts != nullptr;
   return mhcudaSuccess;
 }
 
@@ -1378,8 +1394,8 @@ enum MHCUDAResult mhcuda_calc(const MinhashCudaGenerator *gen, const float *weig
   a.cols = gen->d_cols.as<uint32_t>();
   a.indptr = gen->d_indptr.as<uint32_t>();
   a.out = gen->d_out.as<uint32_t>();
-  MHB_DEBUG(gen, "plan: spl=%u tiles=%u chunk=%u chunks=%u grid=%u\n", plan.spl, plan.ntiles,
-            plan.chunk, plan.nchunks, plan.grid);
+  MHB_DEBUG(gen, "plan: spl=%u tiles=%u chunk=%u chunks=%u grid=%u filter=%u keep=%u\n", plan.spl,
+            plan.ntiles, plan.chunk, plan.nchunks, plan.grid, plan.filter, plan.keep);
   MHB_INFO(gen, "Executing the CUDA kernel...\n");
   r = enqueue_hash(gen, a, plan, st);
   if (r != mhcudaSuccess) return r;
@@ -1541,7 +1557,7 @@ enum MHCUDAResult mhcuda_calc_batch_device(const MinhashCudaGenerator *gen, uint
   // rows is not worth the second launch that takes.
   const int force_filter = env_int("MHCUDA_B200_FILTER", -1);
   const bool may_filter = gen->usable_bounds() && force_filter != 0 &&
-                          (force_filter > 0 || plan_threads >= 512);
+                          (force_filter > 0 || (gen->bounds_fit && plan_threads >= 512));
   // The dense launch of a batch that may be filtered hashes short rows.
   vp.keep = may_filter && vp.spl > 1 && vp.minb == 4;
   TuneChoice tc{};
@@ -1700,7 +1716,7 @@ enum MHCUDAResult mhcuda_autotune(const MinhashCudaGenerator *gen, const float *
     for (uint32_t minb : spl == 4 ? std::vector<uint32_t>{4u, 3u, 2u} : std::vector<uint32_t>{4u})
       for (uint32_t waves : {8u, 32u, 128u}) cands.push_back(TuneChoice{spl, minb, waves});
   }
-  if (gen->usable_bounds())
+  if (gen->usable_bounds() && gen->bounds_fit)
     for (uint32_t waves : {8u, 32u, 128u}) cands.push_back(TuneChoice{4, 4, waves, true});
   cudaEvent_t e0 = nullptr, e1 = nullptr;
   MHB_CHECK(gen, cudaEventCreate(&e0), mhcudaRuntimeError);

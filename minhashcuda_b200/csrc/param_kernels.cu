@@ -34,7 +34,8 @@ template <bool DRAW>
 __global__ void __launch_bounds__(256) pack_kernel(const ParamSources in, uint32_t parts,
                                                    uint32_t dim, uint32_t s_base, uint32_t samples,
                                                    uint32_t s_pad, float *__restrict__ params,
-                                                   uint32_t b_stride, uint8_t *__restrict__ bounds) {
+                                                   uint32_t b_stride, uint8_t *__restrict__ bounds,
+                                                   uint32_t *__restrict__ counts) {
   __shared__ float tile[3][kPackS][kPackD + 1];
   const uint32_t d0 = blockIdx.x * kPackD;
   const uint32_t s0 = blockIdx.y * kPackS;
@@ -73,12 +74,31 @@ __global__ void __launch_bounds__(256) pack_kernel(const ParamSources in, uint32
           tile[which][s][x];
   }
   if (!bounds || parts != 7u) return;
+  uint32_t below[kFitCuts] = {};  // of sample threadIdx.x % kPackS, this thread's columns
 #pragma unroll
   for (uint32_t n = threadIdx.x; n < kPackD * kPackS; n += 256) {
     const uint32_t x = n / kPackS, s = n % kPackS;
-    if (d0 + x < dim && s0 + s < samples)
-      bounds[static_cast<size_t>(d0 + x) * b_stride + s_base + s0 + s] =
-          static_cast<uint8_t>(bound_byte(tile[0][s][x], tile[1][s][x], tile[2][s][x]));
+    if (d0 + x < dim && s0 + s < samples) {
+      const uint32_t byte = bound_byte(tile[0][s][x], tile[1][s][x], tile[2][s][x]);
+      bounds[static_cast<size_t>(d0 + x) * b_stride + s_base + s0 + s] = static_cast<uint8_t>(byte);
+      if constexpr (!DRAW) {
+#pragma unroll
+        for (int k = 0; k < kFitCuts; ++k) below[k] += byte < fit_byte(k);
+      }
+    }
+  }
+  if constexpr (!DRAW) {
+    if (!counts) return;
+    __shared__ uint32_t sums[kPackS][kFitCuts];
+    if (threadIdx.x < kPackS * kFitCuts) sums[threadIdx.x / kFitCuts][threadIdx.x % kFitCuts] = 0;
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < kFitCuts; ++k)
+      if (below[k]) atomicAdd(&sums[threadIdx.x % kPackS][k], below[k]);
+    __syncthreads();
+    const uint32_t s = threadIdx.x / kFitCuts, k = threadIdx.x % kFitCuts;
+    if (s < kPackS && s0 + s < samples && sums[s][k])
+      atomicAdd(&counts[static_cast<size_t>(s_base + s0 + s) * kFitCuts + k], sums[s][k]);
   }
 }
 
@@ -105,17 +125,17 @@ __global__ void unpack_kernel(const float *__restrict__ params, uint32_t which, 
 
 cudaError_t launch_pack_params(const ParamSources &in, bool draw, uint32_t parts, uint32_t dim, uint32_t s_base,
                                uint32_t samples, uint32_t s_pad, float *params, uint8_t *bounds,
-                               cudaStream_t stream) {
+                               uint32_t *counts, cudaStream_t stream) {
   const dim3 block(256);
   const dim3 grid((dim + kPackD - 1) / kPackD, (samples + kPackS - 1) / kPackS);
   if (grid.x == 0 || grid.y == 0) return cudaSuccess;
   const uint32_t stride = bound_stride(s_pad);
   if (draw) {
     pack_kernel<true><<<grid, block, 0, stream>>>(in, parts, dim, s_base, samples, s_pad, params,
-                                                  stride, bounds);
+                                                  stride, bounds, nullptr);
   } else {
     pack_kernel<false><<<grid, block, 0, stream>>>(in, parts, dim, s_base, samples, s_pad, params,
-                                                   stride, bounds);
+                                                   stride, bounds, counts);
   }
   return cudaGetLastError();
 }

@@ -2,6 +2,7 @@
 // Nothing here is part of the public ABI (include/minhashcuda*.h is).
 #pragma once
 
+#include <cmath>
 #include <cstddef>
 #include <cstdint>
 
@@ -87,6 +88,38 @@ constexpr int clamp_weight(int q) {
 // The 16-bit difference whose bit 15 is clear when the entry passes.
 constexpr uint32_t filter_diff(uint32_t byte, int m, int l) {
   return 0xC000u + byte - static_cast<uint32_t>(m + kThrBias) - static_cast<uint32_t>(l);
+}
+// Whether a parameter table is one the filter kernels were made for.  Their
+// guesses and thresholds expect row minima of a generator's distribution; with
+// others every entry passes or samples are scanned twice, and the dense kernels
+// are up to 17 times faster (128 samples, rows of 1400
+// entries: ln_c - 500 4.5 ms against 0.77, ln_c + 6 12.1, ln_c + 1 0.99, all
+// entries equal 8.3).  What matters is how many (column, sample) have ln_c - r
+// below a value: it is compared at four, over the table and for each sample.
+constexpr int kFitCuts = 4;
+// In bytes of the bound table (ln_c - r below -8, -6, -4, -2; a byte of 0 counts
+// at all of them), and the share of a generator's entries below: ln_c of a
+// Gamma(2, 1) variate minus another one, integrated numerically.
+constexpr uint32_t fit_byte(int k) { return 80u + 40u * k; }
+constexpr double kFitShare[kFitCuts] = {0.0028256, 0.0159236, 0.0811733, 0.3368440};
+// counts[s][k]: entries of sample s below cut k, of dim columns.  Beyond six
+// standard deviations (and six entries, for expectations near zero) the table
+// may be off by a tenth, a shift of ln_c by 0.1, and a sample by half.
+inline bool bounds_fit(const uint32_t *counts, uint32_t dim, uint32_t samples) {
+  for (int k = 0; k < kFitCuts; ++k) {
+    double all = 0.0;
+    auto off = [&](double count, double entries, double share) {
+      const double e = entries * kFitShare[k];
+      return std::abs(count - e) > share * e + 6.0 * std::sqrt(e) + 6.0;
+    };
+    for (uint32_t s = 0; s < samples; ++s) {
+      const double n = counts[s * kFitCuts + k];
+      if (off(n, dim, 0.5)) return false;
+      all += n;
+    }
+    if (off(all, static_cast<double>(dim) * samples, 0.1)) return false;
+  }
+  return true;
 }
 // Work division of a filtered launch over `total` = entries x sample tiles and
 // `warps` resident warps: positions per chunk and the snap distance.  `waves`
@@ -224,10 +257,11 @@ struct ParamSources {
 };
 // Fills samples [s_base, s_base + samples) of every column of the parameter
 // table and, if there is one, of the bound table (bound_byte).  parts: bits 0,
-// 1, 2 for r, ln_c, beta; the bound table is written when all are.
+// 1, 2 for r, ln_c, beta; the bound table is written when all are.  counts (not
+// draw; or nullptr): what bounds_fit compares, added to counts[s_base + s].
 cudaError_t launch_pack_params(const ParamSources &in, bool draw, uint32_t parts, uint32_t dim, uint32_t s_base,
                                uint32_t samples, uint32_t s_pad, float *params, uint8_t *bounds,
-                               cudaStream_t stream);
+                               uint32_t *counts, cudaStream_t stream);
 // dst[s*dim + d] = r, ln_c or beta (which 0, 1, 2) of column d, sample
 // s_base + s, for s < samples.
 cudaError_t launch_unpack_params(const float *params, uint32_t which, uint32_t dim,
