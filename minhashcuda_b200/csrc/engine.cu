@@ -303,18 +303,6 @@ bool tuned_choice(const Gen *gen, uint64_t nnz, uint64_t rows, TuneChoice *out,
   return true;
 }
 
-// The filtered kernel evaluates 11-17 candidates per (row, sample) whatever the
-// row's length, the dense one every entry.  Measured on 8M entries in uniform
-// rows, 128 samples (ms, dense / filtered): rows of 60 entries 1.99 / 2.52, of
-// 80 1.97 / 2.02, of 100 1.95 / 1.77, of 120 1.94 / 1.54; 13,003 heavy-tailed
-// rows of 101 on average at 200 samples 652 / 661 us.
-constexpr uint32_t kFilterMinRow = 104;
-// Below it a launch is over before the chip is full: 30,000 entries in
-// 300-entry rows 31 / 34 us, 90,000 entries 69 / 51 us.
-constexpr uint64_t kFilterMinEvals = 1ull << 23;
-// Dense launches under 2^26 evaluations with fewer 64-entry items than this
-// take one sample per lane, for more items.
-constexpr uint64_t kSmallItems = 9472;  // two per resident warp
 // Entries x tiles per resident warp below which tiles are made narrower: twice
 // the warps share a row, each with half the candidates, for a second pass over
 // the CSR.  3,000 rows of 1400 entries (1417 per warp): 485 us whole, 408
@@ -335,7 +323,7 @@ bool use_filter(const Gen *gen, uint64_t nnz, uint64_t rows, const TuneChoice *t
   if (forced >= 0) return forced != 0;
   if (!gen->bounds_fit) return false;
   if (tuned) return tuned->filter;
-  return nnz >= kFilterMinRow * rows && nnz * gen->s_pad >= kFilterMinEvals;
+  return mhb::filter_pays(gen->s_pad, gen->samples, nnz, rows);
 }
 
 // min_items: items per resident warp the chunk is capped to give (8 for the
@@ -360,11 +348,7 @@ HashPlan make_plan(const Gen *gen, uint64_t nnz, uint64_t rows, const TuneChoice
     // Wide tiles amortise the per-nnz overhead (shuffles, addressing, the
     // logf share); narrow tiles give small inputs more warps.  Keep lane
     // utilisation of the last tile >= 3/4.
-    const uint64_t evals = nnz * static_cast<uint64_t>(gen->samples);
-    spl = mhb::tile_fills(s_pad, 4) ? 4 : mhb::tile_fills(s_pad, 2) ? 2 : 1;
-    // Small inputs: more items, unless there are chunks enough as it is.
-    const uint32_t tiles = (s_pad + 32 * spl - 1) / (32 * spl);
-    if (evals < (1ull << 26) && nnz / 64 * tiles < kSmallItems) spl = 1;
+    spl = static_cast<int>(mhb::dense_spl(s_pad, gen->samples, nnz));
   }
   p.spl = static_cast<uint32_t>(spl);
   p.minb = 4;
@@ -1575,8 +1559,8 @@ enum MHCUDAResult mhcuda_calc_batch_device(const MinhashCudaGenerator *gen, uint
     plans[f]->grid = static_cast<uint32_t>(static_cast<uint64_t>(gen->sm_count) * bps);
   }
   b.waves = static_cast<uint64_t>(waves);
-  b.filter_min_row = !may_filter ? 0 : force_filter > 0 ? 1 : kFilterMinRow;
-  b.filter_min_nnz = force_filter > 0 ? 0 : kFilterMinEvals / gen->s_pad;
+  b.filter_min_row = !may_filter ? 0 : force_filter > 0 ? 1 : mhb::filter_rule(gen->s_pad).min_row;
+  b.filter_min_nnz = force_filter > 0 ? 0 : mhb::filter_rule(gen->s_pad).min_batch / gen->s_pad;
   const uint64_t max_chunks64 = count + resident_warps * 8 + 1;
   if (max_chunks64 >= 0xFFFFFFFFull) return mhcudaInvalidArguments;
   const uint32_t max_chunks = static_cast<uint32_t>(max_chunks64);

@@ -80,7 +80,7 @@ extern "C" enum MHCUDAResult mhcuda_calc_device_noalloc(
   // Work decomposition that fits the fixed scratch.
   const uint32_t s_pad = g.s_pad;
   mhb::HashPlan plan{};
-  plan.spl = mhb::tile_fills(s_pad, 4) ? 4 : mhb::tile_fills(s_pad, 2) ? 2 : 1;
+  plan.spl = mhb::dense_spl(s_pad);
   plan.minb = 4;
   plan.ntiles = (s_pad + 32u * plan.spl - 1) / (32u * plan.spl);
   const uint64_t per_chunk = 4 + 2 * static_cast<uint64_t>(s_pad) * (sizeof(float) + sizeof(uint2));

@@ -89,6 +89,62 @@ constexpr int clamp_weight(int q) {
 constexpr uint32_t filter_diff(uint32_t byte, int m, int l) {
   return 0xC000u + byte - static_cast<uint32_t>(m + kThrBias) - static_cast<uint32_t>(l);
 }
+// Samples per lane of the dense kernel: one hash launch of a whole batch or a
+// large matrix, and one of `nnz` entries.  Launches under 2^26 evaluations with
+// fewer 64-entry items than two per resident warp take one sample per lane, for
+// more items.
+constexpr uint64_t kSmallItems = 9472;
+constexpr uint32_t dense_spl(uint32_t s_pad) {
+  return tile_fills(s_pad, 4) ? 4 : tile_fills(s_pad, 2) ? 2 : 1;
+}
+constexpr uint32_t dense_spl(uint32_t s_pad, uint32_t samples, uint64_t nnz) {
+  const uint32_t spl = dense_spl(s_pad), tiles = (s_pad + 32 * spl - 1) / (32 * spl);
+  return nnz * samples < (1ull << 26) && nnz / 64 * tiles < kSmallItems ? 1 : spl;
+}
+// Which launches the filter kernels hash.  They evaluate 11-17 candidates per
+// (row, sample) whatever the row's length, the dense ones every entry; and their
+// warps wait longer for each step, which small launches do not hide.  The lines
+// lie where the dense kernels stop being faster on Zipf(1.1) columns, whose
+// parameters come from L2; uniform columns over large tables, where the dense
+// kernels wait for HBM, gain before that.  Dense / filtered time, Zipf columns
+// (uniform ones in brackets):
+//  - mean row, 512M evaluations: 64 samples rows of 150 0.99, 190 1.15 (200 1.26),
+//    but ragged rows of 230 0.89 and of 268 1.01; 128 samples 130 0.85, 170 0.99,
+//    190 1.09 (130 1.17, 200 1.43), ragged 206 0.98; 256 170 0.97, 190 1.07.
+//    Sample counts that fill the dense tiles less: 100 samples 130 0.95, 160 1.10,
+//    ragged 142 0.88, 170 0.97-1.04; 60 samples 124 1.09; one sample per lane (32,
+//    48, 80) 104 1.09 and more, ragged 112 0.97.
+//  - evaluations, rows of 300 and of 1400: 128 samples 70M 0.82 0.82 (1.08 1.04),
+//    100M 0.92 0.81, 150M 1.20 0.99 (1.46 1.26), 220M 1.31 1.18; 100 samples 100M
+//    1.20 0.93, 150M 1.33 1.18.  Where the dense launch takes one sample per lane:
+//    18M 0.85 0.97, 26M 1.06 1.18, 50M 1.13 1.20.
+//  - long rows, which dense chunks cut into many partials: rows of 12,000 at 70M
+//    1.05, 100M 0.99; with one sample per lane rows of 3000 at 9M 1.04.
+//  - a device batch, whose tiles are always the widest: 128 samples 200M 0.91 0.87,
+//    400M 1.02 0.91, 800M 1.35 1.12; 100 samples 100M 1.06 1.10, 52M 0.84 0.91; 32
+//    samples 18M 0.93, 36M 1.13.
+struct FilterRule {
+  uint32_t min_row;                // entries of the mean row
+  uint64_t min_evals, min_batch;   // evaluations of a launch, of a device batch
+};
+constexpr FilterRule filter_rule(uint32_t s_pad) {
+  const uint32_t spl = dense_spl(s_pad);
+  const uint32_t lanes = (s_pad + 32 * spl - 1) / (32 * spl) * (32 * spl);
+  if (spl == 1) return {112, 3ull << 23, 1ull << 25};
+  if (s_pad == 64) return {288, 5ull << 25, 9ull << 26};
+  if (spl == 2) return {120, 1ull << 27, 1ull << 27};
+  if (5 * s_pad <= 4 * lanes) return {152, 1ull << 27, 1ull << 27};
+  return {184, 5ull << 25, 9ull << 26};
+}
+constexpr bool filter_pays(uint32_t s_pad, uint32_t samples, uint64_t nnz, uint64_t rows) {
+  const FilterRule rule = filter_rule(s_pad);
+  const uint64_t evals = nnz * s_pad;
+  if (nnz < rule.min_row * rows) return false;
+  const bool narrow = dense_spl(s_pad, samples, nnz) == 1;
+  if (nnz >= (narrow ? 3072 : 12288) * rows) return evals >= 1ull << 23;
+  return evals >= rule.min_evals || (narrow && evals >= 3ull << 23);
+}
+
 // Whether a parameter table is one the filter kernels were made for.  Their
 // guesses and thresholds expect row minima of a generator's distribution; with
 // others every entry passes or samples are scanned twice, and the dense kernels

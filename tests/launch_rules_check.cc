@@ -1,0 +1,21 @@
+// Prints the planner's size rules (wmh_internal.h) for the arguments
+// "filter s_pad samples nnz rows" or "batch s_pad nnz rows".
+#include <cstdio>
+#include <cstdlib>
+#include <cstring>
+
+#include "wmh_internal.h"
+
+int main(int argc, char **argv) {
+  auto arg = [&](int i) { return i < argc ? strtoull(argv[i], nullptr, 10) : 0ull; };
+  const uint32_t s_pad = static_cast<uint32_t>(arg(2));
+  if (!strcmp(argv[1], "filter")) {
+    printf("%d", mhb::filter_pays(s_pad, static_cast<uint32_t>(arg(3)), arg(4), arg(5)));
+  } else if (!strcmp(argv[1], "batch")) {
+    const mhb::FilterRule r = mhb::filter_rule(s_pad);
+    printf("%d", arg(3) >= r.min_row * arg(4) && arg(3) >= r.min_batch / s_pad);
+  } else {
+    return 2;
+  }
+  return 0;
+}

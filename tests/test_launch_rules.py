@@ -1,0 +1,64 @@
+"""The planner's size rules on the CPU, against which kernel was measured faster
+(or as fast) on columns whose parameters come from L2, where the filtered kernel
+gains least: a launch that the dense kernel hashes faster stays with it."""
+import os
+import shutil
+import subprocess
+
+import pytest
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+CUDA_INCLUDE = os.path.join(os.environ.get("CUDA_HOME", "/usr/local/cuda"), "include")
+
+pytestmark = pytest.mark.skipif(
+    shutil.which("g++") is None or not os.path.exists(os.path.join(CUDA_INCLUDE, "cuda_runtime.h")),
+    reason="needs g++ and the CUDA headers")
+
+
+@pytest.fixture(scope="module")
+def rule(tmp_path_factory):
+    exe = tmp_path_factory.mktemp("rules") / "check"
+    subprocess.check_call(["g++", "-O1", "-std=c++17", "-I", os.path.join(ROOT, "minhashcuda_b200", "csrc"),
+                           "-I", CUDA_INCLUDE, os.path.join(ROOT, "tests", "launch_rules_check.cc"),
+                           "-o", str(exe)])
+    return lambda *args: subprocess.run([str(exe), *map(str, args)], check=True, capture_output=True,
+                                        text=True).stdout
+
+
+M = 1_000_000
+
+
+# Zipf(1.1) columns over 2^20 dimensions: (samples, evaluations, entries per row),
+# how much faster the filtered kernel is.
+@pytest.mark.parametrize("samples,evals,row,gain", [
+    (64, 512 * M, 104, 0.77), (64, 512 * M, 150, 0.99), (64, 597 * M, 233, 0.89), (64, 686 * M, 268, 0.93),
+    (128, 512 * M, 104, 0.74), (128, 512 * M, 150, 0.94), (256, 512 * M, 130, 0.81),
+    (100, 400 * M, 104, 0.84), (200, 512 * M, 130, 0.95), (384, 512 * M, 150, 0.93),
+    (96, 542 * M, 142, 0.88), (112, 512 * M, 130, 0.92), (48, 9 * M, 106, 0.76),
+    (128, 70 * M, 300, 0.82), (128, 100 * M, 1400, 0.81), (256, 100 * M, 600, 0.79),
+    (64, 70 * M, 1400, 0.86), (64, 40 * M, 300, 0.85), (100, 100 * M, 1400, 0.93),
+    (128, 9 * M, 104, 0.87), (128, 18 * M, 300, 0.85), (32, 18 * M, 300, 0.88),
+    (128, 100 * M, 6000, 0.87),
+    (32, 128 * M, 200, 1.52), (32, 26 * M, 300, 1.06), (64, 512 * M, 300, 1.32),
+    (100, 600 * M, 300, 1.5), (128, 512 * M, 210, 1.10), (128, 220 * M, 300, 1.31),
+    (128, 220 * M, 1400, 1.18), (128, 50 * M, 300, 1.13), (256, 512 * M, 240, 1.14),
+    (200, 512 * M, 170, 1.12), (160, 512 * M, 150, 1.22), (128, 70 * M, 12288, 1.05),
+    (128, 20 * M, 20000, 1.45),
+])
+def test_launches(rule, samples, evals, row, gain):
+    nnz = evals // samples
+    s_pad = (samples + 3) // 4 * 4
+    assert rule("filter", s_pad, samples, nnz, max(1, nnz // row)) == str(int(gain > 1))
+
+
+@pytest.mark.parametrize("samples,evals,row,gain", [
+    (128, 13 * M, 104, 0.58), (128, 101 * M, 600, 0.79), (128, 201 * M, 300, 0.91),
+    (128, 401 * M, 1400, 0.91), (256, 403 * M, 600, 0.90), (64, 200 * M, 300, 0.98),
+    (100, 52 * M, 300, 0.84), (32, 18 * M, 300, 0.86),
+    (128, 801 * M, 300, 1.35), (256, 803 * M, 1400, 1.13), (64, 801 * M, 600, 1.50),
+    (100, 202 * M, 300, 1.21), (32, 50 * M, 300, 1.20),
+    (256, 6000 * M, 195, 1.0001),  # uniform columns, ragged: 2.15
+])
+def test_device_batches(rule, samples, evals, row, gain):
+    nnz = evals // samples
+    assert rule("batch", (samples + 3) // 4 * 4, nnz, max(1, nnz // row)) == str(int(gain > 1))
