@@ -309,13 +309,6 @@ bool tuned_choice(const Gen *gen, uint64_t nnz, uint64_t rows, TuneChoice *out,
 // halved; 20,011 rows of 300 (2030 per warp): 481 whole, 567 halved.
 constexpr uint64_t kFilterShare = 1500;
 
-// Mean rows below which the dense kernel keeps t with each minimum (RowState):
-// rows of 20 entries 2.64 -> 2.21 ms, of 60 2.27 -> 1.99, of 420 (heavy tail,
-// 256 samples) 6.14 -> 5.86; rows of 1400 Zipf entries 27.9 -> 28.5.  With one
-// sample per lane only tiny launches do (one 300-entry row 21.9 -> 17.8 us
-// alone); others lose (400,000 rows of 20 at 32 samples 0.84 -> 0.99 ms).
-constexpr uint64_t kKeepMaxRow = 512;
-
 // Whether a launch takes the bound-filtered kernel (filter_kernels.cu).
 bool use_filter(const Gen *gen, uint64_t nnz, uint64_t rows, const TuneChoice *tuned) {
   if (!gen->usable_bounds()) return false;
@@ -400,7 +393,7 @@ HashPlan make_plan(const Gen *gen, uint64_t nnz, uint64_t rows, const TuneChoice
           least_chunk, (((nnz * p.ntiles + resident_warps - 1) / resident_warps) + 7) & ~7ull);
     }
   }
-  p.keep = !p.filter && p.minb == 4 && (p.spl > 1 || tiny) && avg_row < kKeepMaxRow;
+  p.keep = !p.filter && p.minb == 4 && avg_row < mhb::keep_rows(s_pad, p.spl, tiny);
   const int forced = env_int("MHCUDA_B200_CHUNK", 0);
   if (forced > 0) chunk = static_cast<uint64_t>(forced);
   if (!tiny || forced > 0) chunk = std::max<uint64_t>(64, (chunk + 31) & ~31ull);
@@ -1542,8 +1535,7 @@ enum MHCUDAResult mhcuda_calc_batch_device(const MinhashCudaGenerator *gen, uint
   const int force_filter = env_int("MHCUDA_B200_FILTER", -1);
   const bool may_filter = gen->usable_bounds() && force_filter != 0 &&
                           (force_filter > 0 || (gen->bounds_fit && plan_threads >= 512));
-  // The dense launch of a batch that may be filtered hashes short rows.
-  vp.keep = may_filter && vp.spl > 1 && vp.minb == 4;
+  vp.keep = 0;  // the batch kernels do without (keep_rows)
   TuneChoice tc{};
   const int waves = std::max(1, env_int("MHCUDA_B200_WAVES", static_cast<int>(tc.waves)));
   mhb::BatchArgs b{};
@@ -1568,10 +1560,9 @@ enum MHCUDAResult mhcuda_calc_batch_device(const MinhashCudaGenerator *gen, uint
   big.nchunks = max_chunks;
   HashArgs base{};
   big.filter = may_filter;  // for next_item
-  big.keep = vp.keep;
   MHCUDAResult r = prepare_launch(gen, 0, 0, big, &base);
   if (r != mhcudaSuccess) return r;
-  base.part_t = vp.keep;  // a filtered batch has it too (matrix_view)
+  base.part_t = 0;  // set for a filtered batch by matrix_view
   MHB_CHECK(gen, gen->d_chunk_owner.ensure(static_cast<size_t>(max_chunks) * 4),
             mhcudaMemoryAllocationFailure);
   MHB_CHECK(gen, gen->d_batch_plan.ensure(sizeof(mhb::BatchPlan)), mhcudaMemoryAllocationFailure);

@@ -499,7 +499,7 @@ __device__ __forceinline__ HashArgs matrix_view(const BatchArgs &b, const BatchM
   v.chunk = chunk;
   v.nchunks = m.nchunks;
   v.snap = b.plan->snap;
-  v.part_t = b.base.part_t || b.plan->filter;
+  v.part_t = b.plan->filter;
   v.chunk_row = b.base.chunk_row + m.chunk_base;
   v.part_ln = b.base.part_ln + static_cast<size_t>(2) * m.chunk_base * b.base.s_pad;
   v.part_kt = b.base.part_kt + static_cast<size_t>(2) * m.chunk_base * b.base.s_pad;

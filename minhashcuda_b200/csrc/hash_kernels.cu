@@ -547,7 +547,7 @@ __global__ void batch_plan_kernel(const BatchArgs b, uint32_t plan_threads) {
 // The matrix view of an item is kept in shared memory, one per warp: its
 // fields are read where the item needs them (per row or window), so the
 // evaluation loop's registers are the single-matrix kernel's.
-template <int SPL, int MINB, int SPAD, bool KEEP>
+template <int SPL, int MINB, int SPAD>
 __global__ void __launch_bounds__(kHashBlock, MINB) hash_batch_kernel(const BatchArgs b) {
   __shared__ WarpStage stage_all[kHashBlock / 32];
   __shared__ HashArgs views[kHashBlock / 32];
@@ -567,7 +567,7 @@ __global__ void __launch_bounds__(kHashBlock, MINB) hash_batch_kernel(const Batc
     __syncwarp();
     if (wc.lane == 0) view = matrix_view(b, b.mats[m], chunk);
     __syncwarp();
-    if (!hash_item<SPL, SPAD, false, param_depth(MINB), KEEP>(view, gc - base, item - gc * ntiles, wc))
+    if (!hash_item<SPL, SPAD, false, param_depth(MINB), false>(view, gc - base, item - gc * ntiles, wc))
       return;
   }
 }
@@ -617,36 +617,35 @@ using BatchFn = void (*)(const BatchArgs);
 // Instantiated (samples per lane, minimum resident blocks per SM) variants,
 // with s_pad compiled in for the common sample counts.  The 4-block ones come
 // with and without KEEP.
-#define MHB_PICK(KERNEL, ...)                                      \
-  switch (spl * 100000 + minb * 10000 + s_pad) {                   \
-    case 440128: return KERNEL<4, 4, 128, __VA_ARGS__ KEEP>;       \
-    case 440256: return KERNEL<4, 4, 256, __VA_ARGS__ KEEP>;       \
-    case 240064: return KERNEL<2, 4, 64, __VA_ARGS__ KEEP>;        \
-    case 430128: return KERNEL<4, 3, 128, __VA_ARGS__ false>;      \
-    case 420128: return KERNEL<4, 2, 128, __VA_ARGS__ false>;      \
-    case 430256: return KERNEL<4, 3, 256, __VA_ARGS__ false>;      \
-    case 420256: return KERNEL<4, 2, 256, __VA_ARGS__ false>;      \
-    default: break;                                                \
-  }                                                                \
-  switch (spl * 10 + minb) {                                       \
-    case 44: return KERNEL<4, 4, 0, __VA_ARGS__ KEEP>;             \
-    case 24: return KERNEL<2, 4, 0, __VA_ARGS__ KEEP>;             \
-    case 14: return KERNEL<1, 4, 0, __VA_ARGS__ KEEP>;             \
-    case 43: return KERNEL<4, 3, 0, __VA_ARGS__ false>;            \
-    case 42: return KERNEL<4, 2, 0, __VA_ARGS__ false>;            \
-    default: return nullptr;                                       \
+#define MHB_PICK(PICKED)                          \
+  switch (spl * 100000 + minb * 10000 + s_pad) {  \
+    case 440128: return PICKED(4, 4, 128, KEEP);  \
+    case 440256: return PICKED(4, 4, 256, KEEP);  \
+    case 240064: return PICKED(2, 4, 64, KEEP);   \
+    case 430128: return PICKED(4, 3, 128, false); \
+    case 420128: return PICKED(4, 2, 128, false); \
+    case 430256: return PICKED(4, 3, 256, false); \
+    case 420256: return PICKED(4, 2, 256, false); \
+    default: break;                               \
+  }                                               \
+  switch (spl * 10 + minb) {                      \
+    case 44: return PICKED(4, 4, 0, KEEP);        \
+    case 24: return PICKED(2, 4, 0, KEEP);        \
+    case 14: return PICKED(1, 4, 0, KEEP);        \
+    case 43: return PICKED(4, 3, 0, false);       \
+    case 42: return PICKED(4, 2, 0, false);       \
+    default: return nullptr;                      \
   }
-#define MHB_COMMA ,
+#define MHB_BATCH(SPL, MINB, SPAD, KEEP) hash_batch_kernel<SPL, MINB, SPAD>
+#define MHB_HASH(SPL, MINB, SPAD, KEEP) hash_kernel<SPL, MINB, SPAD, PACKED, KEEP>
 
-template <bool KEEP>
-BatchFn pick_batch(uint32_t spl, uint32_t minb, uint32_t s_pad) {
-  MHB_PICK(hash_batch_kernel)
-}
+BatchFn pick_batch(uint32_t spl, uint32_t minb, uint32_t s_pad) { MHB_PICK(MHB_BATCH) }
 template <bool PACKED, bool KEEP>
 HashFn pick_hash(uint32_t spl, uint32_t minb, uint32_t s_pad) {
-  MHB_PICK(hash_kernel, PACKED MHB_COMMA)
+  MHB_PICK(MHB_HASH)
 }
-#undef MHB_COMMA
+#undef MHB_HASH
+#undef MHB_BATCH
 #undef MHB_PICK
 
 HashFn pick_hash(uint32_t spl, uint32_t minb, uint32_t s_pad, bool packed, bool keep) {
@@ -676,8 +675,7 @@ cudaError_t launch_finalize(const HashArgs &a, cudaStream_t stream) {
 
 cudaError_t launch_batch(const BatchArgs &b, const HashPlan &dense, const HashPlan &filtered,
                          uint32_t plan_threads, cudaStream_t stream) {
-  const BatchFn fn = dense.keep ? pick_batch<true>(dense.spl, dense.minb, b.base.s_pad)
-                                : pick_batch<false>(dense.spl, dense.minb, b.base.s_pad);
+  const BatchFn fn = pick_batch(dense.spl, dense.minb, b.base.s_pad);
   if (!fn || b.count == 0 || b.max_chunks == 0) return cudaErrorInvalidValue;
   batch_setup_kernel<<<1, kSetupThreads, 0, stream>>>(b);
   if (plan_threads)

@@ -101,6 +101,28 @@ constexpr uint32_t dense_spl(uint32_t s_pad, uint32_t samples, uint64_t nnz) {
   const uint32_t spl = dense_spl(s_pad), tiles = (s_pad + 32 * spl - 1) / (32 * spl);
   return nnz * samples < (1ull << 26) && nnz / 64 * tiles < kSmallItems ? 1 : spl;
 }
+// Mean rows below which a dense launch keeps t with each minimum (RowState): an
+// instruction more per evaluation, against three gathers, a logarithm and a
+// division per (row, sample) at the row's end.  4M entries, without / with it on
+// uniform columns [on Zipf ones, whose parameters come from L2]:
+//  - 128 samples (s_pad compiled in) rows of 20 1.28 / 1.08 ms [0.72 / 0.67], 70
+//    1.12 / 1.03 [0.57 / 0.57], 100 1.08 / 1.02 [0.571 / 0.580], 140 and more 3%
+//    faster [2-4% slower]; 64 samples rows of 50 10% faster [0.4% slower], 70 9%
+//    faster [2% slower], 140 5% faster [4% slower];
+//  - other sample counts never lose: 200 samples rows of 100 5% faster [0.5%],
+//    of 500 even.
+//  - One sample per lane only in tiny launches (one 300-entry row 21.9 -> 17.8 us
+//    alone); 400,000 rows of 20 at 32 samples 0.84 -> 0.99 ms.
+//  - Not in device batches, whose mean row the host does not know: 128 samples
+//    rows of 10 to 60 1.12-1.07 times as fast [1.14-0.97], of 100 and more 1.04-1.0
+//    [0.96-0.93]; 64 samples 0.86-0.99 [1.12-1.0].
+constexpr uint32_t keep_rows(uint32_t s_pad, uint32_t spl, bool tiny) {
+  if (tiny) return 512;
+  if (spl == 4 && (s_pad == 128 || s_pad == 256)) return 96;
+  if (spl == 2 && s_pad == 64) return 64;
+  return spl > 1 ? 512 : 0;
+}
+
 // Which launches the filter kernels hash.  They evaluate 11-17 candidates per
 // (row, sample) whatever the row's length, the dense ones every entry; and their
 // warps wait longer for each step, which small launches do not hide.  The lines

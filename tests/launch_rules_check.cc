@@ -1,5 +1,6 @@
 // Prints the planner's size rules (wmh_internal.h) for the arguments
-// "filter s_pad samples nnz rows" or "batch s_pad nnz rows".
+// "filter s_pad samples nnz rows", "batch s_pad nnz rows" or "keep s_pad spl
+// tiny mean_row".
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
@@ -14,6 +15,8 @@ int main(int argc, char **argv) {
   } else if (!strcmp(argv[1], "batch")) {
     const mhb::FilterRule r = mhb::filter_rule(s_pad);
     printf("%d", arg(3) >= r.min_row * arg(4) && arg(3) >= r.min_batch / s_pad);
+  } else if (!strcmp(argv[1], "keep")) {
+    printf("%d", arg(5) < mhb::keep_rows(s_pad, static_cast<uint32_t>(arg(3)), arg(4) != 0));
   } else {
     return 2;
   }

@@ -62,3 +62,20 @@ def test_launches(rule, samples, evals, row, gain):
 def test_device_batches(rule, samples, evals, row, gain):
     nnz = evals // samples
     assert rule("batch", (samples + 3) // 4 * 4, nnz, max(1, nnz // row)) == str(int(gain > 1))
+
+
+# How much faster a dense launch is with t kept, on Zipf columns and on uniform
+# ones: kept where the loss on the one side is below 2%, or nothing is lost.
+@pytest.mark.parametrize("s_pad,spl,row,zipf,uniform", [
+    (64, 2, 20, 1.04, 1.11), (64, 2, 50, 0.996, 1.11), (64, 2, 100, 0.966, 1.07),
+    (64, 2, 300, 0.94, 1.01), (128, 4, 20, 1.08, 1.18), (128, 4, 70, 1.004, 1.08),
+    (128, 4, 140, 0.976, 1.03), (128, 4, 500, 0.956, 1.0), (256, 4, 70, 1.006, 1.08),
+    (256, 4, 180, 0.968, 1.02), (200, 4, 100, 1.005, 1.05), (200, 4, 300, 1.0, 1.004),
+    (512, 4, 140, 0.997, 1.03), (32, 1, 20, 0.85, 0.85),
+])
+def test_t_kept(rule, s_pad, spl, row, zipf, uniform):
+    assert rule("keep", s_pad, spl, 0, row) == str(int(min(zipf, uniform) > 0.98))
+
+
+def test_t_kept_in_tiny_launches(rule):
+    assert rule("keep", 128, 1, 1, 300) == "1"
