@@ -335,6 +335,10 @@ HashPlan make_plan(const Gen *gen, uint64_t nnz, uint64_t rows, const TuneChoice
   } else {
     have_tuned = tuned_choice(gen, nnz, rows, &tuned);
   }
+  const bool filter = allow_filter && use_filter(gen, nnz, rows, have_tuned ? &tuned : nullptr);
+  // The autotuner chose the filtered kernel, whose samples per lane and blocks
+  // stand in for settings it has not; a dense launch is then not tuned.
+  if (have_tuned && tuned.filter && !filter) have_tuned = false;
   int spl = env_int("MHCUDA_B200_SPL", 0);
   if (have_tuned && spl == 0) spl = static_cast<int>(tuned.spl);
   if (spl != 1 && spl != 2 && spl != 4) {
@@ -345,7 +349,7 @@ HashPlan make_plan(const Gen *gen, uint64_t nnz, uint64_t rows, const TuneChoice
   }
   p.spl = static_cast<uint32_t>(spl);
   p.minb = 4;
-  if (allow_filter && use_filter(gen, nnz, rows, have_tuned ? &tuned : nullptr)) {
+  if (filter) {
     p.filter = mhb::filter_lanes(s_pad);
     p.spl = 4;
   }
