@@ -381,7 +381,7 @@ HashPlan make_plan(const Gen *gen, uint64_t nnz, uint64_t rows, const TuneChoice
       p.filter /= 2;
       p.ntiles = mhb::filter_tiles(s_pad, p.filter);
     }
-    const mhb::FilterSplit sp = mhb::filter_split(nnz * p.ntiles, resident_warps, waves, avg_row);
+    const mhb::FilterSplit sp = mhb::filter_split(nnz * p.ntiles, resident_warps, waves, avg_row, min_items);
     chunk = sp.chunk;
     p.snap = sp.snap;
   } else {

@@ -303,7 +303,8 @@ MHCUDAResult MinhashCudaServer_::run_units(Lane &lane, const std::vector<Unit> &
   const uint32_t s_pad = g.s_pad;
   // Batches are small next to a plain call: at least two waves of warp items
   // even when rows are long (the plain plan keeps a few rows per chunk);
-  // several lanes' launches overlap, so two are enough.
+  // several lanes' launches overlap, so two are enough.  Filtered batches are
+  // cut into eight or more (filter_split).
   mhb::HashPlan plan = mhb::plan_for_generator(units.front().req->gen, N, R,
                                                high ? min_items_high : min_items_low,
                                                !zc && g.bounds != nullptr);

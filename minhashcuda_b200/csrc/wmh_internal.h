@@ -202,18 +202,21 @@ inline bool bounds_fit(const uint32_t *counts, uint32_t dim, uint32_t samples) {
 // Work division of a filtered launch over `total` = entries x sample tiles and
 // `warps` resident warps: positions per chunk and the snap distance.  `waves`
 // chunks per warp, but none shorter than a mean row as long as that leaves
-// eight per warp, nor than 128 positions; rows are kept whole up to a quarter
-// of a warp's share.
+// `parts` per warp, nor than 128 positions; rows are kept whole up to two such
+// parts.  parts: eight, or min_items if that is more (a server that wants short
+// items): rows in pieces start their search anew.
 struct FilterSplit {
   uint32_t chunk, snap;
 };
 __host__ __device__ inline FilterSplit filter_split(uint64_t total, uint64_t warps, uint64_t waves,
-                                                    uint64_t avg_row) {
+                                                    uint64_t avg_row, uint32_t min_items = 8) {
   const uint64_t share = total / warps;
-  uint64_t chunk = share / waves, whole = share / 8 < avg_row ? share / 8 : avg_row;
-  chunk = chunk > whole ? chunk : whole;
+  const uint64_t parts = min_items > 8 ? min_items : 8;
+  const uint64_t shortest = share / (min_items > waves ? min_items : waves);
+  const uint64_t whole = share / parts < avg_row ? share / parts : avg_row;
+  uint64_t chunk = shortest > whole ? shortest : whole;
   chunk = chunk < 128 ? 128 : chunk > (1u << 24) ? (1u << 24) : (chunk + 31) & ~31ull;
-  uint64_t snap = share / 4 < 8192 ? share / 4 : 8192;
+  uint64_t snap = 2 * share / parts < 8192 ? 2 * share / parts : 8192;
   snap = snap > chunk ? snap : chunk;
   return FilterSplit{static_cast<uint32_t>(chunk), static_cast<uint32_t>(snap)};
 }

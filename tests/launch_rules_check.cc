@@ -1,6 +1,6 @@
 // Prints the planner's size rules (wmh_internal.h) for the arguments
-// "filter s_pad samples nnz rows", "batch s_pad nnz rows" or "keep s_pad spl
-// tiny mean_row".
+// "filter s_pad samples nnz rows", "batch s_pad nnz rows", "keep s_pad spl
+// tiny mean_row" or "split total warps waves mean_row min_items".
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
@@ -17,6 +17,9 @@ int main(int argc, char **argv) {
     printf("%d", arg(3) >= r.min_row * arg(4) && arg(3) >= r.min_batch / s_pad);
   } else if (!strcmp(argv[1], "keep")) {
     printf("%d", arg(5) < mhb::keep_rows(s_pad, static_cast<uint32_t>(arg(3)), arg(4) != 0));
+  } else if (!strcmp(argv[1], "split")) {
+    const mhb::FilterSplit p = mhb::filter_split(arg(2), arg(3), arg(4), arg(5), static_cast<uint32_t>(arg(6)));
+    printf("%u %u", p.chunk, p.snap);
   } else {
     return 2;
   }

@@ -79,3 +79,18 @@ def test_t_kept(rule, s_pad, spl, row, zipf, uniform):
 
 def test_t_kept_in_tiny_launches(rule):
     assert rule("keep", 128, 1, 1, 300) == "1"
+
+
+@pytest.mark.parametrize("mean_row", [130, 1400, 60_000])
+@pytest.mark.parametrize("share", [2000, 40_000, 300_000])
+def test_filtered_items_follow_min_items(rule, share, mean_row):
+    """Up to eight items per warp asked for, chunks are what they are without; more
+    make them shorter, also beyond the 32 waves aimed at."""
+    split = lambda items: list(map(int, rule("split", share * 3552, 3552, 32, mean_row, items).split()))  # noqa: E731
+    chunk = max(share // 32, min(share // 8, mean_row))
+    chunk = max(128, (chunk + 31) // 32 * 32)
+    assert split(2) == split(8) == [chunk, max(chunk, min(share // 4, 8192))]
+    for items in (16, 64):
+        got = split(items)
+        assert got[0] <= max(128, share // items + 31)
+        assert got[0] + got[1] <= max(256, 3 * share // items + 31)
