@@ -1534,11 +1534,11 @@ enum MHCUDAResult mhcuda_calc_batch_device(const MinhashCudaGenerator *gen, uint
   HashPlan fp = vp;
   fp.filter = mhb::filter_lanes(gen->s_pad);
   fp.ntiles = mhb::filter_tiles(gen->s_pad, fp.filter);
-  // Whether the batch is filtered is decided on the device too; a batch of few
-  // rows is not worth the second launch that takes.
+  // Whether the batch is filtered is decided on the device too, unless it has too
+  // few rows for the second launch that takes.
   const int force_filter = env_int("MHCUDA_B200_FILTER", -1);
   const bool may_filter = gen->usable_bounds() && force_filter != 0 &&
-                          (force_filter > 0 || (gen->bounds_fit && plan_threads >= 512));
+                          (force_filter > 0 || (gen->bounds_fit && plan_threads >= mhb::filter_batch_rows(gen->s_pad)));
   vp.keep = 0;  // the batch kernels do without (keep_rows)
   TuneChoice tc{};
   const int waves = std::max(1, env_int("MHCUDA_B200_WAVES", static_cast<int>(tc.waves)));

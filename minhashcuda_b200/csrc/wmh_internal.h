@@ -158,6 +158,13 @@ constexpr FilterRule filter_rule(uint32_t s_pad) {
   if (5 * s_pad <= 4 * lanes) return {152, 1ull << 27, 1ull << 27};
   return {184, 5ull << 25, 9ull << 26};
 }
+// Rows (and one per matrix) from which a device batch launches both kernels, one
+// of which returns at once: 2 us of a batch that takes 55-80 with 600 rows of 100
+// entries.  Fewer rows reach min_batch only with over 4096 entries each.
+constexpr uint64_t filter_batch_rows(uint32_t s_pad) {
+  const uint64_t rows = filter_rule(s_pad).min_batch / (4096ull * s_pad);
+  return rows > 512 ? rows : 512;
+}
 constexpr bool filter_pays(uint32_t s_pad, uint32_t samples, uint64_t nnz, uint64_t rows) {
   const FilterRule rule = filter_rule(s_pad);
   const uint64_t evals = nnz * s_pad;

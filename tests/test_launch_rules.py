@@ -94,3 +94,11 @@ def test_filtered_items_follow_min_items(rule, share, mean_row):
         got = split(items)
         assert got[0] <= max(128, share // items + 31)
         assert got[0] + got[1] <= max(256, 3 * share // items + 31)
+
+
+@pytest.mark.parametrize("s_pad,rows,both", [
+    (128, 600, 0), (128, 1200, 1), (64, 2000, 0), (64, 2400, 1), (256, 600, 1), (32, 500, 0), (32, 520, 1)])
+def test_batches_that_launch_both_kernels(rule, s_pad, rows, both):
+    """A batch that could only be filtered with rows of over 4096 entries is spared
+    the second launch."""
+    assert rule("both", s_pad, rows) == str(both)
