@@ -1299,7 +1299,16 @@ enum MHCUDAResult mhcuda_assign_random_vars(const MinhashCudaGenerator *gen, con
   std::vector<uint32_t> counts(static_cast<size_t>(S) * mhb::kFitCuts);
   const size_t count_bytes = counts.size() * sizeof(uint32_t);
   const bool whole = tmp.ensure(3 * block * sizeof(float) + count_bytes) == cudaSuccess;
-  if (!whole) MHB_CHECK(gen, tmp.ensure(block * sizeof(float)), mhcudaMemoryAllocationFailure);
+  if (!whole) {
+    MHB_CHECK(gen, tmp.ensure(block * sizeof(float)), mhcudaMemoryAllocationFailure);
+    // Calls no longer take the bound table, but a caller's CUDA graph of an
+    // earlier filtered call still reads it: with zeros every entry passes.
+    if (gen->bounds)
+      MHB_CHECK(gen, cudaMemsetAsync(gen->bounds, 0,
+                                     static_cast<size_t>(D) * mhb::bound_stride(gen->s_pad),
+                                     gen->stream),
+                mhcudaRuntimeError);
+  }
   uint32_t *d_counts = nullptr;
   if (whole && gen->bounds) {
     d_counts = reinterpret_cast<uint32_t *>(tmp.as<float>() + 3 * block);
