@@ -51,8 +51,11 @@ def test_captured_filtered_call_follows_assign(scarce, monkeypatch):
             free = torch.cuda.mem_get_info()[0]
             hold = torch.empty(free - 2 * block, dtype=torch.uint8, device="cuda")
             assert block < torch.cuda.mem_get_info()[0] < 3 * block
-        eng.assign(*second)
-        del hold
+        try:
+            eng.assign(*second)
+        finally:
+            del hold
+            torch.cuda.empty_cache()  # back to the device: the engine allocates beside torch
         out.zero_()
         graph.replay()
         torch.cuda.synchronize()
