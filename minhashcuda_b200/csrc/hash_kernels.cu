@@ -465,8 +465,8 @@ __global__ void __launch_bounds__(kSetupThreads) batch_setup_kernel(const BatchA
   block_exclusive_scan(nonempty, &total_nonempty);
   __shared__ uint32_t s_chunk;
   if (t == 0) {
-    const uint32_t f = b.filter_min_row && total_nnz >= total_rows * b.filter_min_row &&
-                       total_nnz >= b.filter_min_nnz;
+    const uint32_t f = b.filter_min_row && total_nnz >= b.filter_min_nnz &&
+                       total_nnz >= total_rows * filter_row(b.filter_min_row, total_nnz * b.base.s_pad / 2);
     b.plan->filter = f;
     const uint64_t ntiles = b.ntiles[f], target = b.warps[f] * b.waves, want = b.warps[f] * 8;
     uint64_t chunk = (total_nnz * ntiles + target - 1) / target;

@@ -125,38 +125,55 @@ constexpr uint32_t keep_rows(uint32_t s_pad, uint32_t spl, bool tiny) {
 
 // Which launches the filter kernels hash.  They evaluate 11-17 candidates per
 // (row, sample) whatever the row's length, the dense ones every entry; and their
-// warps wait longer for each step, which small launches do not hide.  The lines
-// lie where the dense kernels stop being faster on Zipf(1.1) columns, whose
-// parameters come from L2; uniform columns over large tables, where the dense
-// kernels wait for HBM, gain before that.  Dense / filtered time, Zipf columns
-// (uniform ones in brackets):
-//  - mean row, 512M evaluations: 64 samples rows of 150 0.99, 190 1.15 (200 1.26),
-//    but ragged rows of 230 0.89 and of 268 1.01; 128 samples 130 0.85, 170 0.99,
-//    190 1.09 (130 1.17, 200 1.43), ragged 206 0.98; 256 170 0.97, 190 1.07.
-//    Sample counts that fill the dense tiles less: 100 samples 130 0.95, 160 1.10,
-//    ragged 142 0.88, 170 0.97-1.04; 60 samples 124 1.09; one sample per lane (32,
-//    48, 80) 104 1.09 and more, ragged 112 0.97.
-//  - evaluations, rows of 300 and of 1400: 128 samples 70M 0.82 0.82 (1.08 1.04),
-//    100M 0.92 0.81, 150M 1.20 0.99 (1.46 1.26), 220M 1.31 1.18; 100 samples 100M
-//    1.20 0.93, 150M 1.33 1.18.  Where the dense launch takes one sample per lane:
-//    18M 0.85 0.97, 26M 1.06 1.18, 50M 1.13 1.20.
-//  - long rows, which dense chunks cut into many partials: rows of 12,000 at 70M
-//    1.05, 100M 0.99; with one sample per lane rows of 3000 at 9M 1.04.
-//  - a device batch, whose tiles are always the widest: 128 samples 200M 0.91 0.87,
-//    400M 1.02 0.91, 800M 1.35 1.12; 100 samples 100M 1.06 1.10, 52M 0.84 0.91; 32
-//    samples 18M 0.93, 36M 1.13.
+// warps wait longer for each step, which small launches do not hide.  On Zipf(1.1)
+// columns, whose parameters come from L2, the dense kernels are faster than on
+// uniform columns over large tables, where they wait for HBM; the host knows
+// neither, so the lines lie where Zipf columns stop losing (by a few percent
+// where uniform ones gain a fifth).  The mean row that takes falls as launches
+// grow.  Dense / filtered time over 16,767 launches and 4,482 device batches of
+// 32 to 512 samples, rows of even length and ragged ones, as geometric means on
+// Zipf [uniform] columns for mean rows of 105-120, 150-170 and 215-250 entries:
+//  - full dense tiles (128, 256, 384 samples): 134-168M evaluations .71 [.98], .81
+//    [1.16], .98 [1.26]; 268-400M .77 [.98], .90 [1.20], 1.01 [1.39]; 800-1200M .93
+//    [1.17], 1.11 [1.31], 1.25 [1.54]; above 1800M 1.00 [1.18], 1.19 [1.42], 1.44
+//    [1.78]; at 67-134M .92-.99 [1.15-1.33] even in rows of 400;
+//  - 64 samples: 268-400M .78 [.84], .88 [.97], 1.04 [1.29]; 800-1200M .80 [.98],
+//    .94 [1.18], 1.09 [1.52]; above 1800M .88 [1.0], 1.02 [1.21], 1.29 [1.35];
+//  - tiles filled less (96, 100, 200): 168-268M .86 [.98], 1.00 [1.19], 1.18 [1.35];
+//    800-1200M 1.07 [1.07], 1.34 [1.31], 1.51 [1.79];
+//  - two samples per lane (48, 60, 160): 67-100M .86 [.96], .96 [1.13], 1.17 [1.31];
+//    168-268M .95 [.97], 1.10 [1.14], 1.34 [1.26];
+//  - one sample per lane (32, 80): 67-100M 1.11 [1.19], 1.11 [1.46], 1.29 [1.48];
+//  - small launches of 128 samples, which the dense kernel takes with one sample per
+//    lane: 25-38M .86 [.99], .99 [1.09], 1.08 [1.27]; 38-67M .93 [1.18], 1.15 [1.34],
+//    1.15 [1.43]; 12-25M rows of 190 .98 [1.1], of 300 1.03-1.09 [1.18-1.29];
+//  - long rows, which dense chunks cut into many partials: rows of 12,000 at 70M 1.05;
+//  - a device batch of 128 or 256 samples, whose tiles are always the widest: rows of
+//    170 and 300 at 268-400M .84 [1.22], 1.01 [1.19], at 400-600M 1.10 [1.23], 1.10
+//    [1.38]; rows of 135 at 1200-1800M 1.03 [1.31].
 struct FilterRule {
-  uint32_t min_row;                // entries of the mean row
+  uint32_t min_row;                // entries of the mean row (filter_row)
   uint64_t min_evals, min_batch;   // evaluations of a launch, of a device batch
 };
 constexpr FilterRule filter_rule(uint32_t s_pad) {
   const uint32_t spl = dense_spl(s_pad);
   const uint32_t lanes = (s_pad + 32 * spl - 1) / (32 * spl) * (32 * spl);
-  if (spl == 1) return {112, 3ull << 23, 1ull << 25};
-  if (s_pad == 64) return {288, 5ull << 25, 9ull << 26};
-  if (spl == 2) return {120, 1ull << 27, 1ull << 27};
-  if (5 * s_pad <= 4 * lanes) return {152, 1ull << 27, 1ull << 27};
-  return {184, 5ull << 25, 9ull << 26};
+  if (spl == 1) return {104, 1ull << 26, 1ull << 25};
+  if (s_pad == 64) return {288, 1ull << 27, 9ull << 26};
+  if (spl == 2) return {120, 9ull << 22, 1ull << 27};
+  if (5 * s_pad <= 4 * lanes) return {152, 7ull << 24, 1ull << 27};
+  return {168, 1ull << 27, 7ull << 26};
+}
+// The mean row from which a launch of `evals` evaluations is filtered.  A device
+// batch needs those of a launch of half its size.
+constexpr uint64_t filter_row(uint64_t row, uint64_t evals) {
+  if (row <= 104) return row;
+  if (evals < 1ull << 26) row = 2 * row;
+  else if (evals < 5ull << 25) row = row * 5 / 4 < 288 ? row * 5 / 4 : 288;
+  else if (evals >= 3ull << 30) row = row / 2;
+  else if (evals >= 3ull << 29) row = row * 5 / 8;
+  else if (evals >= 3ull << 28) row = row * 3 / 4;
+  return row > 104 ? row : 104;
 }
 // Rows (and one per matrix) from which a device batch launches both kernels, one
 // of which returns at once: 2 us of a batch that takes 55-80 with 600 rows of 100
@@ -168,10 +185,11 @@ constexpr uint64_t filter_batch_rows(uint32_t s_pad) {
 constexpr bool filter_pays(uint32_t s_pad, uint32_t samples, uint64_t nnz, uint64_t rows) {
   const FilterRule rule = filter_rule(s_pad);
   const uint64_t evals = nnz * s_pad;
-  if (nnz < rule.min_row * rows) return false;
-  const bool narrow = dense_spl(s_pad, samples, nnz) == 1;
-  if (nnz >= (narrow ? 3072 : 12288) * rows) return evals >= 1ull << 23;
-  return evals >= rule.min_evals || (narrow && evals >= 3ull << 23);
+  if (evals < 1ull << 23) return false;
+  if (nnz >= 12288 * rows) return true;
+  if (evals < 1ull << 26 && dense_spl(s_pad, samples, nnz) == 1)
+    return nnz >= (evals >= 9ull << 22 ? 120 : evals >= 3ull << 23 ? 144 : 320) * rows;
+  return evals >= rule.min_evals && nnz >= filter_row(rule.min_row, evals) * rows;
 }
 
 // Whether a parameter table is one the filter kernels were made for.  Their
@@ -301,9 +319,9 @@ struct BatchArgs {
   uint64_t warps[2];   // resident warps
   uint64_t waves;      // items per resident warp to aim for
   uint32_t ntiles[2];
-  // A batch is filtered when its mean row has this many entries and its
-  // entries reach filter_min_nnz; 0: never (then only the dense kernel is
-  // launched).
+  // A batch is filtered when its entries reach filter_min_nnz and its mean row
+  // has filter_row(filter_min_row, half its evaluations); 0: never (then only
+  // the dense kernel is launched), 1: whatever the row.
   uint32_t filter_min_row;
   uint64_t filter_min_nnz;
 };

@@ -1,5 +1,5 @@
 // Prints the planner's size rules (wmh_internal.h) for the arguments
-// "filter s_pad samples nnz rows", "batch s_pad nnz rows", "keep s_pad spl
+// "row min_row evals", "filter s_pad samples nnz rows", "batch s_pad nnz rows", "keep s_pad spl
 // tiny mean_row", "split total warps waves mean_row min_items" or "both s_pad rows".
 #include <cstdio>
 #include <cstdlib>
@@ -20,6 +20,8 @@ int main(int argc, char **argv) {
   } else if (!strcmp(argv[1], "split")) {
     const mhb::FilterSplit p = mhb::filter_split(arg(2), arg(3), arg(4), arg(5), static_cast<uint32_t>(arg(6)));
     printf("%u %u", p.chunk, p.snap);
+  } else if (!strcmp(argv[1], "row")) {
+    printf("%llu", static_cast<unsigned long long>(mhb::filter_row(arg(2), arg(3))));
   } else if (!strcmp(argv[1], "both")) {
     printf("%d", arg(3) >= mhb::filter_batch_rows(s_pad));
   } else {

@@ -102,3 +102,34 @@ def test_batches_that_launch_both_kernels(rule, s_pad, rows, both):
     """A batch that could only be filtered with rows of over 4096 entries is spared
     the second launch."""
     assert rule("both", s_pad, rows) == str(both)
+
+
+# The rule's lines fall as launches grow: (samples, evaluations, mean row), how much
+# faster the filtered kernel is on Zipf columns and on uniform ones (geometric means
+# over even and ragged rows).
+@pytest.mark.parametrize("samples,evals,row,zipf,uniform", [
+    (128, 900 * M, 140, 1.01, 1.30), (128, 2000 * M, 125, 1.14, 1.32), (128, 4000 * M, 106, 0.98, 1.22),
+    (128, 150 * M, 260, 1.08, 1.33), (128, 150 * M, 160, 0.81, 1.16), (128, 300 * M, 125, 0.79, 1.03),
+    (128, 450 * M, 200, 1.00, 1.27), (128, 50 * M, 125, 1.01, 1.23), (128, 30 * M, 125, 0.86, 0.96),
+    (128, 20 * M, 330, 1.09, 1.29), (128, 20 * M, 200, 0.95, 1.11), (128, 12 * M, 420, 1.06, 1.34),
+    (64, 1000 * M, 240, 1.09, 1.52), (64, 2000 * M, 185, 1.12, 1.32), (64, 4000 * M, 155, 1.02, 1.21),
+    (64, 2000 * M, 110, 0.88, 1.00), (64, 30 * M, 160, 1.06, 1.34), (64, 150 * M, 310, 1.13, 1.40),
+    (100, 1000 * M, 116, 1.07, 1.07), (200, 140 * M, 220, 1.20, 1.26), (100, 300 * M, 130, 0.89, 1.00),
+    (100, 140 * M, 130, 0.78, 1.01), (160, 90 * M, 230, 1.17, 1.31), (48, 50 * M, 420, 1.08, 1.21),
+    (48, 50 * M, 130, 0.77, 0.92), (160, 500 * M, 122, 1.09, 1.11), (32, 140 * M, 106, 1.03, 1.20),
+    (32, 30 * M, 130, 0.96, 1.11), (256, 2000 * M, 110, 1.00, 1.18),
+])
+def test_lines_fall_with_the_launch(rule, samples, evals, row, zipf, uniform):
+    nnz = evals // samples
+    assert rule("filter", (samples + 3) // 4 * 4, samples, nnz, max(1, nnz // row)) == str(
+        int(zipf >= 0.98 and uniform > 1.05))
+
+
+@pytest.mark.parametrize("row", [1, 104, 120, 168, 288])
+def test_batch_lines(rule, row):
+    """A batch's line is that of half its evaluations; a forced one takes any row."""
+    got = [int(rule("row", row, evals // 2)) for evals in (200 * M, 1000 * M, 2000 * M, 4000 * M, 8000 * M)]
+    assert got == sorted(got, reverse=True)
+    assert got[0] <= max(row, 288) and got[-1] >= min(row, 104)
+    if row <= 104:
+        assert got == [row] * 5
