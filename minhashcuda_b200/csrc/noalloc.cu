@@ -120,8 +120,6 @@ extern "C" enum MHCUDAResult mhcuda_calc_device_noalloc(
   a.dim = g.dim;
   a.samples = g.samples;
   a.s_pad = s_pad;
-  a.bounds = g.bounds;
-  a.b_stride = mhb::bound_stride(s_pad);
   a.weights = d_weights;
   a.cols = d_cols;
   a.indptr = d_rows;
