@@ -991,8 +991,8 @@ MHCUDAResult calc_pipelined(const Gen *gen, const HostCsr &in, uint32_t length,
 // block of sample rows at a time (init, retrieve, assign).
 constexpr uint64_t kParamChunkBytes = 512ull << 20;
 
-// Largest bound table: with init's scratch it keeps a generator's device memory
-// within 4 GiB of its parameter table.
+// Largest bound table: with init's scratch (five blocks) it keeps a generator's
+// device memory within 4.5 GiB of its parameter table, and 2 GiB once it is made.
 constexpr size_t kMaxBoundBytes = size_t{2} << 30;
 
 // Sample rows per block: about kParamChunkBytes of floats, whole 8-row groups
@@ -1464,7 +1464,8 @@ enum MHCUDAResult mhcuda_calc_device(const MinhashCudaGenerator *gen, const floa
   a.indptr = d_rows;
   a.out = d_output;
   // Repeated calls with identical arguments replay a CUDA graph of the
-  // memset + plan + hash + finalize sequence (one launch instead of four).
+  // plan + hash + finalize sequence (one launch instead of three, or of four
+  // where the plan takes several blocks and cannot clear the status itself).
   // Not while profiling (per-launch events) or while the caller's stream is
   // itself being captured (the work then simply joins the caller's graph).
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;

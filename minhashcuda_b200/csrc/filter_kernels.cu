@@ -35,8 +35,8 @@
 // Against the dense kernels, device-resident, same box: 524,288 Zipf rows of
 // 1400 entries 98.1 -> 27.7 ms (3.4e12 evals/s), 131,072 ragged rows over 12M
 // columns 16.0 -> 5.3 ms, 256 uneven matrices at 256 samples 12.8 -> 5.9 ms,
-// 20,011 rows of 300 entries 855 -> 418 us.  use_filter in engine.cu says which
-// launches come here.
+// 20,011 rows of 300 entries 855 -> 418 us.  filter_rule in wmh_internal.h says
+// which launches come here.
 //
 // Rounding.  In float32 the computed ln_a may lie below the real
 // ln_c - r - w by at most 2^-24 * (6|w| + 5 r (1 + |beta|) + 3|ln_c|) (one

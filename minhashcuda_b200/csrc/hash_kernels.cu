@@ -17,8 +17,8 @@
 //    one contiguous block (SPL=4: 1536 B),
 //  - a warp owns one (chunk, sample tile) item; each lane keeps SPL running
 //    minima in registers (no shared-memory spill as in kernel.cu:72-74),
-//    each with the position of its entry; (k, t) are recovered once per
-//    (row, sample) at the row's end,
+//    each with the position of its entry and, for short rows, its t; what is
+//    missing of (k, t) is recovered once per (row, sample) at the row's end,
 //  - each warp stages its CSR positions in 256-entry windows with TMA bulk
 //    copies (cp.async.bulk, mbarrier completion, double-buffered), turns the
 //    weights into ln(weight) in place once per nnz, lane-parallel (the
@@ -84,11 +84,12 @@ __global__ void plan_kernel(const HashArgs a, bool clear) {
 // (resident blocks per SM).  The gathers are latency-bound; with 2 blocks per
 // SM there are half the warps of the 4-block budget to hide them, and 128
 // registers per thread, room for a third set (12 registers at 4 samples per
-// lane) that keeps two positions' gathers in flight: 114-118 registers, no
-// spills.  At 524,288 rows of the 1,000,000-dim Zipf(1.1) matrix this took
-// the 2-block kernel from 107.6 to 101.9 ms (4 blocks: 105.6 ms); on uniform
-// columns over 12,000,000 dims from 75.1 to 65.0 ms (4 blocks: 61.6 ms).  The
-// 3- and 4-block budgets (85 and 64 registers) have no room for it.
+// lane) that keeps two positions' gathers in flight: 111-122 registers, no
+// spills.  524,288 rows of the 1,000,000-dim Zipf(1.1) matrix take 106.3 ms
+// with it (3 and 4 blocks: 108.4 and 109.5), of uniform columns over 12,000,000
+// dims 66.0 ms (64.7 and 62.6); with two sets (compared before the samples lay
+// in pairs) the 2-block kernel took 6% and 16% longer.  The 3- and 4-block
+// budgets (85 and 64 registers) have no room for it.
 __host__ __device__ constexpr int param_depth(int minb) { return minb == 2 ? 3 : 2; }
 
 // One (chunk c, sample tile) item over the CSR of `a`: finishes the rows

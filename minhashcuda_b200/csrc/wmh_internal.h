@@ -19,12 +19,12 @@ constexpr uint32_t kStatusBadColumn = 1u;  // a column index >= dim was seen
 constexpr uint32_t kStatusBadIndptr = 2u;  // row offsets decrease or disagree with nnz
 constexpr uint32_t kStatusStall = 4u;      // a bounded wait on a staging copy gave up
 
-// Parameter table: one contiguous block per column d,
-//   params[(d * 3 + 0) * s_pad + s] = r      (rs)
-//   params[(d * 3 + 1) * s_pad + s] = ln_c   (ln_cs)
-//   params[(d * 3 + 2) * s_pad + s] = beta   (betas)
-// s_pad = samples rounded up to a multiple of 4, so every section starts on a
-// 16-byte boundary and a lane can fetch 4 consecutive samples as one float4.
+// Parameter table: one contiguous block of 3 * s_pad floats per column, its
+// samples in pairs r r ln_c ln_c beta beta: r of sample s at
+//   params[d * 3 * s_pad + (s / 2) * 6 + s % 2]      (param_index)
+// and its ln_c and beta 2 and 4 floats further.  s_pad = samples rounded up to
+// a multiple of 4, so a lane can fetch 4 consecutive samples as three aligned
+// float4, and a single sample's three values lie in 24 bytes.
 inline uint32_t padded_samples(uint32_t samples) { return (samples + 3u) & ~3u; }
 
 // Work decomposition of one hash launch.
@@ -45,7 +45,7 @@ struct HashPlan {
   uint32_t spl;      // samples per lane in one item: 1, 2 or 4
   uint32_t minb;     // kernel variant: minimum resident blocks per SM (4; 3 or 2 for spl 4)
   uint32_t ntiles;   // sample tiles of 32*spl samples (filter: of 16*filter)
-  uint32_t grid;     // persistent grid (blocks of kHashBlock threads)
+  uint32_t grid;     // persistent grid (blocks of plan_block_warps warps)
   uint32_t filter;   // 0: the dense kernel; 8, 4, 2: the bound-filtered one
                      // (filter_kernels.cu) with that many lanes per entry
   uint32_t snap;     // HashArgs::snap
