@@ -148,21 +148,24 @@ def kernel_source_sha16():
 
 
 def filtered(nnz, rows, samples):
-    """Whether the engine's rule gives a launch of this size the bound-filtered
-    kernel (make_plan's use_filter in engine.cu; the tuner agrees on these
-    workloads)."""
+    """Whether the engine's rule gives a launch of this size and 128 samples the
+    bound-filtered kernel (filter_rule and filter_row in wmh_internal.h; the tuner
+    agrees on these workloads)."""
     forced = os.environ.get("MHCUDA_B200_FILTER")
     if forced is not None:
         return forced != "0"
-    return samples > 28 and nnz >= 104 * rows and nnz * samples >= 1 << 23
+    evals = nnz * samples
+    row = next((r for least, r in ((3 << 30, 104), (3 << 29, 105), (3 << 28, 126), (5 << 25, 168))
+                if evals >= least), 210)
+    return samples == 128 and evals >= 1 << 27 and nnz >= row * rows
 
 
 def kernel_profile(variant):
     """Counters ncu measured for the hash kernel variant `variant` (the
     filtered kernel's "filter" and "filter_uniform", or a dense one's, e.g.
     "spl4_minb3") on a small case of its workload
-    (profiles/hash_kernel_traffic.json), and whether they were taken on the
-    kernel source this run built."""
+    (profiles/hash_kernel_traffic.json), and whether that variant's were taken on
+    the kernel source this run built."""
     if not os.path.exists(PROFILE_JSON):
         return None, False
     d = json.load(open(PROFILE_JSON))
@@ -170,7 +173,7 @@ def kernel_profile(variant):
     if v is None:
         return None, False
     v = dict({"captured_case": d.get("captured_case")}, **v, variant=variant)
-    return v, d.get("source_sha16") == kernel_source_sha16()
+    return v, v.get("source_sha16") == kernel_source_sha16()
 
 
 def digest(a):

@@ -133,3 +133,16 @@ def test_batch_lines(rule, row):
     assert got[0] <= max(row, 288) and got[-1] >= min(row, 104)
     if row <= 104:
         assert got == [row] * 5
+
+
+def test_the_benchmarks_copy_of_the_rule(rule, monkeypatch):
+    """bench.py names the kernel of its launches by the same lines."""
+    import importlib.util
+    spec = importlib.util.spec_from_file_location("bench_module", os.path.join(ROOT, "bench.py"))
+    bench = importlib.util.module_from_spec(spec)
+    spec.loader.exec_module(bench)
+    monkeypatch.delenv("MHCUDA_B200_FILTER", raising=False)
+    for evals in (140 * M, 200 * M, 900 * M, 2000 * M, 9000 * M):
+        for row in (100, 110, 130, 150, 180, 220, 1400):
+            nnz = evals // 128
+            assert str(int(bench.filtered(nnz, nnz // row, 128))) == rule("filter", 128, 128, nnz, nnz // row)
