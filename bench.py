@@ -173,7 +173,7 @@ def kernel_profile(variant):
     if v is None:
         return None, False
     v = dict({"captured_case": d.get("captured_case")}, **v, variant=variant)
-    return v, v.get("source_sha16") == kernel_source_sha16()
+    return v, v.get("source_sha16", d.get("source_sha16")) == kernel_source_sha16()
 
 
 def digest(a):
